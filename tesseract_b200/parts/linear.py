@@ -1,7 +1,7 @@
 """Matrix product ``y = x @ W^T`` with a weight kept as ``[out, in]``.
 
 Which kernel runs a product is the kernel plan's decision (``tesseract_b200.plan.product``); this class carries
-the decision out.  In float32: the package's own 32-bit kernel (a fixed K-ordered chain per output element).  In
+the decision out.  In float32: the package's own 32-bit kernel (one order of summation per output element, decided by K alone).  In
 bfloat16: the weight-streaming kernels up to 16 rows (``decode_linear``, optionally with the norm in front and
 SwiGLU behind folded in) and up to 128 rows (``skinny_tcgen05``), the tcgen05 GEMM where the plan says so, else
 the library GEMM with 32-bit accumulation, where the reference

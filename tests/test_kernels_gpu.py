@@ -96,6 +96,33 @@ def test_gemm_f32(m, n, k):
                                atol=1e-5 * math.sqrt(k))
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 17, 8), (2, 16, 264), (3, 4737, 2048), (8, 40, 2056), (9, 33, 4104), (48, 65, 256),
+                                     (49, 130, 264), (70, 100, 2048), (130, 3100, 72), (129, 3072, 2048)])
+def test_gemm_f32_streams_and_tiles_sum_in_one_order(m, n, k):
+    """Rows picked from a larger product, and the guarded loads of operands off their alignment, give the same bits, so the
+    streaming kernel (few rows) and both tile shapes are one sum; and that sum is near the 64-bit one."""
+    from tesseract_b200 import kernels
+
+    torch.manual_seed(4)
+    a, w = torch.randn(m, k), torch.randn(n, k)
+    wide = torch.full((m, n + 3), 7.0, device="cuda")
+    out = kernels.gemm_f32_nt(dev(a), dev(w), wide[:, 1:n + 1])
+    assert (wide[:, 0] == 7).all() and (wide[:, n + 1:] == 7).all()
+    # chains of 64 and one addition a chain: the rounding of a sum of k terms of size 1 stays below (64 + k / 64) steps of it
+    want = a.double() @ w.double().T
+    scale = a.double().abs() @ w.double().abs().T
+    assert ((out.cpu().double() - want).abs() <= (64 + k / 64) * 2.0 ** -24 * scale).all()
+    for rows in {1, min(m, 2), min(m, 4), min(m, 8), min(m, 48), m}:
+        part = torch.empty(rows, n, device="cuda")
+        kernels.gemm_f32_nt(dev(a[m - rows:].contiguous()), dev(w), part)
+        assert torch.equal(part, out[m - rows:])
+    shifted = torch.zeros(n, k + 1)
+    shifted[:, 1:] = w
+    guarded = torch.empty(m, n, device="cuda")
+    kernels.gemm_f32_nt(dev(a), dev(shifted)[:, 1:], guarded)
+    assert torch.equal(guarded, out)
+
+
 def test_gemm_f32_is_true_32_bit():
     """A product that a reduced-precision matrix mode (10-bit mantissa) would get visibly wrong."""
     from tesseract_b200 import kernels
