@@ -94,6 +94,13 @@ def test_norms_around_an_addition(width, out_dtype):
     close(out, plain.layer_norm(x.double(), w2.double(), b2.double(), eps), TOL[out_dtype], "norm alone")
 
 
+@pytest.mark.parametrize("width", [256, 768, 3328, 8192, 8448])
+def test_norms_around_an_addition_with_the_row_in_registers(width):
+    """The smallest and largest rows that a block holds in registers, warps that are no power of two, and the width behind."""
+    test_norms_around_an_addition(width, torch.float32)
+    test_norms_around_an_addition(width, torch.bfloat16)
+
+
 @pytest.mark.parametrize("width", [7, 64, 200, 4096])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_over_all_heads_with_a_gate(width, dtype):
