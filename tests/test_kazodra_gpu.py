@@ -195,6 +195,30 @@ def test_recurrence_in_portions_against_token_by_token(dtype, heads, d, dv, deca
         assert bool((state[0] == 5.0).all()) and bool((state[2] == 5.0).all())      # other requests' slots untouched
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,dv", [(1, 5), (127, 33), (128, 128), (129, 64), (300, 40)])
+def test_a_decoded_row_renews_every_number_of_its_state_once(dtype, d, dv):
+    """Key sizes around what a thread holds of the state at a time, by the recurrence in 64 bits."""
+    from tesseract_b200 import kernels
+
+    heads, seqs = 2, 3
+    g = torch.Generator().manual_seed(d)
+    state = torch.randn(seqs + 1, heads, d, dv, generator=g)
+    proj = (torch.randn(seqs, heads * (2 * d + dv), generator=g)).to(dtype)
+    decay = torch.tensor([0.9, 1.0])
+    on, out = state.clone().to(dev()), torch.empty(seqs, heads * dv, device=dev())
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev())         # noqa: E731
+    kernels.lightning(proj.to(dev()), decay.to(dev()), on, out, i32([0, 1, 2, 3]), i32([3, 0, 2]), num_seqs=seqs, heads=heads, dim=d,
+                      vdim=dv, max_new=1)
+    q, k, v = (plain.silu(x.double()).view(seqs, heads, -1) for x in proj.split([heads * d, heads * d, heads * dv], dim=1))
+    for t, slot in enumerate([3, 0, 2]):
+        S = decay.double()[:, None, None] * state[slot].double() + k[t][:, :, None] * v[t][:, None, :]
+        # a product and a sum rounded once each; sums of d products
+        close(on[slot], S, 4 * 2.0 ** -24, "state")
+        close(out[t], torch.einsum("hde,hd->he", S, q[t]).reshape(-1), (d + 8) * 2.0 ** -24, "row")
+    assert torch.equal(on[1].cpu(), state[1])
+
+
 @pytest.mark.parametrize("decay", [1.0, 0.995])
 def test_recurrence_keeps_a_product_from_hundreds_of_tokens_back(decay):
     """One token's key and value are large and every later query points at that key; all else is small: what the rows
@@ -233,7 +257,7 @@ def test_recurrence_keeps_a_product_from_hundreds_of_tokens_back(decay):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,d,dv", [(3, 8, 12), (2, 64, 64), (1, 128, 33), (2, 5, 40)])
-def test_long_portions_side_by_side_continue_each_sequence_from_its_slot(dtype, heads, d, dv):
+def test_long_portions_side_side_by_side_continue_each_sequence_from_its_slot(dtype, heads, d, dv):
     """A step with prompt portions of several chunks (whose chunks run side by side and meet in a scan) beside a single
     row and a short portion, every sequence from a state of its own in a slot of its own; then a second step of the same
     sequences goes on from what the first left."""
@@ -446,6 +470,30 @@ def test_two_maps_see_exactly_their_keys(dtype, heads, kv_heads, d, dv, window, 
                                               torch.arange(T), round_to=torch.bfloat16)
         noise = (coarse - want).abs().max().item()
     run_part_in_cuts(part, h, dtype, T, page, want, window, noise)
+
+
+@pytest.mark.parametrize("dim,vdim", [(576, 512), (288, 256), (160, 128)])
+@pytest.mark.parametrize("rows,heads,window", [(1, 1, None), (3, 17, 40), (9, 16, None)])
+def test_latent_runs_of_a_decoded_row_are_added_up(dim, vdim, rows, heads, window):
+    """Rows of very different reach (most of a short row's runs are empty), against the softmax in 64 bits."""
+    from tesseract_b200 import kernels
+
+    g = torch.Generator().manual_seed(rows * heads)
+    page, pages = 16, 80
+    cache = torch.randn(pages, page, dim, generator=g).to(torch.bfloat16)
+    q = (torch.randn(rows, heads * dim, generator=g) * 0.5).to(torch.bfloat16)
+    positions = [(t * 733 + 1) % 1200 for t in range(rows)]
+    table = torch.stack([torch.randperm(pages, generator=g) for _ in range(rows)]).to(torch.int32)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev())         # noqa: E731
+    out = torch.empty(rows, heads * vdim, dtype=torch.bfloat16, device=dev())
+    kernels.attention_latent_mma(q.to(dev()), out, cache.to(dev()), i32(positions), i32(list(range(rows))), table.to(dev()),
+                                 heads=heads, dim=dim, vdim=vdim, page_size=page, scale=dim ** -0.5,
+                                 mask_kind=kernels.MASK_WINDOW if window else kernels.MASK_CAUSAL, mask_size=window or 0)
+    for t, pos in enumerate(positions):
+        first = max(0, pos - window + 1) if window else 0
+        keys = cache[table[t].long()].reshape(-1, dim)[first:pos + 1].double()
+        weights = torch.softmax(q[t].view(heads, dim).double() @ keys.T * dim ** -0.5, dim=-1)
+        close(out[t], (weights @ keys[:, :vdim]).reshape(-1), TOL[torch.bfloat16], f"row {t}")
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
