@@ -24,12 +24,15 @@
 //   2. per sequence, head and slice, the tiles in order:  S_0 = state,  S_(i+1) = a^(c_i) S_i + U_i ; every S_i is kept
 //      where U_i was, the last one goes back to the state slot
 //   3. every tile's outputs from its S_i and its own rows, as above.
+// Key sizes of 64 and 128 with whole packets take kernels for 1 and 3 that hold blocks of the products in registers, to the
+// same bits.
 #include "common.cuh"
 
 namespace {
 
 constexpr int kThreads = 256;
 constexpr int kSlice = 32;          // value columns a block owns
+constexpr int kScanned = 8;         // tiles a thread of the scan asks for at a time
 constexpr int kRows = 8;            // rows (or key dimensions) a warp carries in registers at a time
 static_assert(kRows == 8, "the vector forms below are written for eight");
 
@@ -423,7 +426,189 @@ lightning_tile_sum_kernel(const T* __restrict__ proj, int64_t proj_stride, int k
     }
 }
 
-// Launch 2: per sequence and head, the tiles in order.  Every number of the state is a chain of its own.
+// ---- the tiles of a long portion, for head sizes that fill them ------------------------------------------------------------
+
+typedef unsigned long long pair32;   // two neighbouring 32-bit floats
+__device__ __forceinline__ pair32 twice(float x) {
+    pair32 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 parts_of(pair32 p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void fma2(pair32& d, pair32 a, pair32 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+constexpr int kTile = 64;            // rows of a tile
+constexpr int kTileCols = 64;        // value columns of a block
+
+// dst[i][t] = act(src[t][i]) for c rows of n numbers, and zeros for the rows up to kTile: a warp takes a packet of every row in
+// turn, so that neighbouring lanes write neighbouring numbers.
+template <typename T>
+__device__ __forceinline__ void load_silu_transposed(float* dst, int dst_stride, const T* src, int64_t stride, int c, int n, int act) {
+    constexpr int N = Packet<T>::N;
+    for (int e = threadIdx.x; e < kTile * (n / N); e += kThreads) {
+        const int t = e % kTile, i = e / kTile * N;
+        float v[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) v[u] = 0.0f;
+        if (t < c) {
+            Packet<T>::load(src + (int64_t)t * stride + i, v);
+#pragma unroll
+            for (int u = 0; u < N; ++u) v[u] = activate(v[u], act);
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) dst[(i + u) * dst_stride + t] = v[u];
+    }
+}
+
+// Launch 3 of the tiled form for D key dimensions (64 or 128) and a multiple of 64 value columns: what lightning_kernel does
+// for a tile, to the bit, as three products of blocks in registers (a thread 4 x 4 numbers, two multiply-adds an instruction),
+// where it read shared memory for every number.  Queries and keys lie transposed, so that every product is a sum over a
+// leading index in order.  The keys' room becomes the state's once the scores are taken; the state is on its way in registers
+// meanwhile.  Bound by the multiply-adds and shared memory's bandwidth.  2,000 rows of 16 heads of 128 x 128, the three
+// launches: 165 us, 427 before.
+template <typename T, int D>
+__global__ void __launch_bounds__(kThreads, 2)
+lightning_tile_out_kernel(const T* proj, int64_t proj_stride, int q_off, int k_off, int v_off, const float* __restrict__ decay,
+                          float* out, const int* row_start, int num_seqs, int heads, int vdim, const float* tile_state, int act) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int P = kTile + 4;
+    float* qs = smem;                              // [D][P]: numbers of a key dimension side by side
+    float* ks = qs + D * P;                        // [D][P], then the state [D][kTileCols]
+    float* A = ks + D * P;                         // [s][t]
+    float* vs = A + kTile * P;                     // [kTile][kTileCols]
+    float* pw = vs + kTile * kTileCols;            // [kTile + 1]
+    pdl_trigger();
+    const int head = blockIdx.y, col0 = blockIdx.z * kTileCols, tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const float a = decay[head];
+    for (int i = tid; i <= kTile; i += kThreads) pw[i] = (float)pow((double)a, (double)i);
+    pdl_wait();
+    int seq, r0, c;
+    if (!find_tile(row_start, num_seqs, kTile, blockIdx.x, seq, r0, c)) return;
+    constexpr int HELD = D * kTileCols / 4 / kThreads;
+    const float* from = tile_state + ((int64_t)blockIdx.x * heads + head) * D * vdim + col0;
+    float4 held[HELD];
+#pragma unroll
+    for (int u = 0; u < HELD; ++u)
+        held[u] = *reinterpret_cast<const float4*>(from + (int64_t)(u * 16 + ty) * vdim + tx * 4);
+    const T* rows_at = proj + (int64_t)r0 * proj_stride;
+    load_silu_transposed<T>(qs, P, rows_at + q_off + (int64_t)head * D, proj_stride, c, D, act);
+    load_silu_transposed<T>(ks, P, rows_at + k_off + (int64_t)head * D, proj_stride, c, D, act);
+    load_silu_rows<T, true>(vs, kTileCols, rows_at + v_off + (int64_t)head * vdim + col0, proj_stride, c, kTileCols, kTileCols, act);
+    for (int e = tid; e < (kTile - c) * kTileCols; e += kThreads) vs[c * kTileCols + e] = 0.0f;
+    __syncthreads();
+    // sum[r][.] += left[i][4 ty + r] * right[i][4 tx ..] over i in order
+    auto add = [&](pair32 (&sum)[4][2], const float* left, const float* right, int right_stride, int n) {
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) {
+            const float4 l = *reinterpret_cast<const float4*>(left + i * P + ty * 4);
+            const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(right + i * right_stride + tx * 4);
+            const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const pair32 both = twice(lv[r]);
+                fma2(sum[r][0], both, m.x);
+                fma2(sum[r][1], both, m.y);
+            }
+        }
+    };
+    {   // scores, kept transposed: this thread's rows are keys s = 4 ty + r, its columns queries t = 4 tx ..
+        pair32 sum[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) sum[r][0] = sum[r][1] = 0;
+        add(sum, ks, qs, P, D);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int s = ty * 4 + r;
+            const float2 lo = parts_of(sum[r][0]), hi = parts_of(sum[r][1]);
+            float dots[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int t = tx * 4 + e;
+                dots[e] = s <= t ? dots[e] * pw[t - s] : 0.0f;
+            }
+            *reinterpret_cast<float4*>(A + s * P + tx * 4) = make_float4(dots[0], dots[1], dots[2], dots[3]);
+        }
+    }
+    __syncthreads();                               // the keys are done with
+    float* S = ks;
+#pragma unroll
+    for (int u = 0; u < HELD; ++u) *reinterpret_cast<float4*>(S + (u * 16 + ty) * kTileCols + tx * 4) = held[u];
+    __syncthreads();
+    // outputs: rows t = 4 ty + r, columns 4 tx ..
+    pair32 from_state[4][2], inside[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) from_state[r][0] = from_state[r][1] = inside[r][0] = inside[r][1] = 0;
+    add(from_state, qs, S, kTileCols, D);
+    add(inside, A, vs, kTileCols, ((ty | 1) + 1) * 4);      // (a row's scores behind itself are zeros; both halves of a warp go as far)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = ty * 4 + r;
+        const pair32 power = twice(pw[t + 1]);
+        fma2(inside[r][0], power, from_state[r][0]);
+        fma2(inside[r][1], power, from_state[r][1]);
+        const float2 lo = parts_of(inside[r][0]), hi = parts_of(inside[r][1]);
+        if (t < c)
+            *reinterpret_cast<float4*>(out + (int64_t)(r0 + t) * heads * vdim + (int64_t)head * vdim + col0 + tx * 4) =
+                make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+}
+
+// Launch 1 of the tiled form for the same sizes: U = sum_s a^(c-1-s) k_s v_s^T, a thread D / 16 x 4 numbers.
+template <typename T, int D>
+__global__ void __launch_bounds__(kThreads, 2)
+lightning_tile_sum_blocks_kernel(const T* proj, int64_t proj_stride, int k_off, int v_off, const float* __restrict__ decay,
+                                 float* tile_state, const int* row_start, int num_seqs, int heads, int vdim, int act) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int DP = D + 4, R = D / 16;
+    float* ks = smem;                              // [kTile][DP]
+    float* vs = ks + kTile * DP;                   // [kTile][kTileCols]
+    float* pw = vs + kTile * kTileCols;            // [kTile]
+    pdl_trigger();
+    const int head = blockIdx.y, col0 = blockIdx.z * kTileCols, tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const float a = decay[head];
+    for (int i = tid; i < kTile; i += kThreads) pw[i] = (float)pow((double)a, (double)i);
+    pdl_wait();
+    int seq, r0, c;
+    if (!find_tile(row_start, num_seqs, kTile, blockIdx.x, seq, r0, c)) return;
+    const T* rows_at = proj + (int64_t)r0 * proj_stride;
+    load_silu_rows<T, true>(ks, DP, rows_at + k_off + (int64_t)head * D, proj_stride, c, D, D, act);
+    load_silu_rows<T, true>(vs, kTileCols, rows_at + v_off + (int64_t)head * vdim + col0, proj_stride, c, kTileCols, kTileCols, act);
+    __syncthreads();
+    pair32 sum[R][2];
+#pragma unroll
+    for (int r = 0; r < R; ++r) sum[r][0] = sum[r][1] = 0;
+#pragma unroll 4
+    for (int s = 0; s < c; ++s) {
+        const float power = pw[c - 1 - s];
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vs + s * kTileCols + tx * 4);
+#pragma unroll
+        for (int g = 0; g < R / 4; ++g) {
+            const float4 k = *reinterpret_cast<const float4*>(ks + s * DP + g * 64 + ty * 4);
+            const float kv[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const pair32 both = twice(kv[r] * power);
+                fma2(sum[g * 4 + r][0], both, v.x);
+                fma2(sum[g * 4 + r][1], both, v.y);
+            }
+        }
+    }
+    float* mine = tile_state + ((int64_t)blockIdx.x * heads + head) * D * vdim + col0 + tx * 4;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const float2 lo = parts_of(sum[r][0]), hi = parts_of(sum[r][1]);
+        *reinterpret_cast<float4*>(mine + (int64_t)(r / 4 * 64 + ty * 4 + r % 4) * vdim) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+}
+
+// Launch 2: per sequence and head, the tiles in order.  Every number of the state is a chain of its own.  Bound by the
+// latency of the chain's loads (tiles are therefore asked for kScanned at a time).
 __global__ void __launch_bounds__(kThreads)
 lightning_scan_kernel(const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ tile_state,
                       const int* __restrict__ row_start, const int* __restrict__ state_slots, int heads, int dim, int vdim,
@@ -444,10 +629,18 @@ lightning_scan_kernel(const float* __restrict__ decay, float* __restrict__ state
     float* kept = tile_state + ((int64_t)first_tile * heads + head) * dim * vdim;
     for (int e = blockIdx.z * kThreads + threadIdx.x; e < dim * vdim; e += gridDim.z * kThreads) {
         float current = slot[e];
-        for (int i = 0; i < tiles; ++i) {
-            const float own = kept[i * stride + e];
-            kept[i * stride + e] = current;
-            current = fmaf(i + 1 < tiles ? whole : rest, current, own);
+        for (int i0 = 0; i0 < tiles; i0 += kScanned) {
+            float own[kScanned];                   // asked for together: a store in between would hold back the next load
+#pragma unroll
+            for (int u = 0; u < kScanned; ++u) own[u] = i0 + u < tiles ? kept[(i0 + u) * stride + e] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < kScanned; ++u) {
+                const int i = i0 + u;
+                if (i < tiles) {
+                    kept[i * stride + e] = current;
+                    current = fmaf(i + 1 < tiles ? whole : rest, current, own[u]);
+                }
+            }
         }
         slot[e] = current;
     }
@@ -540,6 +733,40 @@ int tiles_for(int rows, int num_seqs, int dim, int max_new) {
     return (rows + chunk - 1) / chunk + num_seqs;
 }
 
+// The tiled form's first and third launch as products of blocks: head sizes they are built for, tiles of 64 rows, and rows,
+// outputs and tile states that start on packets.  (Everything else takes the kernels that read a number at a time.)
+template <typename T>
+bool takes_blocks(const void* proj, int64_t proj_stride, int q_off, int k_off, int v_off, const float* out,
+                  const float* tile_state, int dim, int vdim, int chunk) {
+    constexpr int N = Packet<T>::N;
+    return (dim == 64 || dim == 128) && vdim % kTileCols == 0 && chunk == kTile && proj_stride % N == 0 && q_off % N == 0 &&
+           k_off % N == 0 && v_off % N == 0 && ((uintptr_t)proj | (uintptr_t)out | (uintptr_t)tile_state) % 16 == 0;
+}
+
+template <typename T, int D>
+int launch_blocks(const void* proj, int64_t proj_stride, int q_off, int k_off, int v_off, const float* decay, float* state,
+                  float* out, const int* row_start, const int* state_slots, int num_seqs, int heads, int vdim, int tiles,
+                  float* tile_state, int act, cudaStream_t stream) {
+    const size_t out_smem = sizeof(float) * (2 * D * (kTile + 4) + kTile * (kTile + 4) + kTile * kTileCols + kTile + 4);
+    const size_t sum_smem = sizeof(float) * (kTile * (D + 4) + kTile * kTileCols + kTile);
+    auto sums = lightning_tile_sum_blocks_kernel<T, D>;
+    auto outs = lightning_tile_out_kernel<T, D>;
+    cudaError_t err = cudaFuncSetAttribute(sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(outs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+    const dim3 grid(tiles, heads, vdim / kTileCols);
+    if (err == cudaSuccess)
+        err = tb_launch_pdl(sums, grid, dim3(kThreads), sum_smem, stream, (const T*)proj, proj_stride, k_off, v_off, decay,
+                            tile_state, row_start, num_seqs, heads, vdim, act);
+    const int parts = max(1, min(64, (D * vdim + kThreads - 1) / kThreads));
+    if (err == cudaSuccess)
+        err = tb_launch_pdl(lightning_scan_kernel, dim3(num_seqs, heads, parts), dim3(kThreads), (size_t)0, stream, decay, state,
+                            tile_state, row_start, state_slots, heads, D, vdim, kTile);
+    if (err == cudaSuccess)
+        err = tb_launch_pdl(outs, grid, dim3(kThreads), out_smem, stream, (const T*)proj, proj_stride, q_off, k_off, v_off, decay,
+                            out, row_start, num_seqs, heads, vdim, (const float*)tile_state, act);
+    return err == cudaSuccess ? tb_launch_status() : (int)err;
+}
+
 template <typename T>
 int launch(const void* proj, int64_t proj_stride, int q_off, int k_off, int v_off, const float* decay, float* state,
            float* out, const int* row_start, const int* state_slots, int rows, int num_seqs, int heads, int dim, int vdim,
@@ -575,6 +802,11 @@ int launch(const void* proj, int64_t proj_stride, int q_off, int k_off, int v_of
         return launched == cudaSuccess ? tb_launch_status() : (int)launched;
     }
     if (tile_state == nullptr) return TB_ERR_BAD_SIZE;
+    if (takes_blocks<T>(proj, proj_stride, q_off, k_off, v_off, out, tile_state, dim, vdim, chunk)) {
+        auto blocks = dim == 64 ? launch_blocks<T, 64> : launch_blocks<T, 128>;
+        return blocks(proj, proj_stride, q_off, k_off, v_off, decay, state, out, row_start, state_slots, num_seqs, heads, vdim,
+                      tiles, tile_state, act, stream);
+    }
     auto sums = lightning_tile_sum_kernel<T>;
     const size_t sums_smem = sizeof(float) * ((size_t)chunk * row_floats(dim) + (size_t)chunk * kSlice + chunk + 1);
     if (sums_smem > 40 * 1024) {

@@ -256,6 +256,43 @@ def test_recurrence_keeps_a_product_from_hundreds_of_tokens_back(decay):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,d,dv", [(2, 64, 64), (3, 128, 128), (1, 64, 192)])
+def test_long_portions_as_products_of_blocks(dtype, heads, d, dv):
+    """Rows that start on packets take the block kernels: against the recurrence in 64 bits, and against the same rows off
+    their alignment, which take the kernels that read a number at a time; whole tiles, a row more and a row fewer."""
+    from tesseract_b200 import kernels
+
+    g = torch.Generator().manual_seed(d + dv)
+    decay, slots, lengths = torch.tensor([0.9, 1.0, 0.99][:heads]), [4, 0, 2, 1], [256, 65, 1, 319]
+    state = torch.randn(6, heads, d, dv, generator=g)
+    edges = [sum(lengths[:n]) for n in range(len(lengths) + 1)]
+    rows, width = edges[-1], heads * (2 * d + dv)
+    proj = (torch.randn(rows, width, generator=g) * 0.7).to(dtype)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev())         # noqa: E731
+    results = []
+    for shift in (0, 1):
+        wide = torch.zeros(rows, width + 8 * shift, dtype=dtype)
+        wide[:, shift:shift + width] = proj
+        on, out = state.clone().to(dev()), torch.empty(rows, heads * dv, device=dev())
+        kernels.lightning(wide.to(dev())[:, shift:shift + width], decay.to(dev()), on, out, i32(edges), i32(slots),
+                          num_seqs=len(slots), heads=heads, dim=d, vdim=dv, max_new=max(lengths))
+        results.append((out, on))
+    q, k, v = (plain.silu(x.double()).view(rows, heads, -1) for x in proj.split([heads * d, heads * d, heads * dv], dim=1))
+    want, a = torch.empty(rows, heads, dv, dtype=torch.float64), decay.double()[:, None, None]
+    for slot, lo, hi in zip(slots, edges[:-1], edges[1:]):
+        S = state[slot].double()
+        for t in range(lo, hi):
+            S = a * S + k[t][:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hde,hd->he", S, q[t])
+        for out, on in results:
+            close(on[slot], S, 2e-5, "state")
+    for out, on in results:
+        close(out, want.reshape(rows, -1), 2e-5, "rows")
+    for which in (3, 5):
+        assert torch.equal(results[0][1][which].cpu(), state[which])                    # other requests' slots
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,d,dv", [(3, 8, 12), (2, 64, 64), (1, 128, 33), (2, 5, 40)])
 def test_long_portions_side_side_by_side_continue_each_sequence_from_its_slot(dtype, heads, d, dv):
     """A step with prompt portions of several chunks (whose chunks run side by side and meet in a scan) beside a single
