@@ -17,6 +17,7 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;
 constexpr int kKeyBlock = 32;
+constexpr int kFewBlocks = 592;      // up to four blocks a multiprocessor
 
 template <typename T>
 struct Vec16;
@@ -42,7 +43,8 @@ struct Vec16<__nv_bfloat16> {
     }
 };
 
-template <typename T, int NC>
+// UNDER: loads under way at a time (packets of a key, values of a block).
+template <typename T, int NC, int UNDER>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__ out, int64_t out_stride,
                       const T* __restrict__ cache, const int* __restrict__ positions,
@@ -84,11 +86,18 @@ attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__
             key_offset = (int64_t)page * page_block + (int64_t)(key % page_size) * head_dim;
             const T* kp = kbase + key_offset;
             float dot = 0.0f;
-            float kv[Vec16<T>::N];
-            for (int i = 0; i < head_dim; i += Vec16<T>::N) {
-                Vec16<T>::load(kp + i, kv);
+            // (UNDER packets asked for at a time; the sum runs on in order)
+            for (int i0 = 0; i0 < head_dim; i0 += UNDER * Vec16<T>::N) {
+                float kv[UNDER][Vec16<T>::N];
 #pragma unroll
-                for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i + e], kv[e], dot);
+                for (int u = 0; u < UNDER; ++u)
+                    if (i0 + u * Vec16<T>::N < head_dim) Vec16<T>::load(kp + i0 + u * Vec16<T>::N, kv[u]);
+#pragma unroll
+                for (int u = 0; u < UNDER; ++u)
+                    if (i0 + u * Vec16<T>::N < head_dim) {
+#pragma unroll
+                        for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i0 + u * Vec16<T>::N + e], kv[u][e], dot);
+                    }
             }
             s = dot * scale;
         }
@@ -100,15 +109,22 @@ attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__
         for (int c = 0; c < NC; ++c) acc[c] *= corr;
         const float p_mma = Elem<T>::round(p);
         const int keys_here = min(kKeyBlock, pos - kb * kKeyBlock + 1);
-        for (int j = 0; j < keys_here; ++j) {
-            const float pj = __shfl_sync(0xffffffffu, p_mma, j);
-            const int64_t off = __shfl_sync(0xffffffffu, key_offset, j);
-            if (pj != 0.0f) {  // uniform across the warp; masked keys contribute nothing
-                const T* vp = vbase + off;
+        for (int j0 = 0; j0 < keys_here; j0 += UNDER) {
+            float v[UNDER][NC];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int col = c * 32 + lane;
-                    if (col < head_dim) acc[c] = fmaf(pj, Elem<T>::load(vp + col), acc[c]);
+            for (int u = 0; u < UNDER; ++u) {
+                const T* vp = vbase + __shfl_sync(0xffffffffu, key_offset, j0 + u);    // (a lane without a key: offset 0, not used)
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (j0 + u < keys_here && c * 32 + lane < head_dim) v[u][c] = Elem<T>::load(vp + c * 32 + lane);
+            }
+#pragma unroll
+            for (int u = 0; u < UNDER; ++u) {
+                const float pj = __shfl_sync(0xffffffffu, p_mma, j0 + u);
+                if (j0 + u < keys_here && pj != 0.0f) {  // uniform across the warp; masked keys contribute nothing
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (c * 32 + lane < head_dim) acc[c] = fmaf(pj, v[u][c], acc[c]);
                 }
             }
         }
@@ -130,14 +146,26 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
            cudaStream_t stream) {
     dim3 grid(rows, (num_heads + kWarpsPerBlock - 1) / kWarpsPerBlock);
     const size_t smem = (size_t)kWarpsPerBlock * head_dim * sizeof(float);
-#define TB_LAUNCH(NC)                                                                                          \
-    attention_rows_kernel<T, NC><<<grid, kWarpsPerBlock * 32, smem, stream>>>(                                 \
+#define TB_LAUNCH(NC, UNDER)                                                                                          \
+    attention_rows_kernel<T, NC, UNDER><<<grid, kWarpsPerBlock * 32, smem, stream>>>(                                 \
         (const T*)q, q_stride, (T*)out, out_stride, (const T*)cache, positions, seq_of_row, block_table,       \
         bt_stride, num_heads, num_kv_heads, head_dim, page_size, window, scale)
-    if (head_dim <= 32) TB_LAUNCH(1);
-    else if (head_dim <= 64) TB_LAUNCH(2);
-    else if (head_dim <= 128) TB_LAUNCH(4);
-    else TB_LAUNCH(8);
+    // Few warps a multiprocessor (decoded rows) are bound by the latency of their loads: 4 rows of 32 heads of 64 behind some
+    // 100 keys 16.4 us with 32 under way in 32-bit (39 one after another), 24.5 with 16 in bfloat16 (36).  Where the warps fill
+    // the chip the registers that this takes cost more than it gives: 381 prompt rows 76 us with 2 (8: 82, 1: 82), in bfloat16
+    // 55 with 1 (8: 97).  Wide bfloat16 heads stop gaining early (head size 256: 46 us one after another, 38 with 4, 52 with 8).
+    constexpr bool wide = sizeof(T) == 4;
+    if ((int64_t)rows * grid.y <= kFewBlocks) {
+        if (head_dim <= 32) TB_LAUNCH(1, (wide ? 32 : 16));
+        else if (head_dim <= 64) TB_LAUNCH(2, (wide ? 32 : 16));
+        else if (head_dim <= 128) TB_LAUNCH(4, (wide ? 16 : 4));
+        else TB_LAUNCH(8, (wide ? 8 : 4));
+    } else {
+        if (head_dim <= 32) TB_LAUNCH(1, (wide ? 2 : 1));
+        else if (head_dim <= 64) TB_LAUNCH(2, (wide ? 2 : 1));
+        else if (head_dim <= 128) TB_LAUNCH(4, (wide ? 2 : 1));
+        else TB_LAUNCH(8, (wide ? 2 : 1));
+    }
 #undef TB_LAUNCH
     return tb_launch_status();
 }

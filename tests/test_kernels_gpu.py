@@ -204,6 +204,27 @@ def test_attention_rows(dtype, lengths, new, nh, nkv, d, page_size, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d, nh", [(16, 4), (64, 8), (104, 4), (256, 4)])
+def test_attention_rows_gives_few_rows_the_bits_of_many(dtype, d, nh):
+    """Steps of few rows ask for more of their keys at a time; the sums keep their order."""
+    from tesseract_b200 import kernels
+
+    rows, page_size = 620, 16
+    case = paged_case(dtype, [rows + 9], [rows], nh, 2, d, page_size, seed=d)
+    q, out = dev(case["q"]).view(rows, nh * d), torch.empty(rows, nh * d, dtype=dtype, device="cuda")
+
+    def run(lo, hi, window):
+        kernels.attention_rows(q[lo:hi], out[:hi - lo], dev(case["cache"]), dev(case["positions"][lo:hi]),
+                               dev(case["seq_of_row"][lo:hi]), dev(case["table"]), nh, 2, d, page_size, window, d ** -0.5)
+        return out[:hi - lo].clone()
+
+    for window in (0, 45):
+        many = run(0, rows, window)
+        for lo, hi in ((0, 1), (100, 133), (rows - 5, rows)):
+            assert torch.equal(run(lo, hi, window), many[lo:hi])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window", [0, 1, 24, 100])
 def test_attention_rows_at_the_edges_of_what_a_row_sees(dtype, window):
     """Scores that rise by 8 with every key (the position as 16 * hi + lo in two dimensions, exact in bfloat16 too) give
