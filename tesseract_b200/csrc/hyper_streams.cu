@@ -27,15 +27,23 @@ struct Streams {
 };
 
 // S > 0: that many copies, their packets in registers; S == 0: any number up to kMaxStreams, one column a thread at a time.
+// Bound by the chain of a launch where rows are few, by the copies' bytes where they are many: a thread asks for two packets of
+// every copy before it stores one, and for the norm's weights before the wait.  Four copies of 2,048 numbers at 8 / 32 / 2,048 rows:
+// 2.4 / 2.6 / 23.8 us, with a packet after another 3.0 / 3.2 / 26.9.  (The residual is not __restrict__: its loads stay behind the wait.)
 template <typename T, int S>
-__global__ void __launch_bounds__(kThreads)
-mixed_streams_norm_kernel(float* __restrict__ residual, T* __restrict__ out, Streams p) {
+__global__ void __launch_bounds__(kThreads, S == 3 || S == 4 ? 2 : 1)
+mixed_streams_norm_kernel(float* residual, T* out, Streams p) {
     __shared__ float scratch[32];
     pdl_trigger();
     const int W = p.width;
     constexpr int C = S > 0 ? S : 1;
     float mix[C][C], share[C], take[C];
+    float4 weight[2];
     if (S > 0) {                                      // (weights: not written by any kernel in front)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+            if (out != nullptr && n * kThreads + threadIdx.x < W / 4)
+                weight[n] = *reinterpret_cast<const float4*>(p.weight + (n * kThreads + threadIdx.x) * 4);
 #pragma unroll
         for (int t = 0; t < C; ++t) {
             share[t] = p.share != nullptr ? p.share[t] : 0.0f;
@@ -54,15 +62,20 @@ mixed_streams_norm_kernel(float* __restrict__ residual, T* __restrict__ out, Str
     if constexpr (S > 0) {
         float4 kept[kKeep];
         const int packets = W / 4;
-        auto column = [&](int i) {                    // the new copies of columns i .. i + 3 are stored; what the next sublayer reads comes back
-            float4 x[S];
+        struct Column { float4 x[S], y, z; };
+        auto ask = [&](int i, Column& c) {            // everything that columns i .. i + 3 need
 #pragma unroll
-            for (int s = 0; s < S; ++s) x[s] = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
+            for (int s = 0; s < S; ++s) c.x[s] = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
+            if (ua != nullptr) c.y = *reinterpret_cast<const float4*>(ua + i);
+            if (ub != nullptr) c.z = *reinterpret_cast<const float4*>(ub + i);
+        };
+        auto renew = [&](int i, Column& c) {          // the new copies are stored; what the next sublayer reads comes back
+            float4 (&x)[S] = c.x;
             if (ua != nullptr) {
-                float4 y = *reinterpret_cast<const float4*>(ua + i);
+                float4 y = c.y;
                 y.x *= p.scale_a; y.y *= p.scale_a; y.z *= p.scale_a; y.w *= p.scale_a;
                 if (ub != nullptr) {
-                    const float4 z = *reinterpret_cast<const float4*>(ub + i);
+                    const float4 z = c.z;
                     y.x = fmaf(p.scale_b, z.x, y.x); y.y = fmaf(p.scale_b, z.y, y.y);
                     y.z = fmaf(p.scale_b, z.z, y.z); y.w = fmaf(p.scale_b, z.w, y.w);
                 }
@@ -101,19 +114,32 @@ mixed_streams_norm_kernel(float* __restrict__ residual, T* __restrict__ out, Str
         auto square = [&](const float4& u) {
             ss = fmaf(u.x, u.x, ss); ss = fmaf(u.y, u.y, ss); ss = fmaf(u.z, u.z, ss); ss = fmaf(u.w, u.w, ss);
         };
+        // Two packets of the row asked for at a time: a store in between would hold back the next one's loads.  (One or two copies
+        // keep to one: their rows are short, and with the registers of a second 2,048 rows of two copies take 12.2 us, not 10.9.)
+        constexpr int ASK = S >= 3 ? 2 : 1;
 #pragma unroll
-        for (int n = 0; n < kKeep; ++n) {
-            const int q = n * kThreads + threadIdx.x;
-            if (q < packets) {
-                kept[n] = column(q * 4);
-                square(kept[n]);
+        for (int n0 = 0; n0 < kKeep; n0 += ASK) {
+            Column c[ASK];
+#pragma unroll
+            for (int n = 0; n < ASK; ++n)
+                if ((n0 + n) * kThreads + threadIdx.x < packets) ask(((n0 + n) * kThreads + threadIdx.x) * 4, c[n]);
+#pragma unroll
+            for (int n = 0; n < ASK; ++n) {
+                const int q = (n0 + n) * kThreads + threadIdx.x;
+                if (q < packets) {
+                    kept[n0 + n] = renew(q * 4, c[n]);
+                    square(kept[n0 + n]);
+                }
             }
         }
-        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) square(column(q * 4));
+        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) {
+            Column c;
+            ask(q * 4, c);
+            square(renew(q * 4, c));
+        }
         if (to == nullptr) return;
         const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)W + p.eps);
-        auto finish = [&](int i, const float4& u) {
-            const float4 w = *reinterpret_cast<const float4*>(p.weight + i);
+        auto finish = [&](int i, const float4& u, const float4& w) {
             const float v[4] = {u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w};
             if constexpr (sizeof(T) == 4) {
                 *reinterpret_cast<float4*>(to + i) = make_float4(v[0], v[1], v[2], v[3]);
@@ -125,9 +151,10 @@ mixed_streams_norm_kernel(float* __restrict__ residual, T* __restrict__ out, Str
 #pragma unroll
         for (int n = 0; n < kKeep; ++n) {
             const int q = n * kThreads + threadIdx.x;
-            if (q < packets) finish(q * 4, kept[n]);
+            if (q < packets) finish(q * 4, kept[n], n < 2 ? weight[n & 1] : *reinterpret_cast<const float4*>(p.weight + q * 4));
         }
-        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) finish(q * 4, again(q * 4));
+        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads)
+            finish(q * 4, again(q * 4), *reinterpret_cast<const float4*>(p.weight + q * 4));
     } else {
         const int N = p.streams;
         for (int i = threadIdx.x; i < W; i += kThreads) {
