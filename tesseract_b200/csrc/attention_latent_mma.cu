@@ -264,6 +264,218 @@ attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
     }
 }
 
+// Prompt rows over vectors so long that one block of four warps takes a multiprocessor's shared memory: ROWS neighbouring rows a
+// block, four warps each, over one copy of the keys.  Neighbouring rows of a sequence see windows that are one key apart, so a
+// stage holds ROWS - 1 keys more than a tile and every row walks its own tiles at its own offset: the work of a row is that of
+// the kernel above, to the bit.  Rows of different sequences that meet in a block are walked one run after the other.
+// Bound by the latency of a tile's chain of products, softmax and barriers, which the rows of a block hide from one another:
+// 2,000 rows of 16 heads over vectors of 576 under a window of 512 take 247 us, 476 with a block a row.
+template <int D, int DV, int ROWS>
+struct SharedLayout {
+    static constexpr int KS = D * 2 + 16;
+    static constexpr int PS = KT * 2 + 16;
+    static constexpr int KEYS = KT + ROWS - 1;
+    static constexpr int STAGE = KEYS * KS;
+    static constexpr int Q_AT = 2 * STAGE;
+    static constexpr int P_AT = Q_AT + ROWS * 16 * KS;             // per row: hi, then lo
+    static constexpr int STAT_AT = P_AT + ROWS * 2 * 16 * PS;
+    static constexpr int BYTES = STAT_AT + ROWS * 4 * 16 * 4;
+};
+
+template <int D, int DV, int ROWS>
+__global__ void __launch_bounds__(ROWS * 128)
+attention_latent_shared_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache,
+                               const int* positions, const int* seq_of_row, const int* block_table, int bt_stride, int rows,
+                               int heads, int page_size, int mask_kind, int mask_size, float scale) {
+    typedef SharedLayout<D, DV, ROWS> L;
+    constexpr int KS = L::KS, PS = L::PS;
+    constexpr int COLS = DV / 4;
+    extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
+    pdl_wait();
+    const int own = threadIdx.x / 128, tid = threadIdx.x % 128, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int row0 = blockIdx.x * ROWS, n = min(ROWS, rows - row0), head0 = blockIdx.y * 16;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t q_at = base + L::Q_AT + own * 16 * KS;
+    unsigned char* p_smem = smem + L::P_AT + own * 2 * 16 * PS;
+    const uint32_t p_base = base + L::P_AT + own * 2 * 16 * PS;
+    float* stats = reinterpret_cast<float*>(smem + L::STAT_AT) + own * 64;
+    auto row_barrier = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(own + 1) : "memory"); };
+    const int row = row0 + own;
+    if (own < n)
+        for (int index = tid; index < 16 * (D / 8); index += 128) {
+            const int h = index / (D / 8), chunk = index % (D / 8);
+            const bool there = head0 + h < heads;
+            const bf16* src = q + (int64_t)row * q_stride + (int64_t)(there ? head0 + h : head0) * D + chunk * 8;
+            cp_async16(q_at + h * KS + chunk * 16, src, there ? 16 : 0);
+        }
+    const int64_t page_elems = (int64_t)page_size * D;
+    auto first_key = [&](int pos) { return (mask_kind == MASK_WINDOW && pos - mask_size + 1 > 0) ? pos - mask_size + 1 : 0; };
+
+    for (int begin = 0; begin < n;) {
+        const int seq = seq_of_row[row0 + begin], pos_first = positions[row0 + begin];
+        int count = 1;
+        while (begin + count < n && seq_of_row[row0 + begin + count] == seq && positions[row0 + begin + count] == pos_first + count)
+            ++count;
+        const int pos_last = pos_first + count - 1, block_lo = first_key(pos_first);
+        const bool mine = own >= begin && own < begin + count;
+        const int pos = pos_first + (mine ? own - begin : 0);
+        const int key_lo = first_key(pos), shift = key_lo - block_lo;      // 0 .. ROWS - 1
+        const int own_tiles = mine ? (pos - key_lo) / KT + 1 : 0;
+        const int tiles = max((pos_last - first_key(pos_last)) / KT, (pos_last - block_lo - (count - 1)) / KT) + 1;
+        const int* table = block_table + (int64_t)seq * bt_stride;
+        auto fill = [&](int tile) {                                        // a warp a key
+            const uint32_t stage = base + (uint32_t)(tile & 1) * L::STAGE;
+            for (int k = threadIdx.x >> 5; k < L::KEYS; k += ROWS * 4) {
+                const int key = block_lo + tile * KT + k;
+                const bool there = key <= pos_last;
+                const int from = there ? key : pos_last;
+                const bf16* kp = cache + (int64_t)table[from / page_size] * page_elems + (int64_t)(from % page_size) * D;
+                for (int chunk = lane; chunk < D / 8; chunk += 32) cp_async16(stage + k * KS + chunk * 16, kp + chunk * 8, there ? 16 : 0);
+            }
+        };
+        fill(0);
+        cp_async_commit();
+
+        float m[2] = {-1.0e30f, -1.0e30f}, l[2] = {0.0f, 0.0f};
+        float o[COLS / 8][4];
+#pragma unroll
+        for (int j = 0; j < COLS / 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[j][e] = 0.0f;
+
+        for (int tile = 0; tile < tiles; ++tile) {
+            if (tile + 1 < tiles) {
+                fill(tile + 1);
+                cp_async_commit();
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
+            }
+            __syncthreads();                                          // this tile's keys (and the queries) are in shared memory
+            if (tile < own_tiles) {
+                const uint32_t stage = base + (uint32_t)(tile & 1) * L::STAGE + shift * KS;
+                const int key0 = key_lo + tile * KT + warp * 16;      // the warp's 16 keys of the row's tile
+                float s[2][4];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[j][e] = 0.0f;
+                if (key0 <= pos) {
+#pragma unroll 4
+                    for (int ks = 0; ks < D / 16; ++ks) {
+                        uint32_t a[4], b[4];
+                        ldmatrix_x4(a, q_at + (lane & 15) * KS + (ks * 2 + (lane >> 4)) * 16);
+                        ldmatrix_x4(b, stage + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * KS + (ks * 2 + ((lane >> 3) & 1)) * 16);
+                        mma_bf16_16816(s[0], a, b);
+                        mma_bf16_16816(s[1], a, b + 2);
+                    }
+                }
+                float top[2] = {-1.0e30f, -1.0e30f};
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int key = key0 + j * 8 + 2 * t + (e & 1);
+                        s[j][e] = key <= pos ? s[j][e] * scale : -1.0e30f;
+                        top[e >> 1] = fmaxf(top[e >> 1], s[j][e]);
+                    }
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
+                    top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
+                    if (t == 0) stats[warp * 16 + g + r * 8] = top[r];
+                }
+                row_barrier();                                        // the row's four warps' maxima of the tile
+                float corr[2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float all = stats[g + r * 8];
+#pragma unroll
+                    for (int w = 1; w < 4; ++w) all = fmaxf(all, stats[w * 16 + g + r * 8]);
+                    const float m_new = fmaxf(m[r], all);
+                    corr[r] = __expf(m[r] - m_new);
+                    m[r] = m_new;
+                    l[r] *= corr[r];
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float p = s[j][e] > -1.0e29f ? __expf(s[j][e] - m[e >> 1]) : 0.0f;
+                        s[j][e] = p;
+                        l[e >> 1] += p;
+                    }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        uint32_t hi, lo;
+                        split_bf16(s[j][2 * r], s[j][2 * r + 1], hi, lo);
+                        const uint32_t at = (g + r * 8) * PS + (warp * 16 + j * 8 + 2 * t) * 2;
+                        *reinterpret_cast<uint32_t*>(p_smem + at) = hi;
+                        *reinterpret_cast<uint32_t*>(p_smem + 16 * PS + at) = lo;
+                    }
+#pragma unroll
+                for (int j = 0; j < COLS / 8; ++j) {
+                    o[j][0] *= corr[0]; o[j][1] *= corr[0];
+                    o[j][2] *= corr[1]; o[j][3] *= corr[1];
+                }
+                row_barrier();                                        // all 64 keys' weights are in shared memory
+#pragma unroll
+                for (int kk = 0; kk < KT / 16; ++kk) {
+                    const int keys_left = pos - (key_lo + tile * KT + kk * 16);
+                    if (keys_left < 0) break;                         // (keys behind the row's position: weights of zero)
+                    // values behind the row's position belong to later rows: they count as zeros, whatever they are
+                    uint32_t keep[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        keep[h] = (2 * t + h * 8 <= keys_left ? 0xffffu : 0u) | (2 * t + h * 8 + 1 <= keys_left ? 0xffff0000u : 0u);
+                    uint32_t hi[4], lo[4];
+                    const uint32_t p_at = p_base + (lane & 15) * PS + (kk * 2 + (lane >> 4)) * 16;
+                    ldmatrix_x4(hi, p_at);
+                    ldmatrix_x4(lo, p_at + 16 * PS);
+#pragma unroll
+                    for (int jp = 0; jp < COLS / 16; ++jp) {
+                        uint32_t b[4];
+                        ldmatrix_x4_trans(b, stage + (kk * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * KS +
+                                                 (warp * (COLS / 8) + jp * 2 + (lane >> 4)) * 16);
+                        b[0] &= keep[0]; b[1] &= keep[1]; b[2] &= keep[0]; b[3] &= keep[1];
+                        mma_bf16_16816(o[2 * jp], hi, b);
+                        mma_bf16_16816(o[2 * jp], lo, b);
+                        mma_bf16_16816(o[2 * jp + 1], hi, b + 2);
+                        mma_bf16_16816(o[2 * jp + 1], lo, b + 2);
+                    }
+                }
+            }
+            __syncthreads();                                          // the stage and the weights may be written again
+        }
+        if (mine) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+                l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+                if (t == 0) stats[warp * 16 + g + r * 8] = l[r];
+            }
+            row_barrier();
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int head = head0 + g + r * 8;
+                if (head >= heads) continue;
+                float total = 0.0f;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) total += stats[w * 16 + g + r * 8];
+                const float inv = 1.0f / fmaxf(total, 1.0e-30f);
+                bf16* orow = out + (int64_t)row * out_stride + (int64_t)head * DV + warp * COLS;
+#pragma unroll
+                for (int j = 0; j < COLS / 8; ++j)
+                    *reinterpret_cast<uint32_t*>(orow + j * 8 + 2 * t) = pack_bf16(o[j][2 * r] * inv, o[j][2 * r + 1] * inv);
+            }
+        }
+        begin += count;
+    }
+}
+
 // The runs of a row and head, added in order: out = sum_z o_z e^(m_z - M) / sum_z l_z e^(m_z - M), M the largest m_z.
 // Bound by the latency of its loads: a lane takes one run's maximum and sum, and a thread asks for two columns of every run
 // before it adds (8 rows of 16 heads and 16 runs in a decode
@@ -314,13 +526,29 @@ int splits_for(int rows, int heads) {
 
 template <int D, int DV>
 int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache, const int* positions,
-           const int* seq_of_row, const int* block_table, int bt_stride, int rows, int heads, int page_size, int mask_kind,
+           const int* seq_of_row, const int* block_table, int bt_stride, int rows, int num_seqs, int heads, int page_size, int mask_kind,
            int mask_size, float scale, float* parts, cudaStream_t stream) {
     constexpr int smem = Layout<D, DV>::BYTES;
     auto kernel = attention_latent_kernel<D, DV>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return (int)err;
     const int splits = splits_for(rows, heads);
+    // Rows share where a block a row leaves a multiprocessor with four warps (not so at 288 and 160 numbers a vector), where they
+    // still fill the chip in threes (two rows a block: 316 us for the 2,000 rows above), and where most of a block's rows
+    // belong to one sequence: 448 decoded rows of as many take 126 us in threes, 100 alone.
+    constexpr int kShared = 3;
+    if constexpr (D == 576) {
+        if ((int64_t)rows * ((heads + 15) / 16) >= 148 * kShared && rows >= 8 * num_seqs) {
+            constexpr int bytes = SharedLayout<D, DV, kShared>::BYTES;
+            auto shared = attention_latent_shared_kernel<D, DV, kShared>;
+            cudaError_t err = cudaFuncSetAttribute(shared, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (err == cudaSuccess)
+                err = tb_launch_pdl(shared, dim3((rows + kShared - 1) / kShared, (heads + 15) / 16), dim3(kShared * 128), (size_t)bytes,
+                                    stream, (const bf16*)q, q_stride, (bf16*)out, out_stride, (const bf16*)cache, positions, seq_of_row,
+                                    block_table, bt_stride, rows, heads, page_size, mask_kind, mask_size, scale);
+            return err == cudaSuccess ? tb_launch_status() : (int)err;
+        }
+    }
     if (splits > 1 && parts == nullptr) return TB_ERR_BAD_SIZE;
     if (splits > 1 && (uintptr_t)parts % 8 != 0) return TB_ERR_BAD_ALIGN;
     cudaError_t launched = tb_launch_pdl(kernel, dim3(rows, (heads + 15) / 16, splits), dim3(128), (size_t)smem, stream,
@@ -349,12 +577,13 @@ TB_EXPORT int tb_attention_latent_mma_splits(int rows, int heads) {
 }
 
 // q: bfloat16 [rows, heads * dim] (row stride q_stride, elements); out: bfloat16 [rows, heads * vdim]; cache: this
-// layer's pages ([page_size][dim] a page); positions, seq_of_row: int32 [rows]; mask_kind: 0 causal, 1 window; parts:
+// layer's pages ([page_size][dim] a page); positions, seq_of_row: int32 [rows]; num_seqs: the sequences that the
+// rows belong to (it picks the kernel only); mask_kind: 0 causal, 1 window; parts:
 // float32 [rows, splits, heads, vdim + 2] of scratch where tb_attention_latent_mma_splits says more than 1.
 TB_EXPORT int tb_attention_latent_mma(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
                                       const int* positions, const int* seq_of_row, const int* block_table, int bt_stride,
-                                      int rows, int heads, int dim, int vdim, int page_size, int mask_kind, int mask_size,
-                                      float scale, float* parts, cudaStream_t stream) {
+                                      int rows, int num_seqs, int heads, int dim, int vdim, int page_size, int mask_kind,
+                                      int mask_size, float scale, float* parts, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (!tb_attention_latent_mma_supported(dim, vdim)) return TB_ERR_BAD_SIZE;
     if (heads < 1 || (heads + 15) / 16 > 65535 || page_size < 1) return TB_ERR_BAD_SIZE;
@@ -364,7 +593,7 @@ TB_EXPORT int tb_attention_latent_mma(const void* q, int64_t q_stride, void* out
         return TB_ERR_BAD_ALIGN;
 #define TB_ATTEND(D, DV)                                                                                             \
     return launch<D, DV>(q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride, rows,   \
-                         heads, page_size, mask_kind, mask_size, scale, parts, stream)
+                         num_seqs, heads, page_size, mask_kind, mask_size, scale, parts, stream)
     if (dim == 576) TB_ATTEND(576, 512);
     if (dim == 288) TB_ATTEND(288, 256);
     TB_ATTEND(160, 128);

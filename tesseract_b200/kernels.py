@@ -1711,8 +1711,8 @@ def attention_latent_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
                          seq_of_row: torch.Tensor, block_table: torch.Tensor, *, heads: int, dim: int, vdim: int,
                          page_size: int, mask_kind: int, mask_size: int, scale: float) -> torch.Tensor:
     """:func:`attention_masked` with ``kv_heads = 1`` and ``keys_per_value = 0`` (pages of ``[page_size, dim]`` vectors
-    whose first ``vdim`` numbers are the value) on the tensor cores, for bfloat16: a block a row and sixteen query heads;
-    exact bfloat16 products with 32-bit accumulation for the scores, 32-bit softmax, the weights as two bfloat16 halves.
+    whose first ``vdim`` numbers are the value) on the tensor cores, for bfloat16: a block a row (in portions of many
+    rows three neighbouring rows) and sixteen query heads; exact bfloat16 products with 32-bit accumulation for the scores, 32-bit softmax, the weights as two bfloat16 halves.
     In a step of few rows every row's keys are shared out among several blocks, and a second kernel adds their results."""
     _cuda(q, out, cache, positions, seq_of_row, block_table)
     rows = q.shape[0]
@@ -1726,8 +1726,8 @@ def attention_latent_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
     parts = torch.empty((rows, splits, heads, vdim + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     _check(lib.tb_attention_latent_mma(_ptr(q), _i64(q.stride(0)), _ptr(out), _i64(out.stride(0)), _ptr(cache),
                                        _ptr(positions), _ptr(seq_of_row), _ptr(block_table), _i32(block_table.stride(0)),
-                                       _i32(rows), _i32(heads), _i32(dim), _i32(vdim), _i32(page_size), _i32(mask_kind),
-                                       _i32(mask_size), _f32(scale), _ptr(parts), _stream()), "attention_latent_mma")
+                                       _i32(rows), _i32(block_table.shape[0]), _i32(heads), _i32(dim), _i32(vdim), _i32(page_size),
+                                       _i32(mask_kind), _i32(mask_size), _f32(scale), _ptr(parts), _stream()), "attention_latent_mma")
     if splits > 1:
         global launch_count
         launch_count += 1          # (the kernel that adds the runs up)

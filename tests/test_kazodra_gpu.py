@@ -533,6 +533,44 @@ def test_latent_runs_of_a_decoded_row_are_added_up(dim, vdim, rows, heads, windo
         close(out[t], (weights @ keys[:, :vdim]).reshape(-1), TOL[torch.bfloat16], f"row {t}")
 
 
+@pytest.mark.parametrize("heads", [16, 20])
+@pytest.mark.parametrize("window", [None, 512, 70, 1])
+def test_latent_rows_that_share_their_keys_keep_their_bits(heads, window):
+    """Steps of many rows take three rows a block: portions that begin and end inside a block, sequences of one row, rows at a
+    window's first steps, a last block of fewer rows, and a later key that is not finite, against steps that take a block a row."""
+    from tesseract_b200 import kernels
+
+    dim, vdim, page = 576, 512, 16
+    spans = [(0, 100), (3, 101), (700, 1), (0, 1), (505, 130), (9, 2), (62, 117)]      # (first position, rows)
+    g = torch.Generator().manual_seed(heads)
+    width = max(-(-(first + n) // page) for first, n in spans)
+    table = torch.arange(len(spans) * width, dtype=torch.int32).reshape(len(spans), width).flip(1).contiguous()
+    cache = torch.randn(table.numel(), page, dim, generator=g).to(torch.bfloat16)
+    last = spans[0][1] - 1
+    cache[table[0, last // page], last % page] = float("nan")                          # only the first sequence's last row may see it
+    rows = sum(n for _, n in spans)
+    q = (torch.randn(rows, heads * dim, generator=g) * 0.5).to(torch.bfloat16).to(dev())
+    positions = torch.tensor([first + t for first, n in spans for t in range(n)], dtype=torch.int32, device=dev())
+    of_row = torch.tensor([s for s, (_, n) in enumerate(spans) for _ in range(n)], dtype=torch.int32, device=dev())
+    cache, table = cache.to(dev()), table.to(dev())
+
+    def run(lo, hi):
+        out = torch.zeros(hi - lo, heads * vdim, dtype=torch.bfloat16, device=dev())
+        kernels.attention_latent_mma(q[lo:hi], out, cache, positions[lo:hi], of_row[lo:hi], table, heads=heads, dim=dim, vdim=vdim,
+                                     page_size=page, scale=dim ** -0.5, mask_kind=kernels.MASK_WINDOW if window else kernels.MASK_CAUSAL,
+                                     mask_size=window or 0)
+        return out
+
+    per_row = -(-heads // 16)
+    assert rows * per_row >= 444 and 148 <= 200 * per_row < 444
+    got = run(0, rows)
+    parts = torch.cat([run(max(0, min(at, rows - 200)), min(at + 200, rows))[-(min(at + 200, rows) - at):] for at in range(0, rows, 200)])
+    same = (got == parts).all(dim=1)
+    same[last] = bool(torch.isnan(got[last]).all())
+    assert bool(same.all()), same.logical_not().nonzero().flatten().tolist()
+    assert bool(torch.isfinite(got[torch.arange(rows, device=dev()) != last]).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,d,dr,dv,rank", [(3, 12, 8, 10, 20), (2, 16, 4, 24, 12), (1, 10, 6, 14, 9), (4, 8, 0, 4, 8),
                                                 (2, 64, 32, 128, 48), (2, 128, 64, 128, 192), (2, 16, 32, 24, 128),
