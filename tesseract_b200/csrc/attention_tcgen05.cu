@@ -8,6 +8,7 @@
 //                      accumulator in tensor memory (128 columns)
 //   softmax            four warps, one thread per row: tcgen05.ld of the row, scale, mask, running maximum,
 //                      2^x, 32-bit row sum, probabilities rounded to bfloat16 into a swizzled P tile in shared memory
+//                      (blocks of 64 keys: into tensor memory, in two buffers, from where the product takes them)
 //                      (a block that needs no mask is read once, against the maximum that earlier blocks left; the
 //                      row is read twice, maximum first, only where that maximum is exceeded by more than 2^8)
 //   O += P . V         tcgen05.mma, M128 x N64 x K128, P K-major, V MN-major (the cache's [key][dim] rows as they
@@ -40,11 +41,14 @@ constexpr uint32_t kTileBytes = BM * 128;
 template <int D, int BN>
 struct Shape {
     static constexpr uint32_t kQBytes = (D / 64) * kTileBytes;
-    static constexpr int kPTiles = BN / 64;
+    // blocks of 64 keys: the probabilities go to tensor memory, in two buffers of BN / 2 columns behind O, and are the first operand
+    // of P . V from there
+    static constexpr bool kPInTmem = BN == 64;
+    static constexpr int kPTiles = kPInTmem ? 0 : BN / 64;
     static constexpr uint32_t kKVHalfBytes = BN * 128;               // one 64-dim slice of a K or V block
     static constexpr uint32_t kKVTileBytes = (D / 64) * kKVHalfBytes;   // one K or V block
-    static constexpr int kCtasPerSm = D == 64 && BN == 64 ? 3 : 2;
-    static constexpr uint32_t kTmemColumns = BN + D <= 128 ? 128 : 256;   // S: columns 0..BN-1, O: the D columns after them
+    static constexpr int kCtasPerSm = 2;
+    static constexpr uint32_t kTmemColumns = 256;   // S: columns 0..BN-1, O: the D columns after them
     static constexpr size_t kSmemBytes = (size_t)kQBytes + (size_t)kPTiles * kTileBytes + (size_t)2 * STAGES * kKVTileBytes;
 };
 constexpr float kLog2e = 1.4426950408889634f;
@@ -109,6 +113,14 @@ __device__ __forceinline__ void umma_add(uint32_t tmem_d, uint64_t desc_a, uint6
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc) : "memory");
 }
+// D (+)= A . B with A in tensor memory (a row a lane, two neighbouring bfloat16 a column)
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc) : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -127,6 +139,13 @@ __device__ __forceinline__ void tmem_load_32(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_store_16_nowait(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_load_32_nowait(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -222,11 +241,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
     constexpr uint32_t kKVTileBytes = Tiles::kKVTileBytes, kKVHalfBytes = Tiles::kKVHalfBytes;
     constexpr uint32_t kTmemColumns = Tiles::kTmemColumns;
     constexpr int kPTiles = Tiles::kPTiles;
+    constexpr bool kPInTmem = Tiles::kPInTmem;
+    static_assert(!kPInTmem || BN + D + BN <= (int)kTmemColumns, "S, O and two P buffers in the tensor memory of a CTA");
     extern __shared__ __align__(1024) unsigned char smem[];   // the swizzled tiles need 1024-byte alignment
-    // barriers: k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES], s_full, p_ready, o_full, s_free.
+    // barriers: k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES], s_full, s_free, p_ready[2], o_full[2] (with one
+    // buffer of P the first of each alone; with two, block j's are those of buffer j & 1, so that no phase is ever two ahead
+    // of the one that is waited for).
     // Keys and values have rings of their own: a key block's stage is free again as soon as its scores are
     // computed, a whole block before its value stage is.
-    __shared__ __align__(8) uint64_t bars[4 * STAGES + 4];
+    __shared__ __align__(8) uint64_t bars[4 * STAGES + 6];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
     __shared__ int last_to_arrive;
@@ -258,8 +281,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
     const uint32_t kv_tiles = p_tile + kPTiles * kTileBytes;    // [stage][K | V]
     const uint32_t k_full = smem_u32(&bars[0]), k_empty = smem_u32(&bars[STAGES]);
     const uint32_t v_full = smem_u32(&bars[2 * STAGES]), v_empty = smem_u32(&bars[3 * STAGES]);
-    const uint32_t s_full = smem_u32(&bars[4 * STAGES]), p_ready = s_full + 8, o_full = s_full + 16;
-    const uint32_t s_free = s_full + 24;
+    const uint32_t s_full = smem_u32(&bars[4 * STAGES]), s_free = s_full + 8;
+    constexpr int kPBuffers = kPInTmem ? 2 : 1;
+    auto p_ready = [&](int j) { return s_full + 16 + 8 * (j % kPBuffers); };    // P of block j is written
+    auto o_full = [&](int j) { return s_full + 32 + 8 * (j % kPBuffers); };     // P_j V_j is done
+    auto phase = [&](int j) { return (uint32_t)(j / kPBuffers) & 1u; };
 
     const int last_row = min(n_rows, r0 + BM) - 1;
     const int key_hi = begin + last_row / p.group;
@@ -282,8 +308,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             mbar_init(v_empty + 8 * s, 1);
         }
         mbar_init(s_full, 1);
-        mbar_init(p_ready, BM);
-        mbar_init(o_full, 1);
+        for (int b = 0; b < kPBuffers; ++b) {
+            mbar_init(p_ready(b), BM);
+            mbar_init(o_full(b), 1);
+        }
         mbar_init(s_free, BM);
         mbar_fence_init();
     }
@@ -321,6 +349,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
     }
     const uint32_t tmem_base = tmem_base_slot;
     const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + BN;
+    auto tmem_p = [&](int j) { return tmem_o + D + (j & 1) * (BN / 2); };
 
     if (warp == 5) {
         // ------------------------------------------------------------ TMA producer: K and V blocks, page by page
@@ -410,17 +439,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                 }
                 // P_j is in shared memory (and O has been rescaled if the maximum jumped): O += P_j V_j
                 if (!mbar_wait(v_full + 8 * s, parity, &abort_flag)) { ok = false; break; }
-                if (!mbar_wait(p_ready, j & 1, &abort_flag)) { ok = false; break; }
+                if (!mbar_wait(p_ready(j), phase(j), &abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t v_desc = v_desc0 + (uint32_t)s * kStageStep;
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
+                    if constexpr (kPInTmem) {
+                        umma_ts(tmem_o, tmem_p(j) + kk * 8, v_desc + ((kk * 2048) >> 4), idesc_pv, kk != 0 || j != 0);
+                        continue;
+                    }
                     const uint64_t a = p_desc + (((kk >> 2) * kTileBytes + (kk & 3) * 32) >> 4);
                     const uint64_t b = v_desc + ((kk * 2048) >> 4);
                     if (kk == 0) umma(tmem_o, a, b, idesc_pv, j != 0);
                     else umma_add(tmem_o, a, b, idesc_pv);
                 }
-                umma_commit(o_full);
+                umma_commit(o_full(j));
                 umma_commit(v_empty + 8 * s);
                 if (++s == STAGES) { s = 0; parity ^= 1; }
             }
@@ -446,7 +479,152 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
         // by more than 2^8, which keeps every probability at or below 256 and makes the rescaling rare.
         float m = kMasked, l = 0.0f;
         bool ok = true;
-        for (int j = 0; j < n_blocks; ++j) {
+        // Blocks of 64 keys: a row's scores all fit in registers, so S is handed back as soon as they are read and the next
+        // block's are computed under this block's softmax; P goes to tensor memory, which leaves shared memory's bandwidth to
+        // the products' operands and lets a block's probabilities be stored while the product before still reads its own.
+        // 2,048 rows of 32 heads of 128 at context 12,345: 389 us (975 TFLOP/s), 412 with P in shared memory and S kept until
+        // the maximum is known; 57 rows there, eight CTAs a tile: 78 and 113; 512 rows at 8,704, two: 99 and 114.
+        for (int j = 0; kPInTmem && j < n_blocks; ++j) {
+            const int key0 = (kb_first + j) * BN;
+            if (!mbar_wait(s_full, j & 1, &abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t sc[2][32];
+            bool freed = false;
+            tmem_load_32_nowait(tmem_s + lane_base, sc[0]);
+            tmem_wait_ld();
+            tmem_load_32_nowait(tmem_s + lane_base + 32, sc[1]);
+            if (j > 0 && all_rows && p.window <= 0 && key0 + BN - 1 <= warp_lo_pos) {       // uniform across the warp
+                // One pass for a block that needs no mask, against the maximum that earlier blocks left, while the block's own is
+                // followed on the side: the first chunk's exponentials run under the second's load.  Only if that maximum is
+                // exceeded by more than 2^8 in some row of the warp (rare) is the work thrown away and done again below.
+                float mx[4] = {kMasked, kMasked, kMasked, kMasked};
+                uint64_t ls[4] = {0, 0, 0, 0};
+                const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), neg_m2 = pack2(-m, -m);
+                uint32_t packed[16];
+                auto maxima = [&](const uint32_t (&chunk)[32]) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2)
+                        mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], __uint_as_float(chunk[i]), __uint_as_float(chunk[i + 1]));
+                };
+                auto exps = [&](const uint32_t (&chunk)[32]) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float t0, t1;
+                        unpack2(fma2(pack2(__uint_as_float(chunk[i]), __uint_as_float(chunk[i + 1])), scale2, neg_m2), t0, t1);
+                        const float p0 = fast_exp2(t0), p1 = fast_exp2(t1);
+                        ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
+                        packed[i >> 1] = pack_bf16(p0, p1);
+                    }
+                };
+                maxima(sc[0]);
+                exps(sc[0]);
+                tmem_wait_ld();
+                tc_fence_before();
+                mbar_arrive(s_free);                   // (both chunks are in registers)
+                freed = true;
+                // P_{j-2} V_{j-2} has read this buffer
+                if (j >= kPBuffers && !mbar_wait(o_full(j - kPBuffers), phase(j - kPBuffers), &abort_flag)) { ok = false; break; }
+                tmem_store_16_nowait(tmem_p(j) + lane_base, packed);
+                maxima(sc[1]);
+                const float seen = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+                if (!__any_sync(0xffffffffu, seen > m + 8.0f)) {
+                    exps(sc[1]);
+                    tmem_store_16_nowait(tmem_p(j) + lane_base + 16, packed);
+                    float lo_sum, hi_sum;
+                    unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), lo_sum, hi_sum);
+                    l += lo_sum + hi_sum;
+                    tmem_wait_st();
+                    tc_fence_before();
+                    mbar_arrive(p_ready(j));
+                    continue;
+                }
+            }
+            // Any block: all of a row's scores in registers, their maximum first.
+            if (!freed) {
+                tmem_wait_ld();
+                tc_fence_before();
+                mbar_arrive(s_free);                   // S has been read: the issuer may start the next block's scores
+            }
+            // A warp's rows are a few neighbouring positions: of the blocks on the diagonal (and at a window's start) most chunks
+            // of 32 keys lie wholly before or wholly behind what they see, and only the others are masked number by number.
+            const int lo_col = lo - key0, hi_col = pos - key0;      // this row sees columns lo_col..hi_col of the block
+            bool dead[2];
+            float mx[4] = {kMasked, kMasked, kMasked, kMasked};
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int first_key = key0 + c * 32, last_key = first_key + 31;
+                dead[c] = all_rows && (first_key > warp_hi_pos || (p.window > 0 && last_key < warp_lo_pos - p.window + 1));
+                const bool open = all_rows && last_key <= warp_lo_pos && (p.window <= 0 || first_key >= warp_hi_pos - p.window + 1);
+                if (dead[c]) continue;                              // (uniform across the warp, as `open` is)
+                if (!open) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (c * 32 + i < lo_col || c * 32 + i > hi_col) sc[c][i] = __float_as_uint(kMasked);
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                    mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], __uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1]));
+            }
+            const float raw_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            const float block_max = raw_max > 0.5f * kMasked ? raw_max * p.scale_log2 : kMasked;
+            const bool jump = block_max > m + 8.0f;
+            if (__any_sync(0xffffffffu, jump)) {
+                if (j > 0 && !mbar_wait(o_full(j - 1), phase(j - 1), &abort_flag)) { ok = false; break; }
+                const float m_new = fmaxf(m, block_max);
+                const float corr = fast_exp2(m - m_new);
+                m = m_new;
+                l *= corr;
+                if (j > 0) {
+                    tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < D / 32; ++c) {
+                        float v[32];
+                        tmem_load_32(tmem_o + lane_base + c * 32, v);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] *= corr;
+                        tmem_store_32(tmem_o + lane_base + c * 32, v);
+                    }
+                }
+            }
+            // (a row that sees no key yet has m = kMasked, and its masked scores must not become 2^0)
+            const float neg_m = m > 0.5f * kMasked ? -m : 0.0f;
+            const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), neg_m2 = pack2(neg_m, neg_m);
+            uint64_t ls[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float p0, p1;
+                    if (dead[c]) {
+                        sc[c][i >> 1] = 0u;
+                        continue;
+                    }
+                    const uint64_t x2 = fma2(pack2(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
+                    constexpr int kEvery = kPolyEvery<D> > 0 ? kPolyEvery<D> : 1;
+                    if (kPolyEvery<D> > 0 && (i >> 1) % kEvery == kEvery - 1) {
+                        exp2_pair_fma(x2, p0, p1);
+                    } else {
+                        float t0, t1;
+                        unpack2(x2, t0, t1);
+                        p0 = fast_exp2(t0);
+                        p1 = fast_exp2(t1);
+                    }
+                    ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
+                    sc[c][i >> 1] = pack_bf16(p0, p1);
+                }
+                // P_{j-2} V_{j-2} has read this buffer
+                if (c == 0 && j >= kPBuffers && !mbar_wait(o_full(j - kPBuffers), phase(j - kPBuffers), &abort_flag)) ok = false;
+                tmem_store_16_nowait(tmem_p(j) + lane_base + c * 16, sc[c]);
+            }
+            if (!ok) break;
+            float lo_sum, hi_sum;
+            unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), lo_sum, hi_sum);
+            l += lo_sum + hi_sum;
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(p_ready(j));
+        }
+        for (int j = 0; !kPInTmem && j < n_blocks; ++j) {
             const int key0 = (kb_first + j) * BN;
             if (!mbar_wait(s_full, j & 1, &abort_flag)) { ok = false; break; }
             tc_fence_after();
@@ -504,7 +682,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                     maxima(cb);
                     exps(cb, held + 16);
                 }
-                if (!mbar_wait(o_full, (j - 1) & 1, &abort_flag)) { ok = false; break; }
+                if (!mbar_wait(o_full(j - 1), phase(j - 1), &abort_flag)) { ok = false; break; }
                 store(held, 0);
                 if (BN == 128) {
                     store(held + 16, 1);
@@ -527,7 +705,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                     l += lo_sum + hi_sum;
                     fence_async_smem();
                     tc_fence_before();
-                    mbar_arrive(p_ready);
+                    mbar_arrive(p_ready(j));
                     continue;
                 }
             }
@@ -588,7 +766,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             const float raw_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             const float block_max = raw_max > 0.5f * kMasked ? raw_max * p.scale_log2 : kMasked;
             // P_{j-1} V_{j-1} must be complete before the P tile is overwritten (and before O is rescaled)
-            if (j > 0 && !mbar_wait(o_full, (j - 1) & 1, &abort_flag)) { ok = false; break; }
+            if (j > 0 && !mbar_wait(o_full(j - 1), phase(j - 1), &abort_flag)) { ok = false; break; }
             const bool jump = block_max > m + 8.0f;
             if (__any_sync(0xffffffffu, jump)) {
                 const float m_new = fmaxf(m, block_max);
@@ -673,9 +851,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             }
             fence_async_smem();
             tc_fence_before();
-            mbar_arrive(p_ready);
+            mbar_arrive(p_ready(j));
         }
-        if (ok && n_blocks > 0 && !mbar_wait(o_full, (n_blocks - 1) & 1, &abort_flag)) ok = false;
+        if (ok && n_blocks > 0 && !mbar_wait(o_full(n_blocks - 1), phase(n_blocks - 1), &abort_flag)) ok = false;
         const int qpos = pos >= 0 ? fr / p.group : 0, g = pos >= 0 ? fr - qpos * p.group : 0;
         __nv_bfloat16* dst = p.out + (int64_t)(first_row + qpos) * p.out_stride + (int64_t)(kv_head * p.group + g) * D;
         if (!SPLIT) {
