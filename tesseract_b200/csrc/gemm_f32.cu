@@ -41,6 +41,34 @@ __device__ __forceinline__ int next_stage(int t, int stages, int K) {
     return t;
 }
 
+// A thread's totals: rows (i / 4) (BM / 2) + 4 ty + i % 4, columns h (BN / 2) + 4 tx .. of its tile.
+template <int BM, int BN, int TN>
+__device__ __forceinline__ void store_tile(const uint64_t (&total)[8][TN / 2], float* C, int64_t ldc, int m0, int n0, int tx, int ty,
+                                           int M, int N) {
+    constexpr int QN = TN / 4;
+    const bool packets = ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + (i / 4) * (BM / 2) + ty * 4 + i % 4;
+        if (m >= M) continue;
+#pragma unroll
+        for (int h = 0; h < QN; ++h) {
+            const int n = n0 + h * (BN / 2) + tx * 4;
+            float* row = C + (int64_t)m * ldc + n;
+            const float2 lo = *reinterpret_cast<const float2*>(&total[i][h * 2]);
+            const float2 hi = *reinterpret_cast<const float2*>(&total[i][h * 2 + 1]);
+            if (packets && n + 4 <= N) {
+                *reinterpret_cast<float4*>(row) = make_float4(lo.x, lo.y, hi.x, hi.y);
+            } else {
+                if (n < N) row[0] = lo.x;
+                if (n + 1 < N) row[1] = lo.y;
+                if (n + 2 < N) row[2] = hi.x;
+                if (n + 3 < N) row[3] = hi.y;
+            }
+        }
+    }
+}
+
 // A thread keeps 8 x TN sums of the current chain and as many totals in registers.  Bound by the loads from shared memory
 // (the path is 76 % busy, the multiply-add pipe 61 %) where the tiles fill the chip, by the latency of a stage where they
 // do not.  500 rows of 16,384 x 2,048 take 799 us (42 TFLOP/s; single-number instructions 12 % more, 64 x 64 tiles of one
@@ -142,27 +170,128 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
         __syncthreads();
         t = ahead;
     }
-    const bool packets = ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
+    store_tile<BM, BN, TN>(total, C, ldc, m0, n0, tx, ty, M, N);
+}
+
+// The tiles where they are too few to give a multiprocessor more than one: G groups of threads take a tile's chains in turn (K a
+// multiple of 256, packets), and the first group adds every round's sums in the order of the chains, the others' through
+// shared memory, so that the bits are those of the kernel above.  Bound by the latency of a group's stages, which the groups hide
+// from one another.   128 x 64
+// tiles of two groups and 64 x 64 tiles of four take 121 and 72 us for K = 2,048 (one group, where a multiprocessor has one tile:
+// 141 and 95).
+template <int BM, int BN, int TN, int G>
+__global__ void __launch_bounds__((BM / 8) * (BN / TN) * G, 1)
+gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K) {
+    constexpr int THREADS = (BM / 8) * (BN / TN), COLS = BN / TN, QN = TN / 4, SUMS = 8 * TN / 4;
+    constexpr int LA = BM * 4 / THREADS, LW = BN * 4 / THREADS;
+    constexpr int AP = BM + 4, WP = BN + 4, STAGE = BK * (AP + WP);
+    extern __shared__ __align__(16) float shared[];
+    const int group = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
+    float* stages_at = shared + group * 2 * STAGE;                                    // [2][As | Ws] of this group
+    float4* given = reinterpret_cast<float4*>(shared + G * 2 * STAGE);                // [G - 1][SUMS][THREADS]
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int tx = tid % COLS, ty = tid / COLS;
+    const int stages = K / KBLOCK * 16;
+    auto group_barrier = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(THREADS) : "memory"); };
+
+    uint64_t acc[8][TN / 2], total[8][TN / 2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + (i / 4) * (BM / 2) + ty * 4 + i % 4;
-        if (m >= M) continue;
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int h = 0; h < QN; ++h) {
-            const int n = n0 + h * (BN / 2) + tx * 4;
-            float* row = C + (int64_t)m * ldc + n;
-            const float2 lo = *reinterpret_cast<const float2*>(&total[i][h * 2]);
-            const float2 hi = *reinterpret_cast<const float2*>(&total[i][h * 2 + 1]);
-            if (packets && n + 4 <= N) {
-                *reinterpret_cast<float4*>(row) = make_float4(lo.x, lo.y, hi.x, hi.y);
-            } else {
-                if (n < N) row[0] = lo.x;
-                if (n + 1 < N) row[1] = lo.y;
-                if (n + 2 < N) row[2] = hi.x;
-                if (n + 3 < N) row[3] = hi.y;
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = total[i][j] = 0;
+    float a[LA][4], w[LW][4];
+    auto fetch_one = [&](const float* base, int64_t ld, int row, int rows, int kk, float* v) {
+        const float4 t = row < rows ? *reinterpret_cast<const float4*>(base + (int64_t)row * ld + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    };
+    const int q = tid % 4, row_of = tid / 4;
+    auto fetch = [&](int t) {
+        const int kk = stage_start(t) + (q >> 1) * 32 + (q & 1) * 4;
+#pragma unroll
+        for (int l = 0; l < LA; ++l) fetch_one(A, lda, m0 + l * (THREADS / 4) + row_of, M, kk, a[l]);
+#pragma unroll
+        for (int l = 0; l < LW; ++l) fetch_one(W, ldw, n0 + l * (THREADS / 4) + row_of, N, kk, w[l]);
+    };
+    auto put = [&](int buffer) {
+        float *As = stages_at + buffer * STAGE, *Ws = As + BK * AP;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+            for (int l = 0; l < LA; ++l) As[(q * 4 + e) * AP + l * (THREADS / 4) + row_of] = a[l][e];
+#pragma unroll
+            for (int l = 0; l < LW; ++l) Ws[(q * 4 + e) * WP + l * (THREADS / 4) + row_of] = w[l][e];
+        }
+    };
+    pdl_trigger();
+    pdl_wait();
+    int t = group * 4, buffer = 0;                     // (K / 64 chains, a multiple of four: every group takes as many)
+    fetch(t);
+    put(0);
+    group_barrier();
+    while (t < stages) {
+        const bool ends = (t & 3) == 3;                // the chain's last stage; the group's next chain is G further
+        const int ahead = ends ? t + 1 + 4 * (G - 1) : t + 1;
+        if (ahead < stages) fetch(ahead);
+        const float *As = stages_at + buffer * STAGE, *Ws = As + BK * AP;
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            float ar[8];
+            uint64_t wr[TN / 2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 v = *reinterpret_cast<const float4*>(As + k * AP + h * (BM / 2) + ty * 4);
+                ar[h * 4] = v.x; ar[h * 4 + 1] = v.y; ar[h * 4 + 2] = v.z; ar[h * 4 + 3] = v.w;
+            }
+#pragma unroll
+            for (int h = 0; h < QN; ++h) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Ws + k * WP + h * (BN / 2) + tx * 4);
+                wr[h * 2] = v.x; wr[h * 2 + 1] = v.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint64_t both = twice(ar[i]);
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], both, wr[j]);
             }
         }
+        if (ends) {
+            if (group > 0) {
+                if (t >= 4 * G) asm volatile("bar.sync %0, %1;" ::"r"(G + 1), "n"(THREADS * G) : "memory");      // the last round's sums are taken
+#pragma unroll
+                for (int i = 0; i < SUMS; ++i) {
+                    const uint64_t* from = &acc[i * 2 / (TN / 2)][i * 2 % (TN / 2)];
+                    const float2 lo = *reinterpret_cast<const float2*>(from), hi = *reinterpret_cast<const float2*>(from + 1);
+                    given[((group - 1) * SUMS + i) * THREADS + tid] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+                asm volatile("bar.arrive %0, %1;" ::"r"(G + 2), "n"(THREADS * G) : "memory");
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN / 2; ++j) add2(total[i][j], acc[i][j]);
+                asm volatile("bar.sync %0, %1;" ::"r"(G + 2), "n"(THREADS * G) : "memory");                     // this round's sums are there
+#pragma unroll
+                for (int other = 0; other < G - 1; ++other)
+#pragma unroll
+                    for (int i = 0; i < SUMS; ++i) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&given[(other * SUMS + i) * THREADS + tid]);
+                        add2(total[i * 2 / (TN / 2)][i * 2 % (TN / 2)], v.x);
+                        add2(total[i * 2 / (TN / 2)][i * 2 % (TN / 2) + 1], v.y);
+                    }
+                if (ahead < stages) asm volatile("bar.arrive %0, %1;" ::"r"(G + 1), "n"(THREADS * G) : "memory");
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
+        }
+        buffer ^= 1;
+        if (ahead < stages) put(buffer);
+        group_barrier();
+        t = ahead;
     }
+    if (group > 0) return;
+    store_tile<BM, BN, TN>(total, C, ldc, m0, n0, tx, ty, M, N);
 }
 
 // ---- few rows: the weights stream through registers -----------------------------------------------------------------
@@ -321,6 +450,19 @@ cudaError_t launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw
                          C, ldc, M, N, K);
 }
 
+template <int BM, int BN, int TN, int G>
+cudaError_t launch_groups(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
+                          int K, cudaStream_t stream) {
+    constexpr int threads = (BM / 8) * (BN / TN);
+    constexpr int bytes = (G * 2 * BK * (BM + BN + 8) + (G - 1) * BM * BN) * 4;
+    static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_groups_kernel<BM, BN, TN, G>,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (set != cudaSuccess) return set;
+    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    return tb_launch_pdl(gemm_f32_groups_kernel<BM, BN, TN, G>, grid, dim3(threads * G), bytes, stream, A, lda, W, ldw, C, ldc, M,
+                         N, K);
+}
+
 }  // namespace
 
 // Zero padding inside a chain adds exact zeros, which leaves every partial sum unchanged, so the guarded and the packet
@@ -345,6 +487,12 @@ TB_EXPORT int tb_gemm_f32_nt(const float* A, int64_t lda, const float* W, int64_
         return (int)launch_rows<8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
     if (!vec) return (int)launch_tile<false, 64, 64, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    // One tile a multiprocessor: groups of threads share its chains.  200 rows of 2,048 x 2,048 (128 square tiles) 94 -> 72 us,
+    // 160 of 3,072 x 2,048 171 -> 72, 64 rows of 16,384 x 2,048 (tall tiles would be half empty) 220 -> 158; 380 rows of
+    // 3,072 x 2,048 (144 tall tiles) 188 -> 130, 500 of 2,048 x 2,048 203 -> 121.  With more tiles two of one group share a
+    // multiprocessor, which is faster (380 rows of 16,384 x 2,048: 684 against 787).
+    if (K % KBLOCK == 0 && (square <= 148 || M <= 64)) return (int)launch_groups<64, 64, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (K % KBLOCK == 0 && tall <= 148) return (int)launch_groups<128, 64, 8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     // Tall tiles load less from shared memory for a product but leave the chip emptier: 200 rows of 2,048 x 2,048 (64 of
     // them) take 139 us, as square tiles 94; 380 rows (96) 141 against 145, and 547 against 566 at K = 8,192.
     if (tall >= 96) return (int)launch_tile<true, 128, 64, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream);

@@ -97,7 +97,8 @@ def test_gemm_f32(m, n, k):
 
 
 @pytest.mark.parametrize("m, n, k", [(1, 17, 8), (2, 16, 264), (3, 4737, 2048), (8, 40, 2056), (9, 33, 4104), (48, 65, 256),
-                                     (49, 130, 264), (70, 100, 2048), (130, 3100, 72), (129, 3072, 2048)])
+                                     (49, 130, 264), (70, 100, 2048), (130, 3100, 72), (129, 3072, 2048),
+                                     (49, 70, 256), (64, 9500, 256), (130, 2100, 512), (257, 3000, 256), (300, 6500, 256)])
 def test_gemm_f32_streams_and_tiles_sum_in_one_order(m, n, k):
     """Rows picked from a larger product, and the guarded loads of operands off their alignment, give the same bits, so the
     streaming kernel (few rows) and both tile shapes are one sum; and that sum is near the 64-bit one."""
