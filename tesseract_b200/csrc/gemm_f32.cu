@@ -174,7 +174,7 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
 }
 
 // The tiles where they are too few to give a multiprocessor more than one: G groups of threads take a tile's chains in turn (K a
-// multiple of 256, packets), and the first group adds every round's sums in the order of the chains, the others' through
+// multiple of 256, packets), and the first group adds the sums in the order of the chains, the others' through
 // shared memory, so that the bits are those of the kernel above.  Bound by the latency of a group's stages, which the groups hide
 // from one another.   128 x 64
 // tiles of two groups and 64 x 64 tiles of four take 121 and 72 us for K = 2,048 (one group, where a multiprocessor has one tile:
@@ -256,7 +256,7 @@ gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw,
         }
         if (ends) {
             if (group > 0) {
-                if (t >= 4 * G) asm volatile("bar.sync %0, %1;" ::"r"(G + 1), "n"(THREADS * G) : "memory");      // the last round's sums are taken
+                if (t >= 4 * G) asm volatile("bar.sync %0, %1;" ::"r"(G + 1), "n"(THREADS * G) : "memory");      // the last sums are taken
 #pragma unroll
                 for (int i = 0; i < SUMS; ++i) {
                     const uint64_t* from = &acc[i * 2 / (TN / 2)][i * 2 % (TN / 2)];
@@ -269,7 +269,7 @@ gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw,
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < TN / 2; ++j) add2(total[i][j], acc[i][j]);
-                asm volatile("bar.sync %0, %1;" ::"r"(G + 2), "n"(THREADS * G) : "memory");                     // this round's sums are there
+                asm volatile("bar.sync %0, %1;" ::"r"(G + 2), "n"(THREADS * G) : "memory");                     // the others' sums are there
 #pragma unroll
                 for (int other = 0; other < G - 1; ++other)
 #pragma unroll
@@ -434,8 +434,8 @@ template <int ROWS>
 cudaError_t launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
                         int K, cudaStream_t stream) {
     constexpr int bytes = (2 * WARPS * CHAINS * ROWS * FEATURES + WARPS * 2 * ROWS * KBLOCK) * 4;
-    static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_rows_kernel<ROWS>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    // (asked for on every call: the attribute is the current device's)
+    const cudaError_t set = cudaFuncSetAttribute(gemm_f32_rows_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (set != cudaSuccess) return set;
     const int tiles = (N + FEATURES - 1) / FEATURES, groups = (M + ROWS - 1) / ROWS;
     const dim3 grid(tiles < 296 ? tiles : 296, groups);              // two blocks on each of the 148 multiprocessors
@@ -455,8 +455,8 @@ cudaError_t launch_groups(const float* A, int64_t lda, const float* W, int64_t l
                           int K, cudaStream_t stream) {
     constexpr int threads = (BM / 8) * (BN / TN);
     constexpr int bytes = (G * 2 * BK * (BM + BN + 8) + (G - 1) * BM * BN) * 4;
-    static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_groups_kernel<BM, BN, TN, G>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t set = cudaFuncSetAttribute(gemm_f32_groups_kernel<BM, BN, TN, G>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (set != cudaSuccess) return set;
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     return tb_launch_pdl(gemm_f32_groups_kernel<BM, BN, TN, G>, grid, dim3(threads * G), bytes, stream, A, lda, W, ldw, C, ldc, M,
