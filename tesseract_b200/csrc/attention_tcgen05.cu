@@ -484,6 +484,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
         // the products' operands and lets a block's probabilities be stored while the product before still reads its own.
         // 2,048 rows of 32 heads of 128 at context 12,345: 389 us (975 TFLOP/s), 412 with P in shared memory and S kept until
         // the maximum is known; 57 rows there, eight CTAs a tile: 78 and 113; 512 rows at 8,704, two: 99 and 114.
+        // What P_j V_j read and wrote in tensor memory (its buffer of P, and O) may be accessed by this thread again: the barrier
+        // alone does not order tcgen05 accesses behind it, the fence does.
+        auto product_done = [&](int j) {
+            if (!mbar_wait(o_full(j), phase(j), &abort_flag)) return false;
+            tc_fence_after();
+            return true;
+        };
         for (int j = 0; kPInTmem && j < n_blocks; ++j) {
             const int key0 = (kb_first + j) * BN;
             if (!mbar_wait(s_full, j & 1, &abort_flag)) { ok = false; break; }
@@ -523,7 +530,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                 mbar_arrive(s_free);                   // (both chunks are in registers)
                 freed = true;
                 // P_{j-2} V_{j-2} has read this buffer
-                if (j >= kPBuffers && !mbar_wait(o_full(j - kPBuffers), phase(j - kPBuffers), &abort_flag)) { ok = false; break; }
+                if (j >= kPBuffers && !product_done(j - kPBuffers)) { ok = false; break; }
                 tmem_store_16_nowait(tmem_p(j) + lane_base, packed);
                 maxima(sc[1]);
                 const float seen = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
@@ -569,13 +576,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             const float block_max = raw_max > 0.5f * kMasked ? raw_max * p.scale_log2 : kMasked;
             const bool jump = block_max > m + 8.0f;
             if (__any_sync(0xffffffffu, jump)) {
-                if (j > 0 && !mbar_wait(o_full(j - 1), phase(j - 1), &abort_flag)) { ok = false; break; }
+                if (j > 0 && !product_done(j - 1)) { ok = false; break; }
                 const float m_new = fmaxf(m, block_max);
                 const float corr = fast_exp2(m - m_new);
                 m = m_new;
                 l *= corr;
                 if (j > 0) {
-                    tc_fence_after();
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         float v[32];
@@ -613,7 +619,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                     sc[c][i >> 1] = pack_bf16(p0, p1);
                 }
                 // P_{j-2} V_{j-2} has read this buffer
-                if (c == 0 && j >= kPBuffers && !mbar_wait(o_full(j - kPBuffers), phase(j - kPBuffers), &abort_flag)) ok = false;
+                if (c == 0 && j >= kPBuffers && !product_done(j - kPBuffers)) { ok = false; break; }
                 tmem_store_16_nowait(tmem_p(j) + lane_base + c * 16, sc[c]);
             }
             if (!ok) break;
