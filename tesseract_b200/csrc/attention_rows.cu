@@ -43,7 +43,7 @@ struct Vec16<__nv_bfloat16> {
     }
 };
 
-// UNDER: loads under way at a time (packets of a key, values of a block).
+// UNDER: loads under way at a time (packets of a key, values of a block); 0: as they are needed, and none for a key without weight.
 template <typename T, int NC, int UNDER>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__ out, int64_t out_stride,
@@ -86,18 +86,27 @@ attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__
             key_offset = (int64_t)page * page_block + (int64_t)(key % page_size) * head_dim;
             const T* kp = kbase + key_offset;
             float dot = 0.0f;
-            // (UNDER packets asked for at a time; the sum runs on in order)
-            for (int i0 = 0; i0 < head_dim; i0 += UNDER * Vec16<T>::N) {
-                float kv[UNDER][Vec16<T>::N];
+            if constexpr (UNDER == 0) {
+                float kv[Vec16<T>::N];
+                for (int i = 0; i < head_dim; i += Vec16<T>::N) {
+                    Vec16<T>::load(kp + i, kv);
 #pragma unroll
-                for (int u = 0; u < UNDER; ++u)
-                    if (i0 + u * Vec16<T>::N < head_dim) Vec16<T>::load(kp + i0 + u * Vec16<T>::N, kv[u]);
+                    for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i + e], kv[e], dot);
+                }
+            } else {
+                // (UNDER packets asked for at a time; the sum runs on in order)
+                for (int i0 = 0; i0 < head_dim; i0 += UNDER * Vec16<T>::N) {
+                    float kv[UNDER][Vec16<T>::N];
 #pragma unroll
-                for (int u = 0; u < UNDER; ++u)
-                    if (i0 + u * Vec16<T>::N < head_dim) {
+                    for (int u = 0; u < UNDER; ++u)
+                        if (i0 + u * Vec16<T>::N < head_dim) Vec16<T>::load(kp + i0 + u * Vec16<T>::N, kv[u]);
 #pragma unroll
-                        for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i0 + u * Vec16<T>::N + e], kv[u][e], dot);
-                    }
+                    for (int u = 0; u < UNDER; ++u)
+                        if (i0 + u * Vec16<T>::N < head_dim) {
+#pragma unroll
+                            for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i0 + u * Vec16<T>::N + e], kv[u][e], dot);
+                        }
+                }
             }
             s = dot * scale;
         }
@@ -109,22 +118,37 @@ attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__
         for (int c = 0; c < NC; ++c) acc[c] *= corr;
         const float p_mma = Elem<T>::round(p);
         const int keys_here = min(kKeyBlock, pos - kb * kKeyBlock + 1);
-        for (int j0 = 0; j0 < keys_here; j0 += UNDER) {
-            float v[UNDER][NC];
+        if constexpr (UNDER == 0) {
+            for (int j = 0; j < keys_here; ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p_mma, j);
+                const int64_t off = __shfl_sync(0xffffffffu, key_offset, j);
+                if (pj != 0.0f) {  // uniform across the warp; masked keys contribute nothing
+                    const T* vp = vbase + off;
 #pragma unroll
-            for (int u = 0; u < UNDER; ++u) {
-                const T* vp = vbase + __shfl_sync(0xffffffffu, key_offset, j0 + u);    // (a lane without a key: offset 0, not used)
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (j0 + u < keys_here && c * 32 + lane < head_dim) v[u][c] = Elem<T>::load(vp + c * 32 + lane);
+                    for (int c = 0; c < NC; ++c) {
+                        const int col = c * 32 + lane;
+                        if (col < head_dim) acc[c] = fmaf(pj, Elem<T>::load(vp + col), acc[c]);
+                    }
+                }
             }
+        } else {
+            for (int j0 = 0; j0 < keys_here; j0 += UNDER) {
+                float v[UNDER][NC];
 #pragma unroll
-            for (int u = 0; u < UNDER; ++u) {
-                const float pj = __shfl_sync(0xffffffffu, p_mma, j0 + u);
-                if (j0 + u < keys_here && pj != 0.0f) {  // uniform across the warp; masked keys contribute nothing
+                for (int u = 0; u < UNDER; ++u) {
+                    const T* vp = vbase + __shfl_sync(0xffffffffu, key_offset, j0 + u);    // (a lane without a key: offset 0, not used)
 #pragma unroll
                     for (int c = 0; c < NC; ++c)
-                        if (c * 32 + lane < head_dim) acc[c] = fmaf(pj, v[u][c], acc[c]);
+                        if (j0 + u < keys_here && c * 32 + lane < head_dim) v[u][c] = Elem<T>::load(vp + c * 32 + lane);
+                }
+#pragma unroll
+                for (int u = 0; u < UNDER; ++u) {
+                    const float pj = __shfl_sync(0xffffffffu, p_mma, j0 + u);
+                    if (j0 + u < keys_here && pj != 0.0f) {  // uniform across the warp; masked keys contribute nothing
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+                            if (c * 32 + lane < head_dim) acc[c] = fmaf(pj, v[u][c], acc[c]);
+                    }
                 }
             }
         }
@@ -150,21 +174,31 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
     attention_rows_kernel<T, NC, UNDER><<<grid, kWarpsPerBlock * 32, smem, stream>>>(                                 \
         (const T*)q, q_stride, (T*)out, out_stride, (const T*)cache, positions, seq_of_row, block_table,       \
         bt_stride, num_heads, num_kv_heads, head_dim, page_size, window, scale)
-    // Few warps a multiprocessor (decoded rows) are bound by the latency of their loads: 4 rows of 32 heads of 64 behind some
-    // 100 keys 16.4 us with 32 under way in 32-bit (39 one after another), 24.5 with 16 in bfloat16 (36).  Where the warps fill
-    // the chip the registers that this takes cost more than it gives: 381 prompt rows 76 us with 2 (8: 82, 1: 82), in bfloat16
-    // 55 with 1 (8: 97).  Wide bfloat16 heads stop gaining early (head size 256: 46 us one after another, 38 with 4, 52 with 8).
+    // Few warps a multiprocessor (decoded rows) are bound by the latency of their loads, and more under way shorten it: 4 rows of 32
+    // heads of 64 behind some 100 keys take 13.4 us in 32-bit with 32 under way, 30.7 as they are needed.  The registers that this
+    // takes hold back other warps as soon as there are more: 64 rows of 32 heads of 128 behind 300 keys, 32-bit, 8 / 16 under way or
+    // as needed 140 / 288 / 251.  So 592 blocks, four a multiprocessor, take the form that was the fastest or close to it over all
+    // of them (32-bit: 0.4 to 0.8 of the time as needed, bfloat16 0.65 to 0.9), and steps that fill the chip take few or none:
+    // 600 rows of 8 heads of 32 behind up to 1,500 keys 359 us as needed, 395 with two; of 256 in bfloat16 1,462 and 1,681 with one.
+    // The engine takes this kernel in 32-bit; bfloat16 callers have heads that the tensor-core kernels are not built for.
     constexpr bool wide = sizeof(T) == 4;
-    if ((int64_t)rows * grid.y <= kFewBlocks) {
-        if (head_dim <= 32) TB_LAUNCH(1, (wide ? 32 : 16));
-        else if (head_dim <= 64) TB_LAUNCH(2, (wide ? 32 : 16));
-        else if (head_dim <= 128) TB_LAUNCH(4, (wide ? 16 : 4));
-        else TB_LAUNCH(8, (wide ? 8 : 4));
+    const int64_t blocks = (int64_t)rows * grid.y;
+    const bool few = blocks <= kFewBlocks, some = blocks <= 2 * kFewBlocks;
+    if (head_dim <= 32) {
+        if (few) TB_LAUNCH(1, (wide ? 16 : 8));
+        else TB_LAUNCH(1, 0);
+    } else if (head_dim <= 64) {
+        if (few) TB_LAUNCH(2, (wide ? 32 : 4));
+        else TB_LAUNCH(2, (wide ? 2 : 1));
+    } else if (head_dim <= 128) {
+        // (bfloat16: one under way where its blocks, ten a multiprocessor, take no more waves than the twelve without)
+        if (wide && few) TB_LAUNCH(4, (wide ? 8 : 1));
+        else if (wide ? some : (blocks + 1479) / 1480 <= (blocks + 1775) / 1776) TB_LAUNCH(4, (wide ? 2 : 1));
+        else TB_LAUNCH(4, 0);
     } else {
-        if (head_dim <= 32) TB_LAUNCH(1, (wide ? 2 : 1));
-        else if (head_dim <= 64) TB_LAUNCH(2, (wide ? 2 : 1));
-        else if (head_dim <= 128) TB_LAUNCH(4, (wide ? 2 : 1));
-        else TB_LAUNCH(8, (wide ? 2 : 1));
+        if (few) TB_LAUNCH(8, (wide ? 8 : 4));
+        else if (wide && some) TB_LAUNCH(8, (wide ? 2 : 0));
+        else TB_LAUNCH(8, 0);
     }
 #undef TB_LAUNCH
     return tb_launch_status();

@@ -226,6 +226,28 @@ def test_attention_rows_gives_few_rows_the_bits_of_many(dtype, d, nh):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d, nh", [(24, 4), (56, 4), (104, 4), (232, 4)])
+def test_attention_rows_gives_steps_of_any_size_the_same_bits(dtype, d, nh):
+    """Steps that fill the chip ask for a key's numbers as they need them, smaller ones for several at a time."""
+    from tesseract_b200 import kernels
+
+    rows, page_size = 1500, 16
+    case = paged_case(dtype, [rows + 9], [rows], nh, 2, d, page_size, seed=d)
+    q, out = dev(case["q"]).view(rows, nh * d), torch.empty(rows, nh * d, dtype=dtype, device="cuda")
+    cache, table = dev(case["cache"]), dev(case["table"])
+
+    def run(lo, hi, window):
+        kernels.attention_rows(q[lo:hi], out[:hi - lo], cache, dev(case["positions"][lo:hi]), dev(case["seq_of_row"][lo:hi]), table, nh, 2,
+                               d, page_size, window, d ** -0.5)
+        return out[:hi - lo].clone()
+
+    for window in (0, 45):
+        many = run(0, rows, window)
+        for lo, hi in ((rows - 3, rows), (700, 1292), (592, 1185), (310, 1494)):       # up to, and one past, four blocks a multiprocessor; eight
+            assert torch.equal(run(lo, hi, window), many[lo:hi])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window", [0, 1, 24, 100])
 def test_attention_rows_at_the_edges_of_what_a_row_sees(dtype, window):
     """Scores that rise by 8 with every key (the position as 16 * hi + lo in two dimensions, exact in bfloat16 too) give
