@@ -26,24 +26,39 @@ struct Streams {
     float eps;
 };
 
+__device__ __forceinline__ float4 scaled(float4 v, float by) { return make_float4(v.x * by, v.y * by, v.z * by, v.w * by); }
+__device__ __forceinline__ float4 plus_scaled(float4 sum, const float4& v, float by) {
+    return make_float4(fmaf(by, v.x, sum.x), fmaf(by, v.y, sum.y), fmaf(by, v.z, sum.z), fmaf(by, v.w, sum.w));
+}
+// Copy t of four columns from the old copies and the sublayers' output.
+template <int S>
+__device__ __forceinline__ float4 mixed(const float (&mix)[S][S], const float (&share)[S], const float4 (&x)[S], const float4& y, int t) {
+    float4 n = scaled(y, share[t]);
+#pragma unroll
+    for (int s = 0; s < S; ++s) n = plus_scaled(n, x[s], mix[s][t]);
+    return n;
+}
+template <typename T>
+__device__ __forceinline__ void put_normed(T* to, const float4& u, float inv, const float4& w) {
+    const float v[4] = {u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w};
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+        __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+        *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+    }
+}
+
 // S > 0: that many copies, their packets in registers; S == 0: any number up to kMaxStreams, one column a thread at a time.
-// Bound by the chain of a launch where rows are few, by the copies' bytes where they are many: a thread asks for two packets of
-// every copy before it stores one, and for the norm's weights before the wait.  Four copies of 2,048 numbers at 8 / 32 / 2,048 rows:
-// 2.4 / 2.6 / 23.8 us, with a packet after another 3.0 / 3.2 / 26.9.  (The residual is not __restrict__: its loads stay behind the wait.)
 template <typename T, int S>
-__global__ void __launch_bounds__(kThreads, S == 3 || S == 4 ? 2 : 1)
-mixed_streams_norm_kernel(float* residual, T* out, Streams p) {
+__global__ void __launch_bounds__(kThreads)
+mixed_streams_norm_kernel(float* __restrict__ residual, T* __restrict__ out, Streams p) {
     __shared__ float scratch[32];
     pdl_trigger();
     const int W = p.width;
     constexpr int C = S > 0 ? S : 1;
     float mix[C][C], share[C], take[C];
-    float4 weight[2];
     if (S > 0) {                                      // (weights: not written by any kernel in front)
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-            if (out != nullptr && n * kThreads + threadIdx.x < W / 4)
-                weight[n] = *reinterpret_cast<const float4*>(p.weight + (n * kThreads + threadIdx.x) * 4);
 #pragma unroll
         for (int t = 0; t < C; ++t) {
             share[t] = p.share != nullptr ? p.share[t] : 0.0f;
@@ -62,32 +77,17 @@ mixed_streams_norm_kernel(float* residual, T* out, Streams p) {
     if constexpr (S > 0) {
         float4 kept[kKeep];
         const int packets = W / 4;
-        struct Column { float4 x[S], y, z; };
-        auto ask = [&](int i, Column& c) {            // everything that columns i .. i + 3 need
+        auto column = [&](int i) {                    // the new copies of columns i .. i + 3 are stored; what the next sublayer reads comes back
+            float4 x[S];
 #pragma unroll
-            for (int s = 0; s < S; ++s) c.x[s] = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
-            if (ua != nullptr) c.y = *reinterpret_cast<const float4*>(ua + i);
-            if (ub != nullptr) c.z = *reinterpret_cast<const float4*>(ub + i);
-        };
-        auto renew = [&](int i, Column& c) {          // the new copies are stored; what the next sublayer reads comes back
-            float4 (&x)[S] = c.x;
+            for (int s = 0; s < S; ++s) x[s] = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
             if (ua != nullptr) {
-                float4 y = c.y;
-                y.x *= p.scale_a; y.y *= p.scale_a; y.z *= p.scale_a; y.w *= p.scale_a;
-                if (ub != nullptr) {
-                    const float4 z = c.z;
-                    y.x = fmaf(p.scale_b, z.x, y.x); y.y = fmaf(p.scale_b, z.y, y.y);
-                    y.z = fmaf(p.scale_b, z.z, y.z); y.w = fmaf(p.scale_b, z.w, y.w);
-                }
+                float4 y = scaled(*reinterpret_cast<const float4*>(ua + i), p.scale_a);
+                if (ub != nullptr) y = plus_scaled(y, *reinterpret_cast<const float4*>(ub + i), p.scale_b);
                 float4 n[S];
 #pragma unroll
                 for (int t = 0; t < S; ++t) {
-                    n[t] = make_float4(share[t] * y.x, share[t] * y.y, share[t] * y.z, share[t] * y.w);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        n[t].x = fmaf(mix[s][t], x[s].x, n[t].x); n[t].y = fmaf(mix[s][t], x[s].y, n[t].y);
-                        n[t].z = fmaf(mix[s][t], x[s].z, n[t].z); n[t].w = fmaf(mix[s][t], x[s].w, n[t].w);
-                    }
+                    n[t] = mixed<S>(mix, share, x, y, t);
                     *reinterpret_cast<float4*>(res + (int64_t)t * W + i) = n[t];
                 }
 #pragma unroll
@@ -95,66 +95,36 @@ mixed_streams_norm_kernel(float* residual, T* out, Streams p) {
             }
             float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-                u.x = fmaf(take[s], x[s].x, u.x); u.y = fmaf(take[s], x[s].y, u.y);
-                u.z = fmaf(take[s], x[s].z, u.z); u.w = fmaf(take[s], x[s].w, u.w);
-            }
+            for (int s = 0; s < S; ++s) u = plus_scaled(u, x[s], take[s]);
             return u;
         };
         auto again = [&](int i) {                     // (its own stores)
             float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-                const float4 x = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
-                u.x = fmaf(take[s], x.x, u.x); u.y = fmaf(take[s], x.y, u.y);
-                u.z = fmaf(take[s], x.z, u.z); u.w = fmaf(take[s], x.w, u.w);
-            }
+            for (int s = 0; s < S; ++s) u = plus_scaled(u, *reinterpret_cast<const float4*>(res + (int64_t)s * W + i), take[s]);
             return u;
         };
         auto square = [&](const float4& u) {
             ss = fmaf(u.x, u.x, ss); ss = fmaf(u.y, u.y, ss); ss = fmaf(u.z, u.z, ss); ss = fmaf(u.w, u.w, ss);
         };
-        // Two packets of the row asked for at a time: a store in between would hold back the next one's loads.  (One or two copies
-        // keep to one: their rows are short, and with the registers of a second 2,048 rows of two copies take 12.2 us, not 10.9.)
-        constexpr int ASK = S >= 3 ? 2 : 1;
-#pragma unroll
-        for (int n0 = 0; n0 < kKeep; n0 += ASK) {
-            Column c[ASK];
-#pragma unroll
-            for (int n = 0; n < ASK; ++n)
-                if ((n0 + n) * kThreads + threadIdx.x < packets) ask(((n0 + n) * kThreads + threadIdx.x) * 4, c[n]);
-#pragma unroll
-            for (int n = 0; n < ASK; ++n) {
-                const int q = (n0 + n) * kThreads + threadIdx.x;
-                if (q < packets) {
-                    kept[n0 + n] = renew(q * 4, c[n]);
-                    square(kept[n0 + n]);
-                }
-            }
-        }
-        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) {
-            Column c;
-            ask(q * 4, c);
-            square(renew(q * 4, c));
-        }
-        if (to == nullptr) return;
-        const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)W + p.eps);
-        auto finish = [&](int i, const float4& u, const float4& w) {
-            const float v[4] = {u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w};
-            if constexpr (sizeof(T) == 4) {
-                *reinterpret_cast<float4*>(to + i) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-                __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-                *reinterpret_cast<uint2*>(to + i) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
-            }
-        };
 #pragma unroll
         for (int n = 0; n < kKeep; ++n) {
             const int q = n * kThreads + threadIdx.x;
-            if (q < packets) finish(q * 4, kept[n], n < 2 ? weight[n & 1] : *reinterpret_cast<const float4*>(p.weight + q * 4));
+            if (q < packets) {
+                kept[n] = column(q * 4);
+                square(kept[n]);
+            }
         }
-        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads)
-            finish(q * 4, again(q * 4), *reinterpret_cast<const float4*>(p.weight + q * 4));
+        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) square(column(q * 4));
+        if (to == nullptr) return;
+        const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)W + p.eps);
+        auto finish = [&](int i, const float4& u) { put_normed(to + i, u, inv, *reinterpret_cast<const float4*>(p.weight + i)); };
+#pragma unroll
+        for (int n = 0; n < kKeep; ++n) {
+            const int q = n * kThreads + threadIdx.x;
+            if (q < packets) finish(q * 4, kept[n]);
+        }
+        for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) finish(q * 4, again(q * 4));
     } else {
         const int N = p.streams;
         for (int i = threadIdx.x; i < W; i += kThreads) {
@@ -182,6 +152,104 @@ mixed_streams_norm_kernel(float* residual, T* out, Streams p) {
             for (int t = 0; t < N; ++t) u = fmaf(p.take[t], res[(int64_t)t * W + i], u);
             Elem<T>::store(to + i, u * inv * p.weight[i]);
         }
+    }
+}
+
+// The same work, to the bit, for S copies in packets, with more asked for ahead: two packets of every copy (of three or more) before
+// one of them is stored, for a store would hold back the next one's loads, and the norm's weights before the wait.  That takes
+// registers, so fewer blocks run side by side and steps of many rows may be faster without (launch() below).  Four copies of
+// 2,048 numbers at 8 / 32 / 2,048 rows: 2.4 / 2.6 / 23.8 us, 3.0 / 3.2 / 26.9 by the kernel above.
+// (The residual is not __restrict__: its loads stay behind the wait.)
+template <int S>
+constexpr int kAheadBlocks = S <= 4 ? 2 : 1;          // a multiprocessor, by the registers
+
+template <typename T, int S>
+__global__ void __launch_bounds__(kThreads, kAheadBlocks<S>)
+mixed_streams_norm_ahead_kernel(float* residual, T* out, Streams p) {
+    __shared__ float scratch[32];
+    pdl_trigger();
+    const int W = p.width, packets = W / 4;
+    float mix[S][S], share[S], take[S];
+    float4 weight[2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)                       // (weights: not written by any kernel in front)
+        if (out != nullptr && n * kThreads + threadIdx.x < packets)
+            weight[n] = *reinterpret_cast<const float4*>(p.weight + (n * kThreads + threadIdx.x) * 4);
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+        share[t] = p.share != nullptr ? p.share[t] : 0.0f;
+        take[t] = p.take != nullptr ? p.take[t] : 0.0f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) mix[s][t] = p.mix != nullptr ? p.mix[s * S + t] : 0.0f;
+    }
+    pdl_wait();
+    const int64_t row = blockIdx.x;
+    float* res = residual + row * S * W;
+    const float* ua = p.update_a == nullptr ? nullptr : p.update_a + row * W;
+    const float* ub = p.update_b == nullptr ? nullptr : p.update_b + row * W;
+    T* to = out == nullptr ? nullptr : out + row * W;
+    float ss = 0.0f;
+    float4 kept[kKeep];
+    struct Column { float4 x[S], y, z; };
+    auto ask = [&](int i, Column& c) {                // everything that columns i .. i + 3 need
+#pragma unroll
+        for (int s = 0; s < S; ++s) c.x[s] = *reinterpret_cast<const float4*>(res + (int64_t)s * W + i);
+        if (ua != nullptr) c.y = *reinterpret_cast<const float4*>(ua + i);
+        if (ub != nullptr) c.z = *reinterpret_cast<const float4*>(ub + i);
+    };
+    auto renew = [&](int i, Column& c) {              // the new copies are stored; what the next sublayer reads comes back
+        if (ua != nullptr) {
+            float4 y = scaled(c.y, p.scale_a), n[S];
+            if (ub != nullptr) y = plus_scaled(y, c.z, p.scale_b);
+#pragma unroll
+            for (int t = 0; t < S; ++t) {
+                n[t] = mixed<S>(mix, share, c.x, y, t);
+                *reinterpret_cast<float4*>(res + (int64_t)t * W + i) = n[t];
+            }
+#pragma unroll
+            for (int s = 0; s < S; ++s) c.x[s] = n[s];
+        }
+        float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int s = 0; s < S; ++s) u = plus_scaled(u, c.x[s], take[s]);
+        return u;
+    };
+    auto square = [&](const float4& u) {
+        ss = fmaf(u.x, u.x, ss); ss = fmaf(u.y, u.y, ss); ss = fmaf(u.z, u.z, ss); ss = fmaf(u.w, u.w, ss);
+    };
+    constexpr int ASK = S >= 3 ? 2 : 1;
+#pragma unroll
+    for (int n0 = 0; n0 < kKeep; n0 += ASK) {
+        Column c[ASK];
+#pragma unroll
+        for (int n = 0; n < ASK; ++n)
+            if ((n0 + n) * kThreads + threadIdx.x < packets) ask(((n0 + n) * kThreads + threadIdx.x) * 4, c[n]);
+#pragma unroll
+        for (int n = 0; n < ASK; ++n) {
+            const int q = (n0 + n) * kThreads + threadIdx.x;
+            if (q < packets) {
+                kept[n0 + n] = renew(q * 4, c[n]);
+                square(kept[n0 + n]);
+            }
+        }
+    }
+    for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) {
+        Column c;
+        ask(q * 4, c);
+        square(renew(q * 4, c));
+    }
+    if (to == nullptr) return;
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)W + p.eps);
+#pragma unroll
+    for (int n = 0; n < kKeep; ++n) {
+        const int q = n * kThreads + threadIdx.x;
+        if (q < packets) put_normed(to + q * 4, kept[n], inv, n < 2 ? weight[n & 1] : *reinterpret_cast<const float4*>(p.weight + q * 4));
+    }
+    for (int q = kKeep * kThreads + threadIdx.x; q < packets; q += kThreads) {
+        float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int s = 0; s < S; ++s) u = plus_scaled(u, *reinterpret_cast<const float4*>(res + (int64_t)s * W + q * 4), take[s]);
+        put_normed(to + q * 4, u, inv, *reinterpret_cast<const float4*>(p.weight + q * 4));
     }
 }
 
@@ -237,19 +305,32 @@ template <typename T>
 int launch(float* residual, void* out, const Streams& p, int rows, cudaStream_t stream) {
     const uintptr_t bits = (uintptr_t)residual | (uintptr_t)out | (uintptr_t)p.update_a | (uintptr_t)p.update_b | (uintptr_t)p.weight;
     const bool packets = p.width % 4 == 0 && bits % 16 == 0;
+    // Asking ahead is taken where it needs no more waves of blocks than the lean kernel, whose blocks fit `lean` a multiprocessor: one
+    // copy of 2,048 numbers, 296 / 400 / 2,048 rows 2.4 / 3.7 / 12.0 us against 3.1 / 3.3 / 7.8, two copies, 148 / 2,048 rows
+    // 2.5 / 14.8 against 2.9 / 11.1, three copies, 512 / 2,048 rows 5.1 / 16.0 against 6.6 / 15.3, four copies in every step.  Rows of
+    // a single packet a thread have little to ask ahead for and take it up to `few` of them (four copies of 512 numbers, 148 /
+    // 2,048 rows: 2.0 / 12.7 against 2.1 / 11.7).
     auto kernel = mixed_streams_norm_kernel<T, 0>;
+    auto choose = [&](auto lean_kernel, auto ahead_kernel, int lean, int ahead, int few) {
+        const int wave = 148 * lean, ahead_wave = 148 * ahead;
+        const bool asks = (rows + ahead_wave - 1) / ahead_wave <= (rows + wave - 1) / wave && (p.width > 4 * kThreads || rows <= few);
+        kernel = asks ? ahead_kernel : lean_kernel;
+    };
+#define TB_COPIES(S, LEAN, FEW)                                                                                               \
+    case S: choose(mixed_streams_norm_kernel<T, S>, mixed_streams_norm_ahead_kernel<T, S>, LEAN, kAheadBlocks<S>, FEW); break
     if (packets) {
         switch (p.streams) {
-            case 1: kernel = mixed_streams_norm_kernel<T, 1>; break;
-            case 2: kernel = mixed_streams_norm_kernel<T, 2>; break;
-            case 3: kernel = mixed_streams_norm_kernel<T, 3>; break;
-            case 4: kernel = mixed_streams_norm_kernel<T, 4>; break;
-            case 5: kernel = mixed_streams_norm_kernel<T, 5>; break;
-            case 6: kernel = mixed_streams_norm_kernel<T, 6>; break;
-            case 8: kernel = mixed_streams_norm_kernel<T, 8>; break;
+            TB_COPIES(1, 5, 296);
+            TB_COPIES(2, 4, 296);
+            TB_COPIES(3, 3, 296);
+            TB_COPIES(4, 2, 148);
+            TB_COPIES(5, 2, 148);
+            TB_COPIES(6, 1, 592);
+            TB_COPIES(8, 1, 592);
             default: break;
         }
     }
+#undef TB_COPIES
     cudaError_t launched = tb_launch_pdl(kernel, dim3(rows), dim3(kThreads), (size_t)0, stream, residual, (T*)out, p);
     return launched == cudaSuccess ? tb_launch_status() : (int)launched;
 }

@@ -132,6 +132,30 @@ def test_copies_are_mixed_and_the_next_norm_taken(width, streams, out_dtype):
                 close(out, want, 2e-5 if out_dtype == torch.float32 else 1e-2, "normed rows")
 
 
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [64, 1028, 4100])
+@pytest.mark.parametrize("streams", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_stream_mixing_gives_few_rows_the_bits_of_many(streams, width, out_dtype):
+    """Steps of few rows ask for more of a row before they store, steps of many may not: the same numbers either way."""
+    from tesseract_b200 import kernels
+
+    rows = 620
+    g = torch.Generator().manual_seed(streams * width)
+    draw = lambda *shape: torch.randn(*shape, generator=g).to(dev())         # noqa: E731
+    old, a, b = draw(rows, streams * width), draw(rows, width), draw(rows, width)
+    mix, share, take, weight = draw(streams, streams), draw(streams), draw(streams), draw(width)
+
+    def run(lo, hi, update):
+        residual, out = old[lo:hi].clone(), torch.empty(hi - lo, width, dtype=out_dtype, device=dev())
+        kernels.mixed_streams_norm(residual, (a[lo:hi], 0.7, b[lo:hi], -1.3) if update else None, mix, share, take, weight, out, streams, 1e-6)
+        return torch.cat([residual, out.float()], dim=1)
+
+    for update in (True, False):
+        many = run(0, rows, update)
+        for lo, hi in ((0, 1), (300, 448), (rows - 290, rows)):
+            assert torch.equal(run(lo, hi, update), many[lo:hi])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width,copies,vocab,buckets,mul_prev,mul_cur", [(24, 1, 50, 1, 3, 4), (42, 3, 77, 97, 101, 12345),
                                                                           (256, 4, 300, 4096, 31, 7), (8, 2, 2 ** 17, 65537, 2 ** 40 + 1, 10 ** 9)])
