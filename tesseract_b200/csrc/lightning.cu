@@ -293,10 +293,11 @@ __device__ __forceinline__ void store_state(float* p, const float* v) {
 // from and to the slot; a lane V value columns, a warp every eighth key dimension, the warps' parts of S^T q summed in
 // warp order.  o = a (S^T q) + (q . k) v,  S' = a S + k v^T.  Bound by the latency of its loads where requests are few and by
 // their bandwidth where they are many, so a thread asks for HELD key dimensions before it stores one.  16 heads of
-// 128 x 128 at 1 / 8 / 32 / 64 requests: 4.3 / 6.4 / 15.6 / 25.7 us, with one number asked for at a time 5.3 / 11.6 / 24.5 / 46.2
-// (the bytes of the state at 64: 20.5).
-template <typename T, int V, int HELD>
-__global__ void __launch_bounds__(kThreads)
+// 128 x 128 at 1 / 8 / 32 / 64 requests, one launch after another on the same state: 4.3 / 4.9 / 11.0 / 18.1 us, with one number asked
+// for at a time 6.6 / 7.5 / 14.1 / 25.4.  In a decode step of many layers, the state from memory: 4.3 / 6.4 / 15.6 / 25.7 and
+// 5.3 / 11.6 / 24.5 / 46.2 (the bytes of the state at 64: 20.5).  BLOCKS: a multiprocessor, by the registers (0: as they come).
+template <typename T, int V, int HELD, int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
 lightning_step_kernel(const T* __restrict__ proj, int64_t proj_stride, int q_off, int k_off, int v_off,
                       const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ out,
                       const int* __restrict__ row_start, const int* __restrict__ state_slots, int heads, int dim, int vdim,
@@ -785,10 +786,18 @@ int launch(const void* proj, int64_t proj_stride, int q_off, int k_off, int v_of
         const int cols = packets ? 128 : 32;
         const size_t step_smem = sizeof(float) * ((size_t)2 * dim + (kThreads / 32) * cols + 1);
         if (step_smem > 40 * 1024) return TB_ERR_BAD_SIZE;
-        // Sixteen numbers asked for at once shorten the chain of a thread, eight leave room for twice the blocks: 8 requests of 16
-        // heads (128 blocks) 6.4 against 7.7 us, 32 requests 19.8 against 15.6; 64 requests of 64 x 64 18.3 against 13.0.
-        auto step = !packets ? lightning_step_kernel<T, 1, 8>
-                             : (int64_t)num_seqs * heads * (vdim / 128) <= 296 ? lightning_step_kernel<T, 4, 16> : lightning_step_kernel<T, 4, 8>;
+        // Numbers asked for at once shorten the chain of a thread and take registers, which many blocks need to run side by side.
+        // Four columns a lane: sixteen where every block has a multiprocessor (8 requests of 16 heads of 128 x 128 4.9 us, eight
+        // 6.5), else eight (16 requests 7.2, sixteen 8.3; 32 requests 11.0 and 15.0).  One column: eight up to four blocks a
+        // multiprocessor and for long columns (24 requests of 8 heads of 96 x 96 4.8, four 5.4), else four, with eight blocks a
+        // multiprocessor (64 requests of 64 heads of 64 x 64 28 us, eight 36, one after another 30; 256 of 8 of 96 x 96 28, 38, 35).
+        // A warp of a short column has no more than four.
+        const int64_t blocks = (int64_t)num_seqs * heads * ((vdim + cols - 1) / cols);
+        auto step = lightning_step_kernel<T, 1, 4, 8>;
+        if (packets)
+            step = dim <= 32 ? lightning_step_kernel<T, 4, 4, 0> : blocks <= 148 ? lightning_step_kernel<T, 4, 16, 0> : lightning_step_kernel<T, 4, 8, 0>;
+        else if (dim > 32 && (blocks <= 592 || dim >= 128))
+            step = lightning_step_kernel<T, 1, 8, 0>;
         cudaError_t launched = tb_launch_pdl(step, dim3(num_seqs, heads, (vdim + cols - 1) / cols), dim3(kThreads), step_smem, stream,
                                              (const T*)proj, proj_stride, q_off, k_off, v_off, decay, state, out, row_start,
                                              state_slots, heads, dim, vdim, act);

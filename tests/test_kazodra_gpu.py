@@ -219,6 +219,31 @@ def test_a_decoded_row_renews_every_number_of_its_state_once(dtype, d, dv):
     assert torch.equal(on[1].cpu(), state[1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,dv", [(32, 33), (33, 64), (96, 96), (128, 40), (24, 128), (40, 256), (128, 128)])
+def test_decoded_rows_of_many_requests_take_the_bits_of_few(dtype, d, dv):
+    """How much of the state a thread asks for at a time goes by the number of requests and the sizes; the sums do not."""
+    from tesseract_b200 import kernels
+
+    heads, seqs = 8, 90
+    g = torch.Generator().manual_seed(d + dv)
+    state = torch.randn(seqs, heads, d, dv, generator=g).to(dev())
+    proj = torch.randn(seqs, heads * (2 * d + dv), generator=g).to(dtype).to(dev())
+    decay = torch.linspace(0.9, 1.0, heads, device=dev())
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev())         # noqa: E731
+
+    def run(lo, hi):
+        on, out = state.clone(), torch.empty(hi - lo, heads * dv, device=dev())
+        kernels.lightning(proj[lo:hi], decay, on, out, i32(list(range(hi - lo + 1))), i32(list(range(lo, hi))), num_seqs=hi - lo, heads=heads,
+                          dim=d, vdim=dv, max_new=1)
+        return on, out
+
+    many_state, many = run(0, seqs)
+    for lo, hi in ((0, 1), (7, 23), (seqs - 3, seqs)):
+        on, out = run(lo, hi)
+        assert torch.equal(out, many[lo:hi]) and torch.equal(on[lo:hi], many_state[lo:hi]) and torch.equal(on[hi:], state[hi:])
+
+
 @pytest.mark.parametrize("decay", [1.0, 0.995])
 def test_recurrence_keeps_a_product_from_hundreds_of_tokens_back(decay):
     """One token's key and value are large and every later query points at that key; all else is small: what the rows
