@@ -34,7 +34,7 @@ __device__ __forceinline__ uint64_t twice(float a) {
 }
 
 // Stage t = 16 b + 4 c + p covers the runs i = 2p, 2p + 1 of chain c of block b; its first number of K:
-__device__ __forceinline__ int stage_start(int t) { return (t >> 4) * KBLOCK + (t & 3) * 64 + ((t >> 2) & 3) * 8; }
+__host__ __device__ __forceinline__ int stage_start(int t) { return (t >> 4) * KBLOCK + (t & 3) * 64 + ((t >> 2) & 3) * 8; }
 // The next stage that reaches into K (the others of the last block would add zeros alone).
 __device__ __forceinline__ int next_stage(int t, int stages, int K) {
     do { ++t; } while (t < stages && stage_start(t) >= K);
@@ -74,6 +74,9 @@ __device__ __forceinline__ void store_tile(const uint64_t (&total)[8][TN / 2], f
 // do not.  500 rows of 16,384 x 2,048 take 799 us (42 TFLOP/s; single-number instructions 12 % more, 64 x 64 tiles of one
 // chain of K, as before, 1,009), 2,048 rows 3.14 ms (3.92).
 // (A is not declared __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
+// The next kernel is let in when the sums are done, as in all tile kernels here: blocks that are placed while a kernel runs go to
+// where room is left, two to a multiprocessor while others stay empty.  200 rows of 2,048 x 128 in a row of such products take
+// 7.5 us, 14.9 with the next one let in at the start; 500 rows of 2,048 x 2,047 165 and 242.
 template <bool VEC, int BM, int BN, int TN>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN))
 gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
@@ -126,7 +129,6 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
         }
     };
 
-    pdl_trigger();
     pdl_wait();
     int t = 0, buffer = 0;
     fetch(t);
@@ -170,7 +172,128 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
         __syncthreads();
         t = ahead;
     }
+    pdl_trigger();
     store_tile<BM, BN, TN>(total, C, ldc, m0, n0, tx, ty, M, N);
+}
+
+// Tiles that walk K as it lies, 32 numbers a stage, with the sums of all four chains of a block side by side (a thread 4 x 4
+// outputs): a short K fills its stages, where a chain after another leaves half or three quarters of one empty.  SHORT (K <= 32):
+// a chain is eight numbers, so one sum at a time is enough and twice the threads fit.  Bound by the latency of a stage: 200 rows of
+// 2,048 x 32 take 2.9 us (the chains one after another, 7.5), 64 rows of 2,048 x 96 6.3 (7.2), 100 rows of 100 x 33 3.8 (5.0); with
+// more than two tiles a multiprocessor the registers cost more than the stages give (300 rows of 5,120 x 96: 17.5 against 14.3).
+constexpr int EK = 32;
+template <bool VEC, bool SHORT>
+__global__ void __launch_bounds__(256, SHORT ? 4 : 2)
+gemm_f32_even_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K) {
+    constexpr int P = 64 + 4;
+    __shared__ __align__(16) float As[2][EK][P];
+    __shared__ __align__(16) float Ws[2][EK][P];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+    const int stages = (K + EK - 1) / EK;
+    // a thread's packets of a stage: row (u >> 1) & 63, numbers 4 q .. 4 q + 3 (neighbouring lanes take a row's 32 bytes, and
+    // write to different banks)
+    const int row_of = (tid >> 1) & 63, q0 = (tid & 1) + 2 * (tid >> 7);
+
+    float a[2][4], w[2][4];
+    auto fetch_one = [&](const float* base, int64_t ld, int row, int rows, int kk, float* v) {
+        v[0] = v[1] = v[2] = v[3] = 0.0f;
+        if (row >= rows) return;
+        if (VEC) {
+            if (kk < K) {
+                const float4 t = *reinterpret_cast<const float4*>(base + (int64_t)row * ld + kk);
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (kk + e < K) v[e] = base[(int64_t)row * ld + kk + e];
+        }
+    };
+    auto fetch = [&](int stage) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const int kk = stage * EK + (q0 + 4 * l) * 4;
+            fetch_one(A, lda, m0 + row_of, M, kk, a[l]);
+            fetch_one(W, ldw, n0 + row_of, N, kk, w[l]);
+        }
+    };
+    auto put = [&](int buffer) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                As[buffer][(q0 + 4 * l) * 4 + e][row_of] = a[l][e];
+                Ws[buffer][(q0 + 4 * l) * 4 + e][row_of] = w[l][e];
+            }
+    };
+
+    constexpr int LIVE = SHORT ? 1 : CHAINS;       // sums of chains that are under way at a time
+    float acc[LIVE][4][4], total[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            total[i][j] = 0.0f;
+#pragma unroll
+            for (int c = 0; c < LIVE; ++c) acc[c][i][j] = 0.0f;
+        }
+    auto add_up = [&](float (&sum)[4][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                total[i][j] += sum[i][j];
+                sum[i][j] = 0.0f;
+            }
+    };
+    pdl_wait();
+    fetch(0);
+    put(0);
+    __syncthreads();
+    for (int stage = 0; stage < stages; ++stage) {
+        const int buffer = stage & 1;
+        const bool more = stage + 1 < stages;
+        if (more) fetch(stage + 1);
+#pragma unroll
+        for (int c = 0; c < CHAINS; ++c) {
+            if (stage * EK + c * 8 >= K) break;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float4 x = *reinterpret_cast<const float4*>(&As[buffer][c * 8 + e][ty * 4]);
+                const float4 y = *reinterpret_cast<const float4*>(&Ws[buffer][c * 8 + e][tx * 4]);
+                const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[SHORT ? 0 : c][i][j] = fmaf(xs[i], ys[j], acc[SHORT ? 0 : c][i][j]);
+            }
+            if (SHORT) add_up(acc[0]);
+        }
+        if (!SHORT && (stage % GROUPS == GROUPS - 1 || !more)) {       // the block ends here: its chains in order
+#pragma unroll
+            for (int c = 0; c < LIVE; ++c) add_up(acc[c]);
+        }
+        if (more) {
+            put(buffer ^ 1);
+            __syncthreads();
+        }
+    }
+    pdl_trigger();
+    const bool packets = ldc % 4 == 0 && (uintptr_t)C % 16 == 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + ty * 4 + i, n = n0 + tx * 4;
+        if (m >= M) continue;
+        float* row = C + (int64_t)m * ldc + n;
+        if (packets && n + 4 <= N) {
+            *reinterpret_cast<float4*>(row) = make_float4(total[i][0], total[i][1], total[i][2], total[i][3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < N) row[j] = total[i][j];
+        }
+    }
 }
 
 // The tiles where they are too few to give a multiprocessor more than one: G groups of threads take a tile's chains in turn (K a
@@ -222,7 +345,6 @@ gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw,
             for (int l = 0; l < LW; ++l) Ws[(q * 4 + e) * WP + l * (THREADS / 4) + row_of] = w[l][e];
         }
     };
-    pdl_trigger();
     pdl_wait();
     int t = group * 4, buffer = 0;                     // (K / 64 chains, a multiple of four: every group takes as many)
     fetch(t);
@@ -290,6 +412,7 @@ gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw,
         group_barrier();
         t = ahead;
     }
+    pdl_trigger();
     if (group > 0) return;
     store_tile<BM, BN, TN>(total, C, ldc, m0, n0, tx, ty, M, N);
 }
@@ -299,6 +422,7 @@ gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw,
 constexpr int WARPS = 8, FEATURES = 16;                // a block: 16 weight rows, eight blocks of K at a time
 constexpr int STEP = WARPS * KBLOCK;
 constexpr int AHEAD = 4;                               // groups of weights in flight a thread
+constexpr int kMostStreamed = 1024;                    // rows (a grid's second dimension is far from its limit)
 
 __device__ __forceinline__ void load8(const float* p, bool in, float* v) {
     if (in) {
@@ -312,13 +436,14 @@ __device__ __forceinline__ void load8(const float* p, bool in, float* v) {
 }
 
 // Bound by the stream of the weights up to four rows (N x K = 16,384 x 2,048: 22 us at one row, 23 at four, 5.9 TB/s; the
-// 64 x 64 tiles 189), by multiply-adds and loads of the rows from shared memory above (33 us at eight, a further 31 for
-// every eight).  2,048 x 8,192 takes 13 to 19 us up to eight rows (the tiles 581), the head of 128,256 x 2,048 at one row
-// 151 (961).  Registers hold four groups of weights in flight a thread, 128 KiB a multiprocessor.
+// 64 x 64 tiles 189): registers hold four groups of weights in flight a thread, 128 KiB a multiprocessor of two blocks.  Blocks of
+// eight rows take 160 KiB of shared memory, so that one fits a multiprocessor and half as much is in flight: 33 us, and as
+// much again for every eight rows.  2,048 x 8,192 takes 13 to 19 us up to eight rows (the tiles 581), the head of
+// 128,256 x 2,048 at one row 151 (961).
 // Lane (f, c) runs chain c of its warp's block for the weight rows f and f + 8 and ROWS rows of A.  The rows' part that
 // a warp needs lies in shared memory that only this warp writes and reads.
 template <int ROWS>
-__global__ void __launch_bounds__(WARPS * 32, 2)
+__global__ void __launch_bounds__(WARPS * 32, 2)                     // (of eight rows one block fits, by its shared memory)
 gemm_f32_rows_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
                      int K) {
     extern __shared__ __align__(16) float shared[];
@@ -438,7 +563,7 @@ cudaError_t launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw
     const cudaError_t set = cudaFuncSetAttribute(gemm_f32_rows_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (set != cudaSuccess) return set;
     const int tiles = (N + FEATURES - 1) / FEATURES, groups = (M + ROWS - 1) / ROWS;
-    const dim3 grid(tiles < 296 ? tiles : 296, groups);              // two blocks on each of the 148 multiprocessors
+    const dim3 grid(tiles < 296 ? tiles : 296, groups);              // two blocks on each of the 148 multiprocessors (of eight rows: one, in turn)
     return tb_launch_pdl(gemm_f32_rows_kernel<ROWS>, grid, dim3(WARPS * 32), bytes, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
@@ -448,6 +573,14 @@ cudaError_t launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     return tb_launch_pdl(gemm_f32_tile_kernel<VEC, BM, BN, TN>, grid, dim3((BM / 8) * (BN / TN)), 0, stream, A, lda, W, ldw,
                          C, ldc, M, N, K);
+}
+
+template <bool VEC>
+cudaError_t launch_even(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
+                        int K, cudaStream_t stream) {
+    const dim3 grid((N + 63) / 64, (M + 63) / 64);
+    auto kernel = K <= EK ? gemm_f32_even_kernel<VEC, true> : gemm_f32_even_kernel<VEC, false>;
+    return tb_launch_pdl(kernel, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
 template <int BM, int BN, int TN, int G>
@@ -463,10 +596,86 @@ cudaError_t launch_groups(const float* A, int64_t lda, const float* W, int64_t l
                          N, K);
 }
 
+// ---- which form a product takes -------------------------------------------------------------------------------------
+//
+// The one whose estimated time is least.  The estimates are fits to 3,374 products (K 1 to 8,192, N 64 to 128,256, 1 to 2,048
+// rows; operands on and off the packets' alignment), each form timed at each: 2 to 6 % off in the middle, 10 to 20 % at nine in
+// ten, and the form they pick takes 1.004 of the best one's time on average, 1.25 at worst.  Against 64 x 64 tiles of one chain
+// of K, which all products took before, a picked form is slower at some K of 33 to 127 alone, whose last stages are partly empty
+// (K = 96: up to 1.18 times; K = 48: up to 1.2 times 3.6 us), and at K of 16 or less with 128,256 features (1.11).
+
+enum Form : int { ROWS = 0, EVEN, SQUARE, TALL, SQUARE_GROUPS, TALL_GROUPS };
+
+// Microseconds: to start, a tile of a multiprocessor, and a stage where a multiprocessor has one tile / for each of several;
+// tiles that fit a multiprocessor side by side.
+struct TileCost {
+    float start, tile, one, many;
+    int side;
+};
+
+float tiles_take(const TileCost& c, int64_t tiles, int stages) {
+    const int64_t wave = 148 * c.side, whole = tiles / wave, left = (tiles % wave + 147) / 148;
+    auto stage = [&](int64_t side_by_side) { return side_by_side == 0 ? 0.0f : fmaxf(c.one, c.many * side_by_side); };
+    return c.start + c.tile * ((tiles + 147) / 148) + stages * (whole * stage(c.side) + stage(left));
+}
+
+// The streaming kernel: units of 16 features x 2,048 numbers of K, `unit` at an empty K, `full` more at a whole one, a pass over
+// the weights for every eight rows at `megabyte` a megabyte.  A unit takes nearly the same whatever part of its K is there, so
+// a short K is read as slowly as a long one: 48 rows of 2,048 x 128 take 23.1 us, as tiles 7.2.
+float rows_take(int M, int N, int K) {
+    const int which = M == 1 ? 0 : M == 2 ? 1 : M <= 4 ? 2 : 3, rows = 1 << which;
+    static const float start[4] = {0.56f, 0.32f, 0.31f, 0.2f}, wave[4] = {0.0f, 0.0f, 0.0f, 1.02f};
+    static const float unit[4] = {1.24f, 1.81f, 3.04f, 2.80f}, full[4] = {0.29f, 0.17f, 0.0f, 0.77f};
+    static const float megabyte[4] = {0.141f, 0.167f, 0.207f, 0.226f};
+    const int64_t tiles = (N + FEATURES - 1) / FEATURES, passes = (M + rows - 1) / rows;
+    const int64_t slots = which == 3 ? 148 : 296, steps = (K + STEP - 1) / STEP;      // (blocks of eight rows fill a multiprocessor)
+    const int64_t waves = ((tiles < 296 ? tiles : 296) * passes + slots - 1) / slots, units = (tiles * passes + slots - 1) / slots * steps;
+    const float mb = 4e-6f * (float)N * (float)K * passes;
+    return start[which] + fmaxf(waves * wave[which] + units * (unit[which] + full[which] * (K < STEP ? K : STEP) / STEP), megabyte[which] * mb);
+}
+
+// packets: rows of both operands start on 16 bytes and K is a multiple of four; streams: the weights' rows start on 32 bytes and K
+// is a multiple of eight as well.
+Form form_for(int M, int N, int K, bool packets, bool streams) {
+    const int64_t across = (N + 63) / 64, square = (M + 63) / 64 * across, tall = (M + 127) / 128 * across;
+    int stages = 0;                                // of 16 numbers of K, chain after chain
+    for (int t = 0; t < 16; ++t) stages += stage_start(t) < K % KBLOCK;
+    stages += K / KBLOCK * 16;
+    Form best = K <= EK ? EVEN : SQUARE;
+    float least = 0.0f;
+    if (K <= EK)
+        least = packets ? 0.56f + 0.06f * K + fmaxf(0.55f, 0.0055f * square) : 1.4f + 0.12f * K + fmaxf(0.2f, 0.00435f * square);
+    else
+        least = tiles_take(packets ? TileCost{1.65f, 0.04f, 0.66f, 0.504f, 4} : TileCost{1.2f, 0.49f, 0.85f, 0.71f, 4}, square, stages);
+    auto consider = [&](Form form, float takes) {
+        if (takes < least) {
+            least = takes;
+            best = form;
+        }
+    };
+    if (K > EK) {
+        if ((K < KBLOCK || !packets) && square <= 296)
+            consider(EVEN, tiles_take(packets ? TileCost{0.85f, 0.14f, 1.49f, 1.26f, 2} : TileCost{0.17f, 0.0f, 1.69f, 1.46f, 2}, square, (K + EK - 1) / EK));
+        consider(TALL, tiles_take(packets ? TileCost{2.0f, 0.51f, 0.964f, 0.835f, 2} : TileCost{2.06f, 0.0f, 1.256f, 1.105f, 2}, tall, stages));
+        if (packets && K % KBLOCK == 0) {
+            consider(SQUARE_GROUPS, tiles_take(TileCost{0.0f, 1.72f, 0.487f, 0.526f, 1}, square, stages));
+            consider(TALL_GROUPS, tiles_take(TileCost{0.0f, 1.48f, 0.905f, 0.905f, 1}, tall, stages));
+        }
+    }
+    if (streams && M <= kMostStreamed) consider(ROWS, rows_take(M, N, K));
+    return best;
+}
+
 }  // namespace
 
+// The form that tb_gemm_f32_nt takes: 0 streamed rows, 1 even tiles, 2 square tiles, 3 tall tiles, 4 and 5 those whose chains
+// groups of threads share.
+TB_EXPORT int tb_gemm_f32_form(int M, int N, int K, int packets, int streams) {
+    return M < 1 || N < 1 || K < 1 ? -1 : (int)form_for(M, N, K, packets != 0, streams != 0);
+}
+
 // Zero padding inside a chain adds exact zeros, which leaves every partial sum unchanged, so the guarded and the packet
-// paths and both kernels give the same bits.
+// paths and all kernels give the same bits.
 TB_EXPORT int tb_gemm_f32_nt(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc,
                              int M, int N, int K, cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
@@ -474,27 +683,25 @@ TB_EXPORT int tb_gemm_f32_nt(const float* A, int64_t lda, const float* W, int64_
     if ((M + 63) / 64 > 65535) return TB_ERR_BAD_SIZE;
     const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (ldw % 4 == 0) && ((uintptr_t)A % 16 == 0) &&
                      ((uintptr_t)W % 16 == 0);
-    const int64_t tall = (int64_t)((M + 127) / 128) * ((N + 63) / 64), square = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
-    // Streaming passes over the weights once for every eight rows, a tile takes 0.7 us for sixteen numbers of K whatever
-    // else runs.  At N x K = 16,384 x 2,048 the two meet near 50 rows (32: 126 against 198 us, 64: 248 against 229); with
-    // few tiles later (3,072 x 2,048, 64 rows: 54 against 100; 2,048 x 8,192, 64 rows: 109 against 398; 2,048 x 2,048,
-    // 200 rows, 128 tiles: 112 against 94).  A short K leaves most of a streaming block's warps without work.
-    const bool stream_weights = M <= 48 || (square <= 80 && K >= STEP);
-    if (stream_weights && vec && K % 8 == 0 && ldw % 8 == 0 && (uintptr_t)W % 32 == 0) {
-        if (M == 1) return (int)launch_rows<1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        if (M == 2) return (int)launch_rows<2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        if (M <= 4) return (int)launch_rows<4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-        return (int)launch_rows<8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    const bool streams = vec && K % 8 == 0 && ldw % 8 == 0 && (uintptr_t)W % 32 == 0;
+    switch (form_for(M, N, K, vec, streams)) {
+        case ROWS:
+            if (M == 1) return (int)launch_rows<1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+            if (M == 2) return (int)launch_rows<2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+            if (M <= 4) return (int)launch_rows<4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+            return (int)launch_rows<8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        case EVEN:
+            return (int)(vec ? launch_even<true>(A, lda, W, ldw, C, ldc, M, N, K, stream)
+                             : launch_even<false>(A, lda, W, ldw, C, ldc, M, N, K, stream));
+        case SQUARE:
+            return (int)(vec ? launch_tile<true, 64, 64, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream)
+                             : launch_tile<false, 64, 64, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream));
+        case TALL:
+            return (int)(vec ? launch_tile<true, 128, 64, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream)
+                             : launch_tile<false, 128, 64, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream));
+        case SQUARE_GROUPS:
+            return (int)launch_groups<64, 64, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+        default:
+            return (int)launch_groups<128, 64, 8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
     }
-    if (!vec) return (int)launch_tile<false, 64, 64, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    // One tile a multiprocessor: groups of threads share its chains.  200 rows of 2,048 x 2,048 (128 square tiles) 94 -> 72 us,
-    // 160 of 3,072 x 2,048 171 -> 72, 64 rows of 16,384 x 2,048 (tall tiles would be half empty) 220 -> 158; 380 rows of
-    // 3,072 x 2,048 (144 tall tiles) 188 -> 130, 500 of 2,048 x 2,048 203 -> 121.  With more tiles two of one group share a
-    // multiprocessor, which is faster (380 rows of 16,384 x 2,048: 684 against 787).
-    if (K % KBLOCK == 0 && (square <= 148 || M <= 64)) return (int)launch_groups<64, 64, 8, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    if (K % KBLOCK == 0 && tall <= 148) return (int)launch_groups<128, 64, 8, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    // Tall tiles load less from shared memory for a product but leave the chip emptier: 200 rows of 2,048 x 2,048 (64 of
-    // them) take 139 us, as square tiles 94; 380 rows (96) 141 against 145, and 547 against 566 at K = 8,192.
-    if (tall >= 96) return (int)launch_tile<true, 128, 64, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    return (int)launch_tile<true, 64, 64, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
 }

@@ -150,3 +150,38 @@ def test_attention_over_cached_latents_goes_to_the_tensor_cores_for_the_sizes_it
     assert plan.latent_attention(torch.bfloat16, 160, 128) == "attention_latent_mma"
     assert plan.latent_attention(torch.bfloat16, 128, 96) == "attention_masked"        # a size it is not built for
     assert plan.latent_attention(torch.float32, 576, 512) == "attention_masked"        # the true 32-bit path
+
+
+def test_32_bit_products_take_the_form_that_was_measured_fastest():
+    """Which kernel a 32-bit product takes, asked of the library: a short K is not streamed past few rows, operands off their
+    alignment and K of any remainder find a form, and the sizes of the 1B model keep theirs."""
+    import ctypes
+
+    from tesseract_b200.csrc.build import load_library
+
+    ROWS, EVEN, SQUARE, TALL, SQUARE_GROUPS, TALL_GROUPS = range(6)
+    ask = load_library("gemm_f32").tb_gemm_f32_form
+
+    def form(m, n, k, packets=True, streams=True):
+        return ask(*(ctypes.c_int(v) for v in (m, n, k, packets, streams)))
+
+    # a unit of the streaming kernel takes as long for 128 numbers of K as for 2,048: few rows and few features alone
+    for n in (2048, 8192, 32768):
+        for k in (16, 32, 64, 128):
+            for rows in (12, 16, 17, 24, 32, 40, 48):
+                assert form(rows, n, k) in (EVEN, SQUARE, TALL), (rows, n, k)
+    assert form(48, 32768, 1024) != ROWS and form(32, 2048, 256) != ROWS
+    for rows in (1, 2, 4, 8, 16):
+        for n, k in ((2048, 2048), (16384, 2048), (2048, 8192), (3072, 2048), (128256, 2048)):
+            assert form(rows, n, k) == ROWS, (rows, n, k)
+    # one tile a multiprocessor or fewer: groups of threads where K is a multiple of 256; tall tiles where many fill the chip
+    assert form(200, 2048, 2048) == SQUARE_GROUPS and form(380, 3072, 2048) == TALL_GROUPS
+    assert form(500, 16384, 2048) == TALL and form(2048, 16384, 2048) == TALL
+    # nothing of that needs alignment that is not there
+    for rows in (1, 8, 48, 200, 2048):
+        for n, k in ((2048, 2047), (100, 33), (64, 1), (8192, 1023)):
+            assert form(rows, n, k, False, False) in (EVEN, SQUARE, TALL)
+            assert form(rows, n, k + 4 - k % 4, True, False) != ROWS
+    for rows, n, k in itertools.product((1, 3, 300, 5000), (1, 17, 4000, 128256), (1, 2, 31, 32, 33, 255, 256, 257, 8192)):
+        assert ROWS <= form(rows, n, k, k % 4 == 0, k % 8 == 0) <= TALL_GROUPS
+    assert form(0, 1, 1) == form(1, 0, 1) == form(1, 1, 0) == -1

@@ -124,6 +124,18 @@ def test_gemm_f32_streams_and_tiles_sum_in_one_order(m, n, k):
     assert torch.equal(guarded, out)
 
 
+@pytest.mark.parametrize("m, n, k", [
+    (65, 130, 8), (1, 200, 32), (67, 129, 32), (67, 129, 31),        # tiles that walk K as it lies, K within a stage
+    (48, 2048, 128), (70, 300, 40), (33, 140, 255), (131, 100, 300), # the same over several stages and blocks (300: guarded)
+    (131, 2100, 200), (40, 8200, 1000), (500, 2048, 264),            # square tiles
+    (700, 2700, 40), (1000, 3000, 96), (300, 3072, 1000),            # tall tiles, with packets and guarded
+    (2048, 128, 512),                                                # groups of threads, many rows of few features
+])
+def test_gemm_f32_forms_sum_in_one_order(m, n, k):
+    """The forms that the sizes above do not reach, on and off the packets' alignment."""
+    test_gemm_f32_streams_and_tiles_sum_in_one_order(m, n, k)
+
+
 def test_gemm_f32_is_true_32_bit():
     """A product that a reduced-precision matrix mode (10-bit mantissa) would get visibly wrong."""
     from tesseract_b200 import kernels
