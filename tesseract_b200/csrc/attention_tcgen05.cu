@@ -19,8 +19,8 @@
 // cp.async.bulk.tensor over a five-dimensional tensor map of the cache (no multicast); one lane of warp 4 issues
 // the tensor-core instructions.  Roles meet on mbarriers; every wait is bounded, and a wait that
 // runs out sets *error, stops the other roles, and the CTA still frees its tensor memory.
-// Two CTAs fit on an SM (112 KiB of shared memory and 256 tensor-memory columns each), so one CTA's softmax
-// overlaps the other's products.
+// Two CTAs fit on an SM (112 KiB of shared memory at head_dim 64, 96 KiB at 128, and 256 tensor-memory columns each), so
+// one CTA's softmax overlaps the other's products.
 #include "tma.cuh"
 
 namespace {
@@ -29,17 +29,18 @@ using namespace tbtma;
 
 constexpr int BM = 128;          // folded query rows per CTA
 // Keys per block for head_dim 64: 128, two CTAs per SM (64 with three CTAs per SM was faster only beyond some 4,000
-// tokens of context).  head_dim 128 takes 64 keys per block, which lets two CTAs share an SM (112 KiB of shared
-// memory and 256 tensor-memory columns each).
+// tokens of context).  head_dim 128 takes 64 keys per block, which lets two CTAs share an SM (96 KiB of shared memory and
+// 256 tensor-memory columns each).
 constexpr int kBlockKeys64 = 128;
 constexpr int STAGES = 2;        // K/V ring depth
 constexpr int kThreads = 192;         // warps 0..3 softmax, warp 4 issuer, warp 5 TMA producer
 // A swizzled tile of 128 rows x 64 bfloat16 (128 bytes a row): the unit that Q, P, K and V tiles are made of.  A Q
-// tile is D / 64 of them side by side (dims 0..63 | 64..127), a P tile BN / 64 (keys 0..63 | 64..127); K and V
+// tile is D / 64 of them side by side (dims 0..63 | 64..127), a P tile in shared memory two (keys 0..63 | 64..127); K and V
 // blocks are D / 64 tiles of BN rows each.
 constexpr uint32_t kTileBytes = BM * 128;
 template <int D, int BN>
 struct Shape {
+    static_assert((D == 64 && BN == 128) || (D == 128 && BN == 64), "the two forms that the kernel's loops are written for");
     static constexpr uint32_t kQBytes = (D / 64) * kTileBytes;
     // blocks of 64 keys: the probabilities go to tensor memory, in two buffers of BN / 2 columns behind O, and are the first operand
     // of P . V from there
@@ -209,12 +210,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // 2^x for a pair of lanes on the FMA pipe, for x <= 8 or so (the softmax's exponents): the special-function unit
 // gives 16 results a cycle and SM, which bounds the unmasked blocks' loop once two CTAs share an SM, so at head
 // size 64 every fourth pair of a row goes this way (2 to 5 % faster; every third or second pair is slower again,
-// and so is any share at head size 128, whose blocks have more products per exponential).  x = n + f with n the
+// and so was any share at head size 128, whose blocks have more products per exponential).  x = n + f with n the
 // nearest integer (the low mantissa bits of x + 1.5 * 2^23) and f in [-0.5, 0.5]; 2^f by a cubic (largest
 // relative error 7.5e-5, far below the rounding of the probabilities to bfloat16); n is added into the exponent
 // field.  All of it in 32-bit arithmetic.
-template <int D>
-constexpr int kPolyEvery = D == 64 ? 4 : 0;
+constexpr int kPolyEvery = 4;
 __device__ __forceinline__ void exp2_pair_fma(uint64_t x2, float& p0, float& p1) {
     float x0, x1;
     unpack2(x2, x0, x1);
@@ -437,7 +437,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                     issue_qk(qs);
                     next_q();
                 }
-                // P_j is in shared memory (and O has been rescaled if the maximum jumped): O += P_j V_j
+                // P_j is stored (and O has been rescaled if the maximum jumped): O += P_j V_j
                 if (!mbar_wait(v_full + 8 * s, parity, &abort_flag)) { ok = false; break; }
                 if (!mbar_wait(p_ready(j), phase(j), &abort_flag)) { ok = false; break; }
                 tc_fence_after();
@@ -605,16 +605,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                         sc[c][i >> 1] = 0u;
                         continue;
                     }
-                    const uint64_t x2 = fma2(pack2(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2);
-                    constexpr int kEvery = kPolyEvery<D> > 0 ? kPolyEvery<D> : 1;
-                    if (kPolyEvery<D> > 0 && (i >> 1) % kEvery == kEvery - 1) {
-                        exp2_pair_fma(x2, p0, p1);
-                    } else {
-                        float t0, t1;
-                        unpack2(x2, t0, t1);
-                        p0 = fast_exp2(t0);
-                        p1 = fast_exp2(t1);
-                    }
+                    float t0, t1;
+                    unpack2(fma2(pack2(__uint_as_float(sc[c][i]), __uint_as_float(sc[c][i + 1])), scale2, neg_m2), t0, t1);
+                    p0 = fast_exp2(t0);
+                    p1 = fast_exp2(t1);
                     ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
                     sc[c][i >> 1] = pack_bf16(p0, p1);
                 }
@@ -656,8 +650,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                     for (int i = 0; i < 32; i += 2) {
                         const uint64_t x2 = fma2(pack2(__uint_as_float(chunk[i]), __uint_as_float(chunk[i + 1])), scale2, neg_m2);
                         float p0, p1;
-                        constexpr int kEvery = kPolyEvery<D> > 0 ? kPolyEvery<D> : 1;
-                        if (kPolyEvery<D> > 0 && (i >> 1) % kEvery == kEvery - 1) {
+                        if ((i >> 1) % kPolyEvery == kPolyEvery - 1) {
                             exp2_pair_fma(x2, p0, p1);
                         } else {
                             float t0, t1;
@@ -676,36 +669,31 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
                         *reinterpret_cast<uint4*>(dst + sw128(r, (c & 1) * 4 + q4)) =
                             make_uint4(packed[q4 * 4], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
                 };
-                constexpr int kLast = BN / 32 - 1;                 // the chunk whose maxima decide
                 tmem_load_32_nowait(tmem_s + lane_base, ca);
                 tmem_wait_ld();
                 tmem_load_32_nowait(tmem_s + lane_base + 32, cb);
                 maxima(ca);
                 exps(ca, held);
                 tmem_wait_ld();
-                if (BN == 128) {
-                    tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
-                    maxima(cb);
-                    exps(cb, held + 16);
-                }
+                tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
+                maxima(cb);
+                exps(cb, held + 16);
                 if (!mbar_wait(o_full(j - 1), phase(j - 1), &abort_flag)) { ok = false; break; }
                 store(held, 0);
-                if (BN == 128) {
-                    store(held + 16, 1);
-                    tmem_wait_ld();
-                    tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
-                    maxima(ca);
-                    exps(ca, held);
-                    store(held, 2);
-                    tmem_wait_ld();
-                }
-                maxima(cb);
+                store(held + 16, 1);
+                tmem_wait_ld();
+                tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
+                maxima(ca);
+                exps(ca, held);
+                store(held, 2);
+                tmem_wait_ld();
+                maxima(cb);                                        // (the chunk whose maxima decide)
                 const float seen = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
                 if (!__any_sync(0xffffffffu, seen > m + 8.0f)) {
                     tc_fence_before();
                     mbar_arrive(s_free);               // S has been read: the issuer may start the next block's scores
                     exps(cb, held);
-                    store(held, kLast);
+                    store(held, 3);
                     float lo_sum, hi_sum;
                     unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), lo_sum, hi_sum);
                     l += lo_sum + hi_sum;
@@ -758,17 +746,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             tmem_load_32_nowait(tmem_s + lane_base + 32, cb);
             reduce_max(ca, 0);
             tmem_wait_ld();
-            if (BN == 128) {
-                tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
-                reduce_max(cb, 1);
-                tmem_wait_ld();
-                tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
-                reduce_max(ca, 2);
-                tmem_wait_ld();
-                reduce_max(cb, 3);
-            } else {
-                reduce_max(cb, 1);
-            }
+            tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
+            reduce_max(cb, 1);
+            tmem_wait_ld();
+            tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
+            reduce_max(ca, 2);
+            tmem_wait_ld();
+            reduce_max(cb, 3);
             const float raw_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             const float block_max = raw_max > 0.5f * kMasked ? raw_max * p.scale_log2 : kMasked;
             // P_{j-1} V_{j-1} must be complete before the P tile is overwritten (and before O is rescaled)
@@ -835,21 +819,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap cache_map, const Tc
             tmem_load_32_nowait(tmem_s + lane_base + 32, cb);
             emit(ca, 0);
             tmem_wait_ld();
-            if (BN == 128) {
-                tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
-                emit(cb, 1);
-                tmem_wait_ld();
-                tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
-                emit(ca, 2);
-                tmem_wait_ld();
-                tc_fence_before();
-                mbar_arrive(s_free);                   // S has been read: the issuer may start the next block's scores
-                emit(cb, 3);
-            } else {
-                tc_fence_before();
-                mbar_arrive(s_free);
-                emit(cb, 1);
-            }
+            tmem_load_32_nowait(tmem_s + lane_base + 64, ca);
+            emit(cb, 1);
+            tmem_wait_ld();
+            tmem_load_32_nowait(tmem_s + lane_base + 96, cb);
+            emit(ca, 2);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(s_free);                   // S has been read: the issuer may start the next block's scores
+            emit(cb, 3);
             {
                 float lo, hi;
                 unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), lo, hi);
