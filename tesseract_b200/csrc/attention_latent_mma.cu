@@ -322,7 +322,7 @@ attention_latent_shared_kernel(const bf16* q, int64_t q_stride, bf16* out, int64
         const int pos = pos_first + (mine ? own - begin : 0);
         const int key_lo = first_key(pos), shift = key_lo - block_lo;      // 0 .. ROWS - 1
         const int own_tiles = mine ? (pos - key_lo) / KT + 1 : 0;
-        const int tiles = max((pos_last - first_key(pos_last)) / KT, (pos_last - block_lo - (count - 1)) / KT) + 1;
+        const int tiles = (pos_last - first_key(pos_last)) / KT + 1;       // (a run's last row sees the most keys)
         const int* table = block_table + (int64_t)seq * bt_stride;
         auto fill = [&](int tile) {                                        // a warp a key
             const uint32_t stage = base + (uint32_t)(tile & 1) * L::STAGE;
