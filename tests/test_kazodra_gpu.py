@@ -94,11 +94,38 @@ def test_norms_around_an_addition(width, out_dtype):
     close(out, plain.layer_norm(x.double(), w2.double(), b2.double(), eps), TOL[out_dtype], "norm alone")
 
 
-@pytest.mark.parametrize("width", [256, 768, 3328, 8192, 8448])
+@pytest.mark.parametrize("width", [4, 100, 132, 252, 256, 768, 3328, 8192, 8448])
 def test_norms_around_an_addition_with_the_row_in_registers(width):
-    """The smallest and largest rows that a block holds in registers, warps that are no power of two, and the width behind."""
+    """The smallest and largest rows that a block holds in registers, threads without a second packet or without any, and the
+    width behind."""
     test_norms_around_an_addition(width, torch.float32)
     test_norms_around_an_addition(width, torch.bfloat16)
+
+
+@pytest.mark.parametrize("width", [8, 104, 136, 256, 768, 2048, 3328, 8192])
+def test_a_row_in_registers_keeps_the_bits_of_one_in_shared_memory(width):
+    """A norm over parts on the other side of the addition takes the kernel that holds the row in shared memory: what both
+    kernels compute is the same to the bit."""
+    from tesseract_b200 import kernels
+
+    g = torch.Generator().manual_seed(width)
+    rows, eps = 13, 1e-5
+    x = (torch.randn(rows, width, generator=g) * 3.0 + 1.5).to(dev())
+    update = (torch.randn(rows, width, generator=g) * 20.0 - 4.0).to(dev())
+    w1, b1, w2 = (torch.randn(width, generator=g).to(dev()) for _ in range(3))
+    halves = (kernels.NORM_RMS, w2, None, 2)
+    out = torch.empty_like(x)
+    for norm in ((kernels.NORM_LAYER, w1, b1), (kernels.NORM_RMS, w1, None)):
+        held, shared = x.clone(), x.clone()
+        kernels.norm_add_norm(held, update, norm, None, None, None, eps)
+        kernels.norm_add_norm(shared, update, norm, halves, out, None, eps)
+        assert torch.equal(held, shared)
+        for dtype in (torch.float32, torch.bfloat16):
+            from_shared, from_held = (torch.empty(rows, width, dtype=dtype, device=dev()) for _ in range(2))
+            stream = x.clone()
+            kernels.norm_add_norm(stream, update, halves, norm, from_shared, None, eps)
+            kernels.norm_add_norm(stream, None, None, norm, from_held, None, eps)
+            assert torch.equal(from_held, from_shared)
 
 
 @pytest.mark.parametrize("width", [7, 64, 200, 4096])
@@ -319,7 +346,7 @@ def test_long_portions_as_products_of_blocks(dtype, heads, d, dv):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,d,dv", [(3, 8, 12), (2, 64, 64), (1, 128, 33), (2, 5, 40)])
-def test_long_portions_side_side_by_side_continue_each_sequence_from_its_slot(dtype, heads, d, dv):
+def test_long_portions_side_by_side_continue_each_sequence_from_its_slot(dtype, heads, d, dv):
     """A step with prompt portions of several chunks (whose chunks run side by side and meet in a scan) beside a single
     row and a short portion, every sequence from a state of its own in a slot of its own; then a second step of the same
     sequences goes on from what the first left."""
