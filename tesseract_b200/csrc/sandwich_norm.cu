@@ -231,8 +231,10 @@ __device__ __forceinline__ void held_statistics(const float (&v)[2][4], const bo
 
 // The same work, to the bit, with the row in registers, two packets of four a thread, for whole-row norms of up to 8,192
 // numbers (what the largest block holds).  Bound by the chain of a launch: the vectors of both norms are asked for before the
-// wait, the stream and the update together behind it, and a sum costs one barrier instead of two.  8 rows of 2,048, two layer
-// norms (a decode step): 2.6 us, with the row in shared memory 4.8; 2,048 rows: 13.3 and 15.9.
+// wait, the stream and the update together behind it, and a sum costs one barrier instead of two.  8 rows, two layer norms (a decode
+// step), 256 / 2,048 / 4,096 / 8,192 numbers: 2.4 / 2.6 / 2.9 / 4.0 us, with the row in shared memory 4.6 / 5.0 / 5.6 / 7.1; 2,048
+// rows: 3.9 / 13.3 / 28.4 / 72.7 and 6.0 / 15.9 / 32.4 / 77.2.  (Blocks of 1,024 threads leave 64 registers, which spills 16 to
+// 24 bytes a thread; that is in the last pair of figures.)
 template <typename T>
 __global__ void __launch_bounds__(1024)
 norm_add_norm_held_kernel(float* res, const float* upd, int post_kind, const float* __restrict__ post_w,
