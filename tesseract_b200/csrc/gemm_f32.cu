@@ -73,10 +73,10 @@ __device__ __forceinline__ void store_tile(const uint64_t (&total)[8][TN / 2], f
 // (the path is 76 % busy, the multiply-add pipe 61 %) where the tiles fill the chip, by the latency of a stage where they
 // do not.  500 rows of 16,384 x 2,048 take 799 us (42 TFLOP/s; single-number instructions 12 % more, 64 x 64 tiles of one
 // chain of K, as before, 1,009), 2,048 rows 3.14 ms (3.92).
-// (A is not declared __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
-// The next kernel is let in when the sums are done, as in all tile kernels here: blocks that are placed while a kernel runs go to
-// where room is left, two to a multiprocessor while others stay empty.  200 rows of 2,048 x 128 in a row of such products take
-// 7.5 us, 14.9 with the next one let in at the start; 500 rows of 2,048 x 2,047 165 and 242.
+// Blocks that are placed while the kernel in front still runs go to where room is left, two or four to a multiprocessor while
+// others stay empty.  So where several fit, these kernels start the ordinary way, behind the kernel in front (39 rows of
+// 16,384 x 2,048 in a layer of the 1B sizes: 117 us less than as a programmatic dependent), and let the next one in when the sums
+// are done (200 rows of 2,048 x 128 one after another 7.8 us, 14.9 with the next one let in at the start).
 template <bool VEC, int BM, int BN, int TN>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN))
 gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
@@ -129,7 +129,6 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
         }
     };
 
-    pdl_wait();
     int t = 0, buffer = 0;
     fetch(t);
     put(0);
@@ -247,7 +246,6 @@ gemm_f32_even_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
                 sum[i][j] = 0.0f;
             }
     };
-    pdl_wait();
     fetch(0);
     put(0);
     __syncthreads();
@@ -302,6 +300,7 @@ gemm_f32_even_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
 // from one another.   128 x 64
 // tiles of two groups and 64 x 64 tiles of four take 121 and 72 us for K = 2,048 (one group, where a multiprocessor has one tile:
 // 141 and 95).
+// (A is not declared __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
 template <int BM, int BN, int TN, int G>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN) * G, 1)
 gemm_f32_groups_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N, int K) {
@@ -567,12 +566,13 @@ cudaError_t launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw
     return tb_launch_pdl(gemm_f32_rows_kernel<ROWS>, grid, dim3(WARPS * 32), bytes, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
+// (not as programmatic dependents: see the kernels)
 template <bool VEC, int BM, int BN, int TN>
 cudaError_t launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
                         int K, cudaStream_t stream) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    return tb_launch_pdl(gemm_f32_tile_kernel<VEC, BM, BN, TN>, grid, dim3((BM / 8) * (BN / TN)), 0, stream, A, lda, W, ldw,
-                         C, ldc, M, N, K);
+    gemm_f32_tile_kernel<VEC, BM, BN, TN><<<grid, (BM / 8) * (BN / TN), 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
+    return cudaGetLastError();
 }
 
 template <bool VEC>
@@ -580,7 +580,8 @@ cudaError_t launch_even(const float* A, int64_t lda, const float* W, int64_t ldw
                         int K, cudaStream_t stream) {
     const dim3 grid((N + 63) / 64, (M + 63) / 64);
     auto kernel = K <= EK ? gemm_f32_even_kernel<VEC, true> : gemm_f32_even_kernel<VEC, false>;
-    return tb_launch_pdl(kernel, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
+    kernel<<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
+    return cudaGetLastError();
 }
 
 template <int BM, int BN, int TN, int G>
