@@ -74,9 +74,10 @@ __device__ __forceinline__ void store_tile(const uint64_t (&total)[8][TN / 2], f
 // do not.  500 rows of 16,384 x 2,048 take 799 us (42 TFLOP/s; single-number instructions 12 % more, 64 x 64 tiles of one
 // chain of K, as before, 1,009), 2,048 rows 3.14 ms (3.92).
 // Blocks that are placed while the kernel in front still runs go to where room is left, two or four to a multiprocessor while
-// others stay empty.  So where several fit, these kernels start the ordinary way, behind the kernel in front (39 rows of
-// 16,384 x 2,048 in a layer of the 1B sizes: 117 us less than as a programmatic dependent), and let the next one in when the sums
-// are done (200 rows of 2,048 x 128 one after another 7.8 us, 14.9 with the next one let in at the start).
+// others stay empty.  So blocks that would fit beyond an even share are kept off by the shared memory they ask for (spread() below:
+// 39 rows of 16,384 x 2,048 in a layer of the 1B sizes 117 us less), and the next kernel is let in when the sums are done (200 rows
+// of 2,048 x 128 one after another 7.5 us, 14.9 with the next one let in at the start).
+// (A is not declared __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
 template <bool VEC, int BM, int BN, int TN>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN))
 gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
@@ -129,6 +130,7 @@ gemm_f32_tile_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
         }
     };
 
+    pdl_wait();
     int t = 0, buffer = 0;
     fetch(t);
     put(0);
@@ -246,6 +248,7 @@ gemm_f32_even_kernel(const float* A, int64_t lda, const float* W, int64_t ldw, f
                 sum[i][j] = 0.0f;
             }
     };
+    pdl_wait();
     fetch(0);
     put(0);
     __syncthreads();
@@ -566,13 +569,26 @@ cudaError_t launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw
     return tb_launch_pdl(gemm_f32_rows_kernel<ROWS>, grid, dim3(WARPS * 32), bytes, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
-// (not as programmatic dependents: see the kernels)
+// Shared memory to ask for beyond a block's `own`, so that no multiprocessor takes more than its share of the tiles (`side`: the blocks
+// that fit without).
+template <typename Kernel>
+cudaError_t spread(Kernel kernel, int64_t tiles, int side, int own, size_t& extra) {
+    const int64_t share = (tiles + 147) / 148;
+    extra = 0;
+    if (share >= side) return cudaSuccess;
+    extra = (size_t)(228 * 1024 / (share + 1) + 1024 - own);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)extra);
+}
+
 template <bool VEC, int BM, int BN, int TN>
 cudaError_t launch_tile(const float* A, int64_t lda, const float* W, int64_t ldw, float* C, int64_t ldc, int M, int N,
                         int K, cudaStream_t stream) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_f32_tile_kernel<VEC, BM, BN, TN><<<grid, (BM / 8) * (BN / TN), 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
-    return cudaGetLastError();
+    auto kernel = gemm_f32_tile_kernel<VEC, BM, BN, TN>;
+    size_t extra;
+    const cudaError_t set = spread(kernel, (int64_t)grid.x * grid.y, BM == 64 ? 4 : 2, 2 * BK * (BM + BN + 8) * 4, extra);
+    if (set != cudaSuccess) return set;
+    return tb_launch_pdl(kernel, grid, dim3((BM / 8) * (BN / TN)), extra, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
 template <bool VEC>
@@ -580,8 +596,10 @@ cudaError_t launch_even(const float* A, int64_t lda, const float* W, int64_t ldw
                         int K, cudaStream_t stream) {
     const dim3 grid((N + 63) / 64, (M + 63) / 64);
     auto kernel = K <= EK ? gemm_f32_even_kernel<VEC, true> : gemm_f32_even_kernel<VEC, false>;
-    kernel<<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);
-    return cudaGetLastError();
+    size_t extra;
+    const cudaError_t set = spread(kernel, (int64_t)grid.x * grid.y, K <= EK ? 4 : 2, 4 * EK * (64 + 4) * 4, extra);
+    if (set != cudaSuccess) return set;
+    return tb_launch_pdl(kernel, grid, dim3(256), extra, stream, A, lda, W, ldw, C, ldc, M, N, K);
 }
 
 template <int BM, int BN, int TN, int G>
