@@ -570,14 +570,14 @@ cudaError_t launch_rows(const float* A, int64_t lda, const float* W, int64_t ldw
 }
 
 // Shared memory to ask for beyond a block's `own`, so that no multiprocessor takes more than its share of the tiles (`side`: the blocks
-// that fit without).
+// that fit without).  The kernel is allowed the most that any product asks for, whatever this one does: another thread's may be
+// on its way.
 template <typename Kernel>
 cudaError_t spread(Kernel kernel, int64_t tiles, int side, int own, size_t& extra) {
+    auto beyond = [&](int64_t share) { return (int)(228 * 1024 / (share + 1) + 1024 - own); };
     const int64_t share = (tiles + 147) / 148;
-    extra = 0;
-    if (share >= side) return cudaSuccess;
-    extra = (size_t)(228 * 1024 / (share + 1) + 1024 - own);
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)extra);
+    extra = share < side ? beyond(share) : 0;
+    return extra == 0 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, beyond(1));
 }
 
 template <bool VEC, int BM, int BN, int TN>

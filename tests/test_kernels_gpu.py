@@ -136,6 +136,41 @@ def test_gemm_f32_forms_sum_in_one_order(m, n, k):
     test_gemm_f32_streams_and_tiles_sum_in_one_order(m, n, k)
 
 
+def test_gemm_f32_from_several_threads():
+    """Products that ask for different shares of a multiprocessor's shared memory, issued side by side on streams of their own."""
+    import threading
+
+    from tesseract_b200 import kernels
+
+    torch.manual_seed(5)
+    sizes = [(128, 2048, 200), (200, 4096, 200), (300, 8192, 200), (130, 2048, 40), (256, 4096, 40)]       # one, two and more tiles each
+    cases = []
+    for m, n, k in sizes:
+        a, w = dev(torch.randn(m, k)), dev(torch.randn(n, k))
+        cases.append((a, w, kernels.gemm_f32_nt(a, w, torch.empty(m, n, device="cuda"))))
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(a, w, want):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                out = torch.empty_like(want)
+                for _ in range(300):
+                    kernels.gemm_f32_nt(a, w, out)
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(out, want):
+                    failures.append("other numbers")
+        except Exception as error:                   # (a refused launch)
+            failures.append(repr(error))
+
+    threads = [threading.Thread(target=work, args=case) for case in cases]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures, failures
+
+
 def test_gemm_f32_is_true_32_bit():
     """A product that a reduced-precision matrix mode (10-bit mantissa) would get visibly wrong."""
     from tesseract_b200 import kernels
