@@ -26,6 +26,7 @@ from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from .. import kernels
 from ..parts.base import CacheBinding, PagedNeed, StateNeed
 from .pages import OutOfPages, PagePool, StateSlots
 
@@ -148,10 +149,9 @@ class CacheManager:
             return False
         slot = self.slots.allocate(request)
         assert slot is not None
+        self._clear_state(slot)                      # a new request starts from empty state
         for g in self.groups:
             if g.pool is None:
-                if g.storage is not None:
-                    g.storage[:, slot].zero_()       # a new request starts from empty state
                 continue
             if reserve_tokens is None:
                 g.pool.register(request)
@@ -162,6 +162,14 @@ class CacheManager:
         self._requests[request] = _Request(slot=slot, pages=[{} for _ in self.groups],
                                            first_live=[0 for _ in self.groups])
         return True
+
+    def _clear_state(self, slot: int) -> None:
+        stores = [g.storage for g in self.groups if g.pool is None and g.storage is not None and g.storage.numel()]
+        if stores and all(s.is_cuda and s.device.index == torch.cuda.current_device() for s in stores):
+            kernels.clear_slot(stores, slot)
+        else:
+            for store in stores:
+                store[:, slot].zero_()
 
     def is_live(self, request: Hashable) -> bool:
         return request in self._requests

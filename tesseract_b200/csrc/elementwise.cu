@@ -4,6 +4,7 @@
 //   tb_gather_rows   out[s, :] = in[rows[s], :]               (src/cuda/kernels.rs:774-801)
 //   tb_silu_mul      out[t, j] = silu(gate[t, j]) * up[t, j]  (src/cuda/kernels.rs:191-208); gate and up lie
 //                    either in the two halves of a row or interleaved in blocks of eight columns
+//   tb_clear_slot    a request's slot in every store of recurrent state = 0
 //
 // The activation is computed in 32-bit: g * (1 / (1 + exp(-g))) * u, rounded once.
 #include "common.cuh"
@@ -178,4 +179,59 @@ TB_EXPORT int tb_select_tokens(const int* tokens, const int* feed, const int* pr
     cudaError_t launched = tb_launch_pdl(select_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0, stream, tokens, feed,
                                          previous, out, n, vocab);
     return launched == cudaSuccess ? tb_launch_status() : (int)launched;
+}
+
+// ---- a request's state slot, cleared in every store at once -----------------------------------------------------------
+
+namespace {
+
+constexpr int kMostStores = 16;
+struct Stores {
+    char* base[kMostStores];         // the slot's first byte in the store's first entry
+    int64_t pitch[kMostStores];      // bytes between entries
+    int64_t bytes[kMostStores];      // of a slot
+    int entries[kMostStores];
+};
+
+// Bound by the stores (25 MB a request at the largest sizes tried, 4 us) or by the launch: one for all stores, where a fill for
+// each takes seven launches of 3.6 us and as many calls on the host.
+__global__ void __launch_bounds__(256) clear_slot_kernel(const Stores s) {
+    pdl_trigger();
+    const int store = blockIdx.y;
+    char* base = s.base[store];
+    const int64_t pitch = s.pitch[store], bytes = s.bytes[store];
+    const bool packets = (((uintptr_t)base | (uintptr_t)pitch | (uintptr_t)bytes) & 15) == 0;
+    const int64_t step = packets ? 16 : 1, each = bytes / step, all = each * s.entries[store];
+    pdl_wait();                      // (a step of the slot's last request may still run)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (int64_t)gridDim.x * blockDim.x) {
+        char* at = base + i / each * pitch + i % each * step;
+        if (packets) *reinterpret_cast<uint4*>(at) = make_uint4(0u, 0u, 0u, 0u);
+        else *at = 0;
+    }
+}
+
+}  // namespace
+
+// store i: entries[i] pieces of bytes[i] bytes, pitch[i] bytes apart, from base[i] on, become zero.
+TB_EXPORT int tb_clear_slot(int stores, void* const* base, const int64_t* pitch, const int64_t* bytes, const int* entries,
+                            cudaStream_t stream) {
+    for (int at = 0; at < stores; at += kMostStores) {
+        Stores s = {};
+        const int count = stores - at < kMostStores ? stores - at : kMostStores;
+        int64_t most = 0;
+        for (int i = 0; i < count; ++i) {
+            s.base[i] = (char*)base[at + i];
+            s.pitch[i] = pitch[at + i];
+            s.bytes[i] = bytes[at + i];
+            s.entries[i] = entries[at + i];
+            if (s.bytes[i] < 1 || s.entries[i] < 0) return TB_ERR_BAD_SIZE;
+            const int64_t work = s.bytes[i] * s.entries[i] / 16;
+            most = work > most ? work : most;
+        }
+        const int64_t blocks = (most + 1023) / 1024;          // four packets a thread
+        const cudaError_t launched = tb_launch_pdl(clear_slot_kernel, dim3(blocks < 1 ? 1 : blocks > 1184 ? 1184 : (unsigned)blocks, count),
+                                                   dim3(256), (size_t)0, stream, s);
+        if (launched != cudaSuccess) return (int)launched;
+    }
+    return tb_launch_status();
 }

@@ -88,6 +88,7 @@ def _cuda(*tensors: torch.Tensor) -> None:
 
 SS_STRIDE = 16      # rows per tile / per CTA in the small side arrays that one kernel leaves for the next
 
+_pointer = ctypes.c_void_p
 _i32 = ctypes.c_int
 _i64 = ctypes.c_int64
 _f32 = ctypes.c_float
@@ -132,6 +133,20 @@ def gather_rows(rows_index: torch.Tensor, src: torch.Tensor, out: torch.Tensor) 
     _check(lib.tb_gather_rows(_ptr(rows_index), _ptr(src), _ptr(out), _i32(rows), _i32(width), _i32(src.shape[0]),
                               _i32(_code(out.dtype)), _stream()), "gather_rows")
     return out
+
+
+def clear_slot(stores, slot: int) -> None:
+    """``store[:, slot] = 0`` for every contiguous store ``[entries, slots, ...]``, in one launch."""
+    _cuda(*stores)
+    count = len(stores)
+    base, pitch, size, entries = (_pointer * count)(), (_i64 * count)(), (_i64 * count)(), (_i32 * count)()
+    for i, store in enumerate(stores):
+        _need(store.is_contiguous() and 0 <= slot < store.shape[1], "clear_slot takes contiguous stores and a slot of theirs")
+        size[i] = store.stride(1) * store.element_size()
+        pitch[i] = store.stride(0) * store.element_size()
+        base[i] = store.data_ptr() + slot * size[i]
+        entries[i] = store.shape[0]
+    _check(load_library("elementwise").tb_clear_slot(_i32(count), base, pitch, size, entries, _stream()), "clear_slot")
 
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False) -> torch.Tensor:

@@ -60,6 +60,20 @@ def test_rms_norm_and_fused_add(dtype, rows, width, eps):
         assert torch.equal(res.cpu(), (x.float() + u.float()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("sizes", [[(1, 1)], [(3, 4), (2, 5), (1, 4096)], [(7, 131072), (4, 33)], [(1, 8)] * 17])
+def test_clear_slot_clears_one_slot_of_every_store(sizes):
+    """Stores whose pieces are and are not made of whole packets, of several types, and more stores than one launch takes."""
+    from tesseract_b200 import kernels
+
+    dtypes = (torch.float32, torch.bfloat16, torch.int32)
+    stores = [torch.ones(entries, 4, numbers, dtype=dtypes[i % 3], device="cuda") for i, (entries, numbers) in enumerate(sizes)]
+    kernels.clear_slot(stores, 2)
+    for store in stores:
+        assert (store[:, 2] == 0).all() and (store[:, [0, 1, 3]] == 1).all()
+    with pytest.raises(kernels.KernelError):
+        kernels.clear_slot(stores, 4)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("rows, inter", [(1, 8), (5, 200), (33, 8192), (2, 333)])
 def test_silu_mul(dtype, rows, inter):
