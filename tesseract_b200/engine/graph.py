@@ -294,17 +294,18 @@ class _ChunkGraph:
         wanted += list(range(prompt_rows, total))
         self.wanted = len(wanted)
         # int32 block: tokens[total] positions[total] begin[seqs] slot[seqs], and with a tail seq_of_row[total]
-        # row_start[seqs + 1] want[wanted]; block tables apart (only the columns in use are copied)
-        self.ints = 2 * total + 2 * seqs + ((total + seqs + 1 + len(wanted)) if tail else 0)
+        # row_start[seqs + 1] want[wanted]; then, each on a 256-byte boundary, the block tables: one copy takes all of it
+        # (the columns in use of a table of several rows are no run of bytes, and a copy of those waits for the device)
+        ints = 2 * total + 2 * seqs + ((total + seqs + 1 + len(wanted)) if tail else 0)
+        table_ints = -(-seqs * columns // 64) * 64
+        self.at_tables = [-(-ints // 64) * 64 + k * table_ints for k in range(len(self.paged))]
+        self.ints = self.at_tables[-1] + table_ints if self.paged else ints
         self.hosts = [torch.zeros(self.ints, dtype=torch.int32, pin_memory=True) for _ in range(HOST_RING)]
-        self.host_tables = [[torch.zeros((seqs, columns), dtype=torch.int32, pin_memory=True) for _ in self.paged]
-                            for _ in range(HOST_RING)]
         self.host_events: List[Optional[torch.cuda.Event]] = [None] * HOST_RING
         self.next_host = 0
         self.dev = torch.zeros(self.ints, dtype=torch.int32, device=device)
-        self.dev_tables = [torch.zeros((seqs, columns), dtype=torch.int32, device=device) for _ in self.paged]
         d = self.dev
-        tables = dict(zip(self.paged, self.dev_tables))
+        tables = {group: self.table(d, k) for k, group in enumerate(self.paged)}
         groups = [GroupView(tables.get(index), cache.page_size if g.pool is not None else 0)
                   for index, g in enumerate(cache.groups)]
         seq_of_row_host = torch.cat([torch.arange(portions, dtype=torch.int32).repeat_interleave(rows),
@@ -368,6 +369,11 @@ class _ChunkGraph:
         self.kernels_per_replay = kernels.launch_count - before
         self.graph = graph
         torch.cuda.synchronize()
+
+    def table(self, block, k: int):
+        """The block table ``[seqs, columns]`` of the ``k``-th paged group in a metadata block (a tensor or an array)."""
+        at = self.at_tables[k]
+        return block[at:at + self.seqs * self.columns].reshape(self.seqs, self.columns)
 
 
 class ChunkGraphs:
@@ -458,7 +464,7 @@ class ChunkGraphs:
 
     def step(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
         stepper, cache = self.stepper, self.stepper.cache
-        stepper._validate(entries)
+        tokens = stepper._validate(entries)
         rows, portions = self.rows, self._portions(entries)
         tail = self._tail(entries, portions)
         first_decode = portions + (1 if tail else 0)
@@ -489,10 +495,10 @@ class ChunkGraphs:
         host[2 * total:2 * total + seqs] = 0
         host[2 * total + seqs:2 * total + 2 * seqs] = cache.scratch_slot
         for k in range(portions):
-            host[k * rows:(k + 1) * rows] = np.asarray(entries[k].tokens, dtype=np.int32)
+            host[k * rows:(k + 1) * rows] = tokens[k]
             host[total + k * rows:total + (k + 1) * rows] = np.arange(begins[k], begins[k] + rows, dtype=np.int32)
         if tail:
-            host[full_rows:full_rows + tail] = np.asarray(entries[portions].tokens, dtype=np.int32)
+            host[full_rows:full_rows + tail] = tokens[portions]
             host[total + full_rows:total + full_rows + tail] = np.arange(begins[portions], begins[portions] + tail,
                                                                          dtype=np.int32)
             host[total + full_rows + tail:total + prompt_rows] = np.arange(tail_rows - tail, dtype=np.int32)   # padding
@@ -511,12 +517,11 @@ class ChunkGraphs:
             host[2 * total + seqs + seq] = slots[k]
         used = min(graph.columns, -(-max([b + len(e.tokens) for b, e in zip(begins, entries)] + [tail_rows])
                                     // cache.page_size))
-        graph.dev.copy_(graph.hosts[index], non_blocking=True)
         for k, group_index in enumerate(graph.paged):
-            table = graph.host_tables[index][k].numpy()
+            table = graph.table(host, k)
             table[:, :used] = 0
             table[seq_of_entry, :used] = cache.block_table_rows(group_index, slots, used)
-            graph.dev_tables[k][:, :used].copy_(graph.host_tables[index][k][:, :used], non_blocking=True)
+        graph.dev.copy_(graph.hosts[index], non_blocking=True)
         copied = torch.cuda.Event()
         copied.record()
         graph.host_events[index] = copied

@@ -86,7 +86,9 @@ class Stepper:
         self._sampler = None
 
     # ------------------------------------------------------------------ validation
-    def _validate(self, entries: Sequence[StepEntry]) -> None:
+    def _validate(self, entries: Sequence[StepEntry]) -> List[Sequence[int]]:
+        """Refuse a step that breaks an invariant; return every entry's tokens, a portion's as the array they were checked in."""
+        checked: List[Sequence[int]] = []
         if not entries:
             raise StepError("a step needs at least one entry")
         seen = set()
@@ -99,10 +101,15 @@ class Stepper:
             count = len(entry.tokens)
             if count == 0:
                 raise StepError(f"request {entry.request!r} brings no tokens")
-            ids = np.asarray(entry.tokens)
-            if ids.dtype.kind not in "iu" or ids.ndim != 1:
-                raise StepError(f"the tokens of request {entry.request!r} are not a list of integers")
-            low, high = int(ids.min()), int(ids.max())
+            ids = entry.tokens
+            if count == 1 and type(ids[0]) is int:          # (a decoded row: an array would cost more than the check)
+                low = high = ids[0]
+            else:
+                ids = np.asarray(ids)
+                if ids.dtype.kind not in "iu" or ids.ndim != 1:
+                    raise StepError(f"the tokens of request {entry.request!r} are not a list of integers")
+                low, high = int(ids.min()), int(ids.max())
+            checked.append(ids)
             if low < 0 or high >= self.vocab_size:
                 raise StepError(f"token id {low if low < 0 else high} of request {entry.request!r} is outside the "
                                 f"vocabulary of {self.vocab_size}")
@@ -112,10 +119,13 @@ class Stepper:
                                     f"{count} tokens")
             if self.cache.length(entry.request) + count > self.max_positions:
                 raise StepError(f"request {entry.request!r} would pass the model's {self.max_positions} positions")
+        return checked
 
     # ------------------------------------------------------------------ the step
-    def build_context(self, entries: Sequence[StepEntry]) -> Tuple[StepContext, Optional[torch.Tensor], int]:
-        """Lower the entries into packed device arrays (pages must already exist)."""
+    def build_context(self, entries: Sequence[StepEntry], tokens: Optional[Sequence[Sequence[int]]] = None
+                      ) -> Tuple[StepContext, Optional[torch.Tensor], int]:
+        """Lower the entries into packed device arrays (pages must already exist).  ``tokens``: the entries' tokens as
+        :meth:`_validate` returned them."""
         cache = self.cache
         new = [len(e.tokens) for e in entries]
         begin = [cache.length(e.request) for e in entries]
@@ -124,7 +134,9 @@ class Stepper:
         num_rows = sum(new)
         row_start = np.zeros(num_seqs + 1, dtype=np.int32)
         np.cumsum(new, out=row_start[1:])
-        token_ids = np.fromiter((int(t) for e in entries for t in e.tokens), dtype=np.int32, count=num_rows)
+        token_ids = np.empty(num_rows, dtype=np.int32)
+        for i, ids in enumerate(tokens if tokens is not None else [e.tokens for e in entries]):
+            token_ids[row_start[i]:row_start[i + 1]] = ids
         seq_of_row = np.repeat(np.arange(num_seqs, dtype=np.int32), new)
         begin_arr = np.asarray(begin, dtype=np.int32)
         positions = (np.arange(num_rows, dtype=np.int32) - row_start[:-1][seq_of_row] + begin_arr[seq_of_row]).astype(np.int32)
@@ -152,10 +164,10 @@ class Stepper:
         prompt portion returns a buffer that the next such step overwrites: read it before that.)"""
         if self.chunk_graphs is not None and self.chunk_graphs.eligible(entries):
             return self.chunk_graphs.step(entries)
-        self._validate(entries)
+        tokens = self._validate(entries)
         for entry in entries:
             self.cache.extend(entry.request, len(entry.tokens))
-        ctx, want_rows, _ = self.build_context(entries)
+        ctx, want_rows, _ = self.build_context(entries, tokens)
         # every place of every entry wanted, in order (a decode step): the model need not pick rows out, and takes
         # the same path as a replayed decode step, bit for bit
         every_row = all(list(e.want) == list(range(len(e.tokens))) for e in entries)
