@@ -384,7 +384,7 @@ class ChunkGraphs:
     (token ids, positions, block tables, and where a tail ends), so the launches of the whole model are replayed
     instead of issued one by one; at 2,048 rows of the 1B sizes that takes the step from 4.6 to 3.9 ms, and a step
     of 100 rows, which the host needs 2.8 ms to issue, takes the 1.2 ms of its kernels.  One graph per (portions,
-    tail rows rounded up to 64, 128, ... ``rows``, decode rows rounded up to a power of two, whether any portion
+    tail rows rounded up to 32, 64, 128, ... ``rows``, decode rows rounded up to a power of two, whether any portion
     wants its last place, block-table width rounded up to a power of two): the width bounds the context, and with
     it the split count that the decode rows' attention is captured with, as for the decode graphs.  Rows that pad
     the tail and the decode part point at the scratch page and the scratch state slot.  If one portion wants its
@@ -430,7 +430,7 @@ class ChunkGraphs:
         """Rows that a tail of ``n`` tokens takes in its graph: more than ``n`` (a padding row at least)."""
         if n == 0:
             return 0
-        bucket = 64
+        bucket = 32          # (a prompt of 23 tokens: 1,008 us on 32 rows, 1,067 on 64)
         while bucket <= n and bucket < self.rows:
             bucket <<= 1
         return min(bucket, self.rows)

@@ -396,6 +396,23 @@ def test_replayed_steps_with_the_end_of_a_prompt_equal_ordinary_steps(model_fold
     stepper.cache.check()
 
 
+@pytest.mark.parametrize("length, rows", [(2, 32), (31, 32), (32, 64), (63, 64), (64, 96), (95, 96)])
+def test_a_short_prompt_takes_the_fewest_rows_that_hold_it(model_folders, length, rows):
+    from tesseract_b200.engine import StepEntry, load_model, make_stepper
+
+    model = load_model(model_folders("c"), dtype="float32")
+    prompt = random_tokens(TINY["c"]["vocab_size"], length, seed=length)
+    got = []
+    for graphs in (False, True):
+        stepper = make_stepper(model, capacity_tokens=256, max_requests=2)
+        if graphs:
+            stepper.enable_graphs(2, chunk_rows=96, max_sequence_length=128)
+        assert stepper.cache.admit("a")
+        got.append([stepper.step([StepEntry("a", prompt, [length - 1])]).clone(), stepper.step([StepEntry("a", [3], [0])]).clone()])
+    assert [key[1] for key in stepper.chunk_graphs.graphs] == [rows]
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 # ----------------------------------------------------------------------------- the layer sizes of Llama 3.2 1B
 
 SIZES_1B = {
