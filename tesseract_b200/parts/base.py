@@ -507,7 +507,11 @@ class Injection(Part):
 
 class TokenInput(Part):
     """What a layer adds to the stream for the token itself, behind its sublayers: ``forward(residual, ctx)`` adds to
-    the 32-bit ``residual`` in place (the step's token ids are ``ctx.token_ids``)."""
+    the 32-bit ``residual`` in place (the step's token ids are ``ctx.token_ids``).  One that ``accepts_following_norm`` has an
+    ``eps`` and takes ``following``, the norm that reads the stream next, into its last addition: it then returns that
+    norm's rows."""
+
+    accepts_following_norm = False
 
     def forward(self, residual: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         raise NotImplementedError

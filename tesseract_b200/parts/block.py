@@ -30,8 +30,8 @@ sum and both norms are one kernel.  A layer without a feed-forward leaves (x, a)
     x <- x + token_input(x, tokens)                                     (absent without a token input)
 
 The norm of a sublayer's result, the addition and the norm in front of the next sublayer are one kernel
-(``norm_add_norm``); it also leaves the rounded stream that the token input's first product reads.  Where a layer has no
-token input, the kernel behind its last sublayer also takes the norm that consumes the stream next (the next block's
+(``norm_add_norm``); it also leaves the rounded stream that the token input's first product reads.  The kernel behind a
+layer's last sublayer, or behind its token input, also takes the norm that consumes the stream next (the next block's
 first norm, or the final norm).
 
 ``gated_pre_norm`` is the pre-norm arrangement over a 32-bit stream in which every sublayer's result is weighted, feature
@@ -199,17 +199,19 @@ class SandwichBlock(Block):
             update, post = self.feed_forward.forward(x, ctx), self.norms["post_feed_forward"]
         else:
             update, post = mixed, self.norms["post_mixer"]
-        following = None
-        if self.token_input is None and hasattr(next_norm, "norm_parameters") and next_norm.eps == self.eps:
-            following = next_norm
-        if following is not None:
+        following = next_norm if hasattr(next_norm, "norm_parameters") and next_norm.eps == self.eps else None
+        if self.token_input is None and following is not None:
             rows = rows_like()
             kernels.norm_add_norm(residual, update, post.norm_parameters(), following.norm_parameters(), rows, None, self.eps)
             return ResidualStream(residual, None, prepared=FinishedNorm(following, residual, rows))
         copy = rows_like() if wants_copy else None
         kernels.norm_add_norm(residual, update, post.norm_parameters(), None, None, copy, self.eps)
         if self.token_input is not None:
-            self.token_input.forward(residual, ctx, rounded=copy if wants_copy else residual)
+            rounded = copy if wants_copy else residual
+            if following is not None and getattr(self.token_input, "accepts_following_norm", False) and self.token_input.eps == self.eps:
+                rows = self.token_input.forward(residual, ctx, rounded=rounded, following=following)
+                return ResidualStream(residual, None, prepared=FinishedNorm(following, residual, rows))
+            self.token_input.forward(residual, ctx, rounded=rounded)
         return ResidualStream(residual, None)
 
 

@@ -34,6 +34,7 @@ class GatedTokenSlice(TokenInput):
     ``[hidden]``."""
 
     graph_safe = True
+    accepts_following_norm = True
 
     def __init__(self, spec: PartSpec, tensors: Mapping[str, torch.Tensor], runtime: Runtime):
         super().__init__(spec, tensors, runtime)
@@ -72,9 +73,11 @@ class GatedTokenSlice(TokenInput):
     def products(self):
         return [("token gate", self.gate_proj, plan.F32), ("token proj", self.out_proj, plan.F32)]
 
-    def forward(self, residual: torch.Tensor, ctx: StepContext, rounded: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def forward(self, residual: torch.Tensor, ctx: StepContext, rounded: Optional[torch.Tensor] = None,
+                following=None) -> torch.Tensor:
         """``residual`` (float32, in place) gains the layer's term; ``rounded``: the stream already rounded to the run
-        dtype, if the caller has it."""
+        dtype, if the caller has it.  ``following``: a norm with ``norm_parameters()`` and this part's eps that reads the
+        stream next; the last addition's kernel then takes it too, and its rows are returned instead of the stream."""
         rows = residual.shape[0]
         if rounded is None:
             rounded = residual if self.runtime.is_float32 else residual.to(self.runtime.dtype)
@@ -82,5 +85,9 @@ class GatedTokenSlice(TokenInput):
         g = torch.empty((rows, self.dim), dtype=self.runtime.dtype, device=residual.device)
         kernels.token_gate(z, ctx.token_ids, self.table, self.slice * self.dim, g, self.activation)
         y = self.out_proj.forward(g, float32_out=True)
-        kernels.norm_add_norm(residual, y, (kernels.NORM_RMS, self.norm_weight, None), None, None, None, self.eps)
-        return residual
+        if following is None:
+            kernels.norm_add_norm(residual, y, (kernels.NORM_RMS, self.norm_weight, None), None, None, None, self.eps)
+            return residual
+        out = torch.empty(residual.shape, dtype=self.runtime.dtype, device=residual.device)
+        kernels.norm_add_norm(residual, y, (kernels.NORM_RMS, self.norm_weight, None), following.norm_parameters(), out, None, self.eps)
+        return out
