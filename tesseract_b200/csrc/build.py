@@ -33,7 +33,9 @@ INCLUDES: Dict[str, List[str]] = {
     "attention_noalloc": ["attention_mma.cu", "attention_noalloc.h"],
     "attention_tcgen05": ["tma.cuh"],
     "gemm_tcgen05": ["tma.cuh", "umma.cuh"],
-    "skinny_tcgen05": ["tma.cuh", "umma.cuh"],
+    "skinny_tcgen05": ["activation.cuh", "tma.cuh", "umma.cuh"],
+    "decode_linear": ["activation.cuh"],
+    "pointwise": ["activation.cuh"],
 }
 
 # Every source file, with the extra flags it needs.

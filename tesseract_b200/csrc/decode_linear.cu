@@ -7,7 +7,10 @@
 //   (src/cuda/kernels.rs:59-103), or the plain RMSNorm of res (src/cuda/kernels.rs:26-57),
 // and, fused behind, either a plain store (bfloat16 or 32-bit) or the SwiGLU activation
 //   out[m, j] = round(silu(gate_j) * up_j)   (src/cuda/kernels.rs:191-208), for a weight whose rows
-// interleave gate and up in blocks of eight: rows 16b..16b+7 = gate 8b..8b+7, rows 16b+8..16b+15 = up 8b..8b+7.
+// interleave gate and up in blocks of eight: rows 16b..16b+7 = gate 8b..8b+7, rows 16b+8..16b+15 = up 8b..8b+7,
+// or over such a weight the activation that a kernel behind the product would apply to its stored rows
+//   out[m, j] = round(act(round(gate_j)) * round(up_j)),  act SiLU or GELU in its tanh form, to the bit.
+// (That kernel's launch is 2.7 us of a decode step for each feed-forward, the activation here is hidden by other CTAs' streams.)
 //
 // Two more forms move a norm's work out of the product behind it and into the product in front of it:
 //   EPI_ADD_NORM (a product without a norm in front, bfloat16 out): with o = round(y), c = res + o (32-bit),
@@ -28,7 +31,7 @@
 // Each lane loads 16 contiguous bytes per weight row and 32-wide K block; the products pair weight
 // and activation elements in the same permuted K order, so no shuffle or shared-memory transpose is
 // needed.  The reduction order depends on K alone.
-#include "common.cuh"
+#include "activation.cuh"
 
 namespace {
 
@@ -38,7 +41,7 @@ constexpr int kThreads = kWarps * 32;
 // to cover the memory latency alone: five stages of 32-feature tiles or six of 16-feature tiles per warp.
 
 enum Prologue : int { PRO_NONE = 0, PRO_NORM = 1, PRO_ADD_NORM = 2, PRO_SCALED = 3, PRO_SCALED_RESIDENT = 4 };
-enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3 };
+enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3, EPI_GATED_SILU = 4, EPI_GATED_GELU = 5 };
 constexpr int kSsStride = 16;      // floats per tile in the sums-of-squares array (rows beyond M hold zeros)
 
 struct LinearParams {
@@ -414,7 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_linear_kernel(const Linear
             scale_s[threadIdx.x] = 1.0f / sqrtf(total / (float)K + p.eps);
         }
         if (kScaled && ti == 0) __syncthreads();
-        if (EPI == EPI_SWIGLU) {
+        if (EPI == EPI_SWIGLU || EPI == EPI_GATED_SILU || EPI == EPI_GATED_GELU) {
             // of every 16 features the first eight are gates, the last eight the matching up projections
             for (int idx = threadIdx.x; idx < 8 * NH * ROWS; idx += kThreads) {
                 const int f = idx / ROWS, m = idx - f * ROWS;   // f: activation column within the tile
@@ -430,7 +433,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_linear_kernel(const Linear
                     gate *= scale_s[m];
                     up *= scale_s[m];
                 }
-                const float act = gate * (1.0f / (1.0f + expf(-gate))) * up;
+                const float act = EPI == EPI_SWIGLU     ? gate * (1.0f / (1.0f + expf(-gate))) * up
+                                  : EPI == EPI_GATED_SILU ? tbact::gated_rounded<tbact::ACT_SILU>(gate, up)
+                                                          : tbact::gated_rounded<tbact::ACT_GELU_TANH>(gate, up);
                 reinterpret_cast<__nv_bfloat16*>(p.out)[(int64_t)m * p.out_stride + tile * 8 * NH + f] =
                     __float2bfloat16_rn(act);
             }
@@ -608,6 +613,8 @@ int dispatch(const LinearParams& p, int prologue, int epilogue, cudaStream_t str
     TB_CASE(PRO_NONE, EPI_BF16)
     TB_CASE(PRO_NONE, EPI_F32)
     TB_CASE(PRO_NONE, EPI_SWIGLU)
+    TB_CASE(PRO_NONE, EPI_GATED_SILU)
+    TB_CASE(PRO_NONE, EPI_GATED_GELU)
     TB_CASE(PRO_NORM, EPI_BF16)
     TB_CASE(PRO_NORM, EPI_F32)
     TB_CASE(PRO_NORM, EPI_SWIGLU)

@@ -2,7 +2,8 @@
 // and of scaled logits.  All arithmetic is 32-bit; each stored value is rounded once.
 //
 //   tb_gated_activation   out[t, j] = act(gate[t, j] + bg[j]) * (up[t, j] + bu[j]); gate and up are the two halves
-//                         of a row of `gu`; the biases (32-bit, [2 * inter], gate then up) may be null.
+//                         of a row of `gu`, or alternate in blocks of eight columns (then there are no biases); the
+//                         biases (32-bit, [2 * inter], gate then up) may be null.
 //                         act: 0 = SiLU, 1 = GELU in its tanh form
 //                         0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))); 2 = both halves clamped: with
 //                         g = min(gate, limit) and u = min(max(up, -limit), limit), g * sigmoid(slope * g) * (u + 1).
@@ -15,18 +16,11 @@
 //   tb_embedding_scaled   out[t, :] = float(table[token[t], :]) * s   (32-bit out; the table 32-bit or bfloat16)
 //   tb_token_gate         out[t, j] = act(z[t, j]) * table[token[t], offset + j]     (32-bit z; a slice of a second
 //                         embedding table gated by a projection of the stream)
-#include "common.cuh"
+#include "activation.cuh"
 
 namespace {
 
-enum Activation : int { ACT_SILU = 0, ACT_GELU_TANH = 1, ACT_CLAMPED = 2 };
-
-template <int ACT>
-__device__ __forceinline__ float activate(float z) {
-    if (ACT == ACT_SILU) return z * (1.0f / (1.0f + expf(-z)));
-    const float inner = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    return 0.5f * z * (1.0f + tanhf(inner));
-}
+using namespace tbact;
 
 template <int ACT>
 __device__ __forceinline__ float gated(float g, float u, float limit, float slope) {
@@ -38,13 +32,15 @@ __device__ __forceinline__ float gated(float g, float u, float limit, float slop
 
 template <typename T, int ACT>
 __global__ void gated_activation_kernel(const T* __restrict__ gu, int64_t gu_stride, const float* __restrict__ bias,
-                                        T* __restrict__ out, int64_t out_stride, int inter, float limit, float slope) {
+                                        T* __restrict__ out, int64_t out_stride, int inter, int interleaved, float limit,
+                                        float slope) {
     pdl_trigger();
     pdl_wait();
     const T* g = gu + (int64_t)blockIdx.x * gu_stride;
     T* o = out + (int64_t)blockIdx.x * out_stride;
     for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < inter; j += gridDim.y * blockDim.x) {
-        float gv = Elem<T>::load(g + j), uv = Elem<T>::load(g + inter + j);
+        const int at = interleaved ? (j >> 3) * 16 + (j & 7) : j;
+        float gv = Elem<T>::load(g + at), uv = Elem<T>::load(g + at + (interleaved ? 8 : inter));
         if (bias != nullptr) {
             gv += bias[j];
             uv += bias[inter + j];
@@ -57,16 +53,18 @@ __global__ void gated_activation_kernel(const T* __restrict__ gu, int64_t gu_str
 template <typename T, int ACT>
 __global__ void gated_activation_packets_kernel(const T* __restrict__ gu, int64_t gu_stride,
                                                 const float* __restrict__ bias, T* __restrict__ out,
-                                                int64_t out_stride, int inter, float limit, float slope) {
+                                                int64_t out_stride, int inter, int interleaved, float limit, float slope) {
     constexpr int N = Packet<T>::N;
+    static_assert(8 % N == 0, "a packet lies within a block of eight columns");
     pdl_trigger();
     pdl_wait();
     const T* g = gu + (int64_t)blockIdx.x * gu_stride;
     T* o = out + (int64_t)blockIdx.x * out_stride;
     for (int j = (blockIdx.y * blockDim.x + threadIdx.x) * N; j < inter; j += gridDim.y * blockDim.x * N) {
         float gv[N], uv[N], ov[N];
-        Packet<T>::load(g + j, gv);
-        Packet<T>::load(g + inter + j, uv);
+        const int at = interleaved ? (j >> 3) * 16 + (j & 7) : j;
+        Packet<T>::load(g + at, gv);
+        Packet<T>::load(g + at + (interleaved ? 8 : inter), uv);
 #pragma unroll
         for (int e = 0; e < N; ++e) {
             if (bias != nullptr) {
@@ -194,7 +192,7 @@ inline int grid_for(int64_t total, int threads) {
 
 template <typename T, int ACT>
 int launch_gated(const void* gu, int64_t gu_stride, const float* bias, void* out, int64_t out_stride, int rows, int inter,
-                 float limit, float slope, cudaStream_t stream) {
+                 int interleaved, float limit, float slope, cudaStream_t stream) {
     constexpr int N = Packet<T>::N;
     const int threads = 256;
     const bool packets = inter % N == 0 && gu_stride % N == 0 && out_stride % N == 0 &&
@@ -202,26 +200,29 @@ int launch_gated(const void* gu, int64_t gu_stride, const float* bias, void* out
     cudaError_t launched;
     if (packets)
         launched = tb_launch_pdl(gated_activation_packets_kernel<T, ACT>, row_grid(rows, inter, threads, N), dim3(threads),
-                                 0, stream, (const T*)gu, gu_stride, bias, (T*)out, out_stride, inter, limit, slope);
+                                 0, stream, (const T*)gu, gu_stride, bias, (T*)out, out_stride, inter, interleaved, limit,
+                                 slope);
     else
         launched = tb_launch_pdl(gated_activation_kernel<T, ACT>, row_grid(rows, inter, threads), dim3(threads), 0,
-                                 stream, (const T*)gu, gu_stride, bias, (T*)out, out_stride, inter, limit, slope);
+                                 stream, (const T*)gu, gu_stride, bias, (T*)out, out_stride, inter, interleaved, limit, slope);
     return launched == cudaSuccess ? tb_launch_status() : (int)launched;
 }
 
 }  // namespace
 
-// limit, slope: only activation 2 reads them.
+// interleaved: gate and up alternate in blocks of eight columns (inter a multiple of eight, no bias).  limit, slope: only
+// activation 2 reads them.
 TB_EXPORT int tb_gated_activation(const void* gu, int64_t gu_stride, const float* bias, void* out, int64_t out_stride,
-                                  int rows, int inter, int activation, float limit, float slope, int dtype,
+                                  int rows, int inter, int interleaved, int activation, float limit, float slope, int dtype,
                                   cudaStream_t stream) {
     if (rows == 0 || inter == 0) return 0;
+    if (interleaved && (inter % 8 != 0 || bias != nullptr)) return TB_ERR_BAD_SIZE;
     if (activation < ACT_SILU || activation > ACT_CLAMPED) return TB_ERR_BAD_SIZE;
     if (dtype != TB_F32 && dtype != TB_BF16) return TB_ERR_BAD_DTYPE;
 #define TB_RUN(ACT)                                                                                                   \
     return dtype == TB_F32                                                                                            \
-               ? launch_gated<float, ACT>(gu, gu_stride, bias, out, out_stride, rows, inter, limit, slope, stream)    \
-               : launch_gated<__nv_bfloat16, ACT>(gu, gu_stride, bias, out, out_stride, rows, inter, limit, slope, stream)
+               ? launch_gated<float, ACT>(gu, gu_stride, bias, out, out_stride, rows, inter, interleaved, limit, slope, stream)    \
+               : launch_gated<__nv_bfloat16, ACT>(gu, gu_stride, bias, out, out_stride, rows, inter, interleaved, limit, slope, stream)
     if (activation == ACT_SILU) TB_RUN(ACT_SILU);
     if (activation == ACT_GELU_TANH) TB_RUN(ACT_GELU_TANH);
     TB_RUN(ACT_CLAMPED);

@@ -35,6 +35,7 @@
 // applied to the 32-bit sums.
 // Every wait on an mbarrier is bounded: a wait that runs out sets *error and tells the other roles to stop; the
 // CTA still meets its cluster barriers and frees its tensor memory.
+#include "activation.cuh"
 #include "umma.cuh"
 
 #include <atomic>
@@ -55,7 +56,9 @@ constexpr int kSumsStride = 128;        // floats per tile in the sums-of-square
 constexpr uint32_t kWBlockBytes = BF * BK * 2;     // 16 KiB
 constexpr size_t kSmemBudget = 208 * 1024;
 
-enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3 };
+enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3, EPI_GATED_SILU = 4, EPI_GATED_GELU = 5 };
+
+__host__ __device__ constexpr bool gate_and_up(int epilogue) { return epilogue == EPI_SWIGLU || epilogue == EPI_GATED_SILU || epilogue == EPI_GATED_GELU; }
 
 struct SkinnyParams {
     void* out;
@@ -127,14 +130,18 @@ __device__ __forceinline__ float epilogue_row(const SkinnyParams& p, float4 v, i
             for (int i = 0; i < 4; ++i)
                 if (n + i < p.N) dst[i] = __float2bfloat16_rn(e[i]);
         }
-    } else if (EPI == EPI_SWIGLU) {
+    } else if (gate_and_up(EPI)) {
         // of every sixteen features (four lanes) the first eight are gates, the last eight the matching up
         // projections: a gate lane takes its four up values from the lane two further on (N is a multiple of 16,
         // so a group of sixteen is whole or absent)
         const float ux = __shfl_down_sync(0xffffffffu, v.x, 2), uy = __shfl_down_sync(0xffffffffu, v.y, 2);
         const float uz = __shfl_down_sync(0xffffffffu, v.z, 2), uw = __shfl_down_sync(0xffffffffu, v.w, 2);
         if ((lane & 2) == 0 && n < p.N) {
-            auto act = [](float gate, float up) { return gate * __fdividef(1.0f, 1.0f + __expf(-gate)) * up; };
+            auto act = [](float gate, float up) {
+                if (EPI == EPI_GATED_SILU) return tbact::gated_rounded<tbact::ACT_SILU>(gate, up);
+                if (EPI == EPI_GATED_GELU) return tbact::gated_rounded<tbact::ACT_GELU_TANH>(gate, up);
+                return gate * __fdividef(1.0f, 1.0f + __expf(-gate)) * up;
+            };
             // gate feature n + i of the tile's group (n >> 4) is activation column (n >> 4) * 8 + (n & 7) + i
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)m * p.out_stride + (n >> 4) * 8 + (n & 7);
             const float a0 = act(v.x, ux), a1 = act(v.y, uy), a2 = act(v.z, uz), a3 = act(v.w, uw);
@@ -550,11 +557,11 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const SkinnyParam
 }  // namespace
 
 // 1 if the kernel takes these sizes.  K and the row strides must be multiples of 8 (16-byte TMA strides); the
-// SwiGLU epilogue needs N to be a multiple of 16.
+// epilogues over gate and up need N to be a multiple of 16.
 TB_EXPORT int tb_skinny_tcgen05_supported(int M, int N, int K, int epilogue) {
     if (M < 1 || M > BF || N < 1 || K < 8 || K % 8 != 0) return 0;
-    if (epilogue == EPI_SWIGLU && N % 16 != 0) return 0;
-    if (epilogue < EPI_BF16 || epilogue > EPI_ADD_NORM) return 0;
+    if (gate_and_up(epilogue) && N % 16 != 0) return 0;
+    if (epilogue < EPI_BF16 || epilogue > EPI_GATED_GELU) return 0;
     return shape_for(M, N, K).stages >= 1;
 }
 
@@ -563,7 +570,7 @@ TB_EXPORT int tb_skinny_tcgen05_supported(int M, int N, int K, int epilogue) {
 TB_EXPORT int tb_skinny_tcgen05_sums_stride() { return kSumsStride; }
 TB_EXPORT int tb_skinny_tcgen05_sums_tiles(int N) { return (N + BF - 1) / BF; }
 
-// x [M, K] (row stride x_stride), w [N, K] (row stride w_stride), out [M, N] ([M, N / 2] for SwiGLU; out_stride in
+// x [M, K] (row stride x_stride), w [N, K] (row stride w_stride), out [M, N] ([M, N / 2] over gate and up; out_stride in
 // elements of the output type; not written by EPI_ADD_NORM).
 // ss_in (or null): sums of squares [ss_tiles][128] that an EPI_ADD_NORM product left; the product is then scaled
 //   per row by rsqrt(sum / K + eps).
@@ -623,6 +630,10 @@ TB_EXPORT int tb_skinny_tcgen05(const void* x, int64_t x_stride, const void* w, 
             return scaled ? launch<EPI_F32, true>(map_w, map_x, p, s, stream) : launch<EPI_F32, false>(map_w, map_x, p, s, stream);
         case EPI_ADD_NORM:
             return launch<EPI_ADD_NORM, false>(map_w, map_x, p, s, stream);
+        case EPI_GATED_SILU:
+            return scaled ? TB_ERR_BAD_SIZE : launch<EPI_GATED_SILU, false>(map_w, map_x, p, s, stream);
+        case EPI_GATED_GELU:
+            return scaled ? TB_ERR_BAD_SIZE : launch<EPI_GATED_GELU, false>(map_w, map_x, p, s, stream);
     }
     return TB_ERR_BAD_SIZE;
 }

@@ -453,6 +453,8 @@ def decode_linear_supported(rows: int, out_features: int, in_features: int, prol
 
 
 EPI_ADD_NORM = 3
+EPI_GATED_SILU, EPI_GATED_GELU = 4, 5
+_OVER_GATE_AND_UP = (EPI_SWIGLU, EPI_GATED_SILU, EPI_GATED_GELU)
 PRO_SCALED = 3
 
 
@@ -530,7 +532,7 @@ def decode_linear(weight: torch.Tensor, out: Optional[torch.Tensor], *, x: Optio
               f"decode_linear prepare sums must be float32 [{tiles}, {SS_STRIDE}]")
         epi = (p_res, p_norm, p_res_out, p_rows, p_sums)
     else:
-        width = n // 2 if epilogue == EPI_SWIGLU else n
+        width = n // 2 if epilogue in _OVER_GATE_AND_UP else n
         _need(out is not None and out.shape == (m, width) and out.stride(1) == 1, "decode_linear out shape")
         _need(out.dtype == (torch.float32 if epilogue == EPI_F32 else torch.bfloat16), "decode_linear out dtype")
     best_values = best_indices = None
@@ -660,7 +662,7 @@ def skinny_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Te
         epi = [_ptr(residual), _ptr(norm_weight), _ptr(new_residual), _ptr(scaled_rows), _ptr(sums)]
         epilogue = EPI_ADD_NORM
     else:
-        width = n // 2 if epilogue == EPI_SWIGLU else n
+        width = n // 2 if epilogue in _OVER_GATE_AND_UP else n
         _cuda(out)
         _need(out.shape == (m, width) and out.stride(1) == 1, "skinny_tcgen05 out shape")
         _need(out.dtype == (torch.float32 if epilogue == EPI_F32 else torch.bfloat16), "skinny_tcgen05 out dtype")
@@ -1141,9 +1143,9 @@ ACT_SILU, ACT_GELU_TANH, ACT_CLAMPED = 0, 1, 2
 
 
 def gated_activation(gate_up: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, activation: int,
-                     limit: float = 0.0, slope: float = 0.0) -> torch.Tensor:
-    """``out = act(gate + bias[:I]) * (up + bias[I:])``; gate and up are the two halves of ``gate_up``'s rows, ``bias``
-    (float32 ``[2 I]``) may be None; ``activation``: ``ACT_SILU`` or ``ACT_GELU_TANH``, or ``ACT_CLAMPED``, which clamps
+                     limit: float = 0.0, slope: float = 0.0, interleaved: bool = False) -> torch.Tensor:
+    """``out = act(gate + bias[:I]) * (up + bias[I:])``; gate and up are the two halves of ``gate_up``'s rows, or
+    (``interleaved``, without bias) alternate in blocks of eight columns; ``bias`` (float32 ``[2 I]``) may be None; ``activation``: ``ACT_SILU`` or ``ACT_GELU_TANH``, or ``ACT_CLAMPED``, which clamps
     both halves: ``g * sigmoid(slope * g) * (u + 1)`` with ``g = min(gate, limit)``, ``u = min(max(up, -limit), limit)``."""
     _cuda(gate_up, bias, out)
     rows, inter = out.shape
@@ -1151,9 +1153,10 @@ def gated_activation(gate_up: torch.Tensor, bias: Optional[torch.Tensor], out: t
           and out.dtype == gate_up.dtype, "gated_activation gate_up/out")
     _need(bias is None or (bias.dtype == torch.float32 and bias.numel() == 2 * inter and bias.is_contiguous()),
           "gated_activation bias")
+    _need(not interleaved or (bias is None and inter % 8 == 0), "gated_activation interleaved: whole blocks of eight, no bias")
     lib = load_library("pointwise")
     _check(lib.tb_gated_activation(_ptr(gate_up), _i64(gate_up.stride(0)), _ptr(bias), _ptr(out), _i64(out.stride(0)),
-                                   _i32(rows), _i32(inter), _i32(activation), _f32(limit), _f32(slope),
+                                   _i32(rows), _i32(inter), _i32(1 if interleaved else 0), _i32(activation), _f32(limit), _f32(slope),
                                    _i32(_code(out.dtype)), _stream()), "gated_activation")
     return out
 

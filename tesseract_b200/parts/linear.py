@@ -60,7 +60,7 @@ class Linear:
                             norm=norm, contiguous_rows=contiguous_rows, follow=follow)
 
     def _out(self, rows: int, choice: plan.ProductPlan, device) -> torch.Tensor:
-        width = self.out_features // 2 if choice.epilogue == plan.SWIGLU else self.out_features
+        width = self.out_features // 2 if choice.epilogue in plan.OVER_GATE_AND_UP else self.out_features
         dtype = torch.float32 if choice.epilogue == plan.F32 else self.runtime.dtype
         return torch.empty((rows, width), dtype=dtype, device=device)
 
@@ -75,7 +75,7 @@ class Linear:
 
     def product(self, x: torch.Tensor, out: Optional[torch.Tensor] = None, float32_out: bool = False,
                 epilogue: Optional[str] = None, follow=None, best=None):
-        """``x @ W^T``; with ``epilogue="swiglu"`` the activated product ``[rows, out / 2]`` if the plan has a kernel
+        """``x @ W^T``; with an ``epilogue`` over gate and up the activated product ``[rows, out / 2]`` if the plan has a kernel
         that folds the activation in, else ``None`` (the caller then activates the plain product itself).  With
         ``follow`` (a :class:`FollowNorm`) the product may do the work of the norm behind it and return a
         :class:`PreparedNorm` instead of its rows, if the plan has a kernel for that."""
@@ -86,7 +86,7 @@ class Linear:
         rows = x.shape[0]
         wanted = epilogue or (plan.F32 if float32_out or self.runtime.is_float32 else plan.BF16)
         choice = self.plan(rows, wanted, contiguous_rows=x.stride(1) == 1)
-        if wanted == plan.SWIGLU and choice.activation_apart:
+        if choice.activation_apart:
             return None
         if follow is not None and out is None and wanted == plan.BF16:
             prepared = self._prepare(x, follow)

@@ -21,6 +21,12 @@ from .base import FEED_FORWARDS, DeferredNorm, FeedForward, Runtime, StepContext
 from .linear import Linear
 
 
+def _interleaved(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """Eight gate rows, the eight matching up rows, and so on."""
+    size, width = gate.shape
+    return torch.stack([gate.reshape(size // 8, 8, width), up.reshape(size // 8, 8, width)], dim=1).reshape(2 * size, width)
+
+
 @FEED_FORWARDS.register("swiglu")
 class SwiGLU(FeedForward):
     """params: ``hidden_size, intermediate_size``; weights: ``gate, up, down``."""
@@ -34,10 +40,7 @@ class SwiGLU(FeedForward):
         self.intermediate_size = int(p["intermediate_size"])
         self.interleaved = self.intermediate_size % 8 == 0
         if self.interleaved:
-            blocks = self.intermediate_size // 8
-            merged = torch.stack([tensors["gate"].view(blocks, 8, self.hidden_size),
-                                  tensors["up"].view(blocks, 8, self.hidden_size)], dim=1)
-            merged = merged.reshape(2 * self.intermediate_size, self.hidden_size)
+            merged = _interleaved(tensors["gate"], tensors["up"])
         else:
             merged = torch.cat([tensors["gate"], tensors["up"]], dim=0)
         self.gate_up_proj = Linear(merged, runtime)
@@ -164,7 +167,7 @@ class PlainMLP(FeedForward):
         return self.down_proj.forward(z, float32_out=self.stream_f32)
 
 
-_ACTIVATIONS = {"silu": kernels.ACT_SILU, "gelu_tanh": kernels.ACT_GELU_TANH}
+_ACTIVATIONS = {"silu": (kernels.ACT_SILU, plan.GATED_SILU), "gelu_tanh": (kernels.ACT_GELU_TANH, plan.GATED_GELU)}
 
 
 @FEED_FORWARDS.register("gated_mlp")
@@ -174,7 +177,9 @@ class GatedMLP(FeedForward):
     params: ``hidden_size, intermediate_size``, ``activation`` (``"silu"`` or ``"gelu_tanh"``: ``0.5 z (1 + tanh(sqrt(2/pi)
     (z + 0.044715 z^3)))``), ``bias`` (bool), optional ``stream``; weights: ``gate, up, down`` and, with ``bias``,
     ``gate_bias, up_bias, down_bias``.  Gate and up are one product; biases, activation and the gating are one kernel
-    in 32-bit behind it; the down product comes out in 32-bit for a residual stream kept in 32-bit."""
+    in 32-bit behind it; the down product comes out in 32-bit for a residual stream kept in 32-bit.  Without biases, and with
+    an intermediate size that is a multiple of eight, the merged rows alternate in blocks of eight, and the products of up
+    to 128 rows activate their own sums, rounded first, to the same bits."""
 
     graph_safe = True
 
@@ -185,10 +190,12 @@ class GatedMLP(FeedForward):
         self.intermediate_size = int(p["intermediate_size"])
         if p.get("activation") not in _ACTIVATIONS:
             raise ValueError(f"activation must be one of {sorted(_ACTIVATIONS)}, got {p.get('activation')!r}")
-        self.activation = _ACTIVATIONS[p["activation"]]
+        self.activation, self.epilogue = _ACTIVATIONS[p["activation"]]
         self.biased = bool(p.get("bias"))
         self.stream_f32 = p.get("stream") == "float32"
-        self.gate_up_proj = Linear(torch.cat([tensors["gate"], tensors["up"]], dim=0), runtime)
+        self.interleaved = not self.biased and self.intermediate_size % 8 == 0
+        merged = _interleaved(tensors["gate"], tensors["up"]) if self.interleaved else torch.cat([tensors["gate"], tensors["up"]], dim=0)
+        self.gate_up_proj = Linear(merged, runtime)
         self.gate_up_bias = None
         if self.biased:
             self.gate_up_bias = torch.cat([tensors["gate_bias"], tensors["up_bias"]]).to(
@@ -214,13 +221,15 @@ class GatedMLP(FeedForward):
 
     def products(self):
         """``(name, Linear, epilogue)`` of the feed-forward's matrix products, for the printed kernel plan."""
-        return [("gate/up", self.gate_up_proj, plan.BF16),
+        return [("gate/up", self.gate_up_proj, self.epilogue if self.interleaved else plan.BF16),
                 ("down", self.down_proj, plan.F32 if self.stream_f32 else plan.BF16)]
 
     def forward(self, x, ctx: StepContext, follow=None):
         if isinstance(x, DeferredNorm):
             x = x.materialize()
-        gate_up = self.gate_up_proj.forward(x)
-        activated = torch.empty((x.shape[0], self.intermediate_size), dtype=gate_up.dtype, device=gate_up.device)
-        kernels.gated_activation(gate_up, self.gate_up_bias, activated, self.activation)
+        activated = self.gate_up_proj.forward(x, epilogue=self.epilogue) if self.interleaved else None
+        if activated is None:
+            gate_up = self.gate_up_proj.forward(x)
+            activated = torch.empty((x.shape[0], self.intermediate_size), dtype=gate_up.dtype, device=gate_up.device)
+            kernels.gated_activation(gate_up, self.gate_up_bias, activated, self.activation, interleaved=self.interleaved)
         return self.down_proj.forward(activated, float32_out=self.stream_f32)

@@ -39,7 +39,10 @@ MAX_ATTENTION_SPLITS = kernels.MAX_ATTENTION_SPLITS
 CLUSTER_SPLITS = 8            # up to this many splits merge inside a thread-block cluster; more go through scratch
 
 BF16, F32, SWIGLU = "bf16", "f32", "swiglu"
-_EPILOGUE_CODE = {BF16: kernels.EPI_BF16, F32: kernels.EPI_F32, SWIGLU: kernels.EPI_SWIGLU}
+GATED_SILU, GATED_GELU = "gated_silu", "gated_gelu"       # the rounded product's gate and up, activated: what a kernel behind it gives
+OVER_GATE_AND_UP = (SWIGLU, GATED_SILU, GATED_GELU)
+_EPILOGUE_CODE = {BF16: kernels.EPI_BF16, F32: kernels.EPI_F32, SWIGLU: kernels.EPI_SWIGLU, GATED_SILU: kernels.EPI_GATED_SILU,
+                  GATED_GELU: kernels.EPI_GATED_GELU}
 
 
 @lru_cache(maxsize=None)
@@ -68,7 +71,7 @@ class ProductPlan:
     ``skinny_tcgen05`` (weight streaming on the tensor-memory cores, at most 128 rows), ``gemm_tcgen05`` (this
     package's tensor-memory GEMM: CTA pairs on 256-row tiles above 128 rows) or ``library``.
     ``norm_folded``: the RMSNorm (and the residual addition) in front runs inside the product's kernel.  ``epilogue``: what the kernel stores;
-    ``activation_apart``: SwiGLU was asked for but runs as a kernel of its own behind the product.
+    ``activation_apart``: an activation was asked for but runs as a kernel of its own behind the product.
     ``prepares_norm``: the product also does the work of the norm BEHIND it (new residual, rows times the norm's
     weights, sums of squares); the product behind that then runs with ``norm="prepared"`` (``takes_prepared``): it
     takes those rows as they are and applies the scale to its 32-bit sums."""
@@ -91,7 +94,7 @@ class ProductPlan:
         elif self.norm_folded:
             extras.insert(0, "add+norm folded in front")
         if self.activation_apart:
-            extras.append("SwiGLU as a kernel of its own")
+            extras.append("activation as a kernel of its own")
         if self.prepares_norm:
             extras.append("does the following add+norm's work")
         return f"{self.kernel} ({', '.join(extras)})"
@@ -101,10 +104,10 @@ def product(dtype: torch.dtype, rows: int, out_features: int, in_features: int, 
             norm: Optional[str] = None, contiguous_rows: bool = True, follow: bool = False) -> ProductPlan:
     """The kernel for ``[rows, in] @ [out, in]^T``.  ``norm``: ``"norm"`` or ``"add_norm"`` if an RMSNorm (with the
     residual addition) stands in front and may be folded in, ``"prepared"`` if the product in front has done that
-    norm's work; ``epilogue``: ``bf16``, ``f32`` (logits) or ``swiglu`` (the weight's rows interleave eight gates
-    and eight up projections); ``follow``: an addition and an RMSNorm of the product's own width follow it."""
+    norm's work; ``epilogue``: ``bf16``, ``f32`` (logits), or ``swiglu``, ``gated_silu`` or ``gated_gelu`` (the weight's rows interleave
+    eight gates and eight up projections; the last two without a norm folded in front); ``follow``: an addition and an RMSNorm of the product's own width follow it."""
     if dtype == torch.float32:
-        return ProductPlan("gemm_f32", False, F32, activation_apart=epilogue == SWIGLU)
+        return ProductPlan("gemm_f32", False, F32, activation_apart=epilogue in OVER_GATE_AND_UP)
     if rows <= DECODE_LINEAR_MAX_ROWS and contiguous_rows:
         if norm == "prepared":
             if _decode_linear_takes(rows, out_features, in_features, kernels.PRO_NONE):
@@ -131,7 +134,7 @@ def product(dtype: torch.dtype, rows: int, out_features: int, in_features: int, 
     if (epilogue == SWIGLU and rows >= FUSED_GATE_UP_MIN_ROWS
             and _gemm_tcgen05_takes(rows, out_features, in_features, kernels.EPI_SWIGLU)):
         return ProductPlan("gemm_tcgen05", False, SWIGLU)
-    if epilogue == SWIGLU:
+    if epilogue in OVER_GATE_AND_UP:
         return ProductPlan("library", False, BF16, activation_apart=True)
     return ProductPlan("library", False, epilogue)
 

@@ -87,6 +87,48 @@ def test_silu_mul(dtype, rows, inter):
     torch.testing.assert_close(out.cpu().double(), g / (1 + torch.exp(-g)) * u, **tol(dtype))
 
 
+def _interleave(gate, up):
+    return torch.stack([gate.reshape(-1, 8, *gate.shape[1:]), up.reshape(-1, 8, *up.shape[1:])], dim=1).reshape(-1, *gate.shape[1:])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows, inter, stride", [(1, 8, 16), (3, 200, 400), (33, 1024, 2051)])
+def test_gated_activation_of_alternating_columns(dtype, rows, inter, stride):
+    """Columns that alternate in blocks of eight give the bits of those in halves, in packets and one by one."""
+    from tesseract_b200 import kernels
+
+    torch.manual_seed(12)
+    halves = (torch.randn(rows, 2 * inter) * 3).to(dtype)
+    halves[0, :4] = torch.tensor([float("inf"), -float("inf"), float("nan"), -200.0])
+    wide = torch.zeros(rows, stride, dtype=dtype)
+    wide[:, :2 * inter] = _interleave(halves[:, :inter].t(), halves[:, inter:].t()).t()
+    for activation in (kernels.ACT_SILU, kernels.ACT_GELU_TANH):
+        want = kernels.gated_activation(dev(halves), None, torch.empty(rows, inter, dtype=dtype, device="cuda"), activation)
+        got = kernels.gated_activation(dev(wide)[:, :2 * inter], None, torch.empty_like(want), activation, interleaved=True)
+        assert torch.equal(got.view(torch.uint8), want.view(torch.uint8))
+    with pytest.raises(kernels.KernelError):
+        kernels.gated_activation(dev(halves), torch.zeros(2 * inter, device="cuda"), torch.empty_like(want), 0, interleaved=True)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 64, 128])
+@pytest.mark.parametrize("inter, k", [(8, 32), (200, 96), (2376, 512), (8192, 2048)])
+def test_products_that_activate_their_sums_store_what_the_kernel_behind_them_would(rows, inter, k):
+    """To the bit: the sums rounded, activated and rounded again, for one and two halves a tile, one and several splits of K."""
+    from tesseract_b200 import kernels
+
+    torch.manual_seed(13)
+    x, gate, up = torch.randn(rows, k).bfloat16(), (torch.randn(inter, k) * 0.1).bfloat16(), (torch.randn(inter, k) * 0.1).bfloat16()
+    weight, x = dev(_interleave(gate, up)), dev(x)
+
+    def product(out, epilogue):
+        return kernels.decode_linear(weight, out, x=x, epilogue=epilogue) if rows <= 16 else kernels.skinny_tcgen05(x, weight, out, epilogue)
+
+    plain = product(torch.empty(rows, 2 * inter, dtype=torch.bfloat16, device="cuda"), kernels.EPI_BF16)
+    for activation, epilogue in ((kernels.ACT_SILU, kernels.EPI_GATED_SILU), (kernels.ACT_GELU_TANH, kernels.EPI_GATED_GELU)):
+        want = kernels.gated_activation(plain, None, torch.empty(rows, inter, dtype=torch.bfloat16, device="cuda"), activation, interleaved=True)
+        assert torch.equal(product(torch.empty_like(want), epilogue), want)
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 1, 1), (3, 5, 7), (64, 64, 16), (65, 130, 33), (200, 96, 96), (17, 331, 72),
                                      (2, 1000, 2048)])
 def test_gemm_f32(m, n, k):
