@@ -9,7 +9,9 @@
 //   out[m, j] = round(silu(gate_j) * up_j)   (src/cuda/kernels.rs:191-208), for a weight whose rows
 // interleave gate and up in blocks of eight: rows 16b..16b+7 = gate 8b..8b+7, rows 16b+8..16b+15 = up 8b..8b+7,
 // or over such a weight the activation that a kernel behind the product would apply to its stored rows
-//   out[m, j] = round(act(round(gate_j)) * round(up_j)),  act SiLU or GELU in its tanh form, to the bit.
+//   out[m, j] = round(act(round(gate_j)) * round(up_j)),  act SiLU or GELU in its tanh form, to the bit;
+// or the gate of a slice of a table by token, out[m, j] = round(act(y[m, j]) * table[token[m], offset + j]), to the bit of the kernel
+// that would read the 32-bit rows (EPI_TOKEN_*).
 // (That kernel's launch is 2.7 us of a decode step for each feed-forward, the activation here is hidden by other CTAs' streams.)
 //
 // Two more forms move a norm's work out of the product behind it and into the product in front of it:
@@ -41,7 +43,9 @@ constexpr int kThreads = kWarps * 32;
 // to cover the memory latency alone: five stages of 32-feature tiles or six of 16-feature tiles per warp.
 
 enum Prologue : int { PRO_NONE = 0, PRO_NORM = 1, PRO_ADD_NORM = 2, PRO_SCALED = 3, PRO_SCALED_RESIDENT = 4 };
-enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3, EPI_GATED_SILU = 4, EPI_GATED_GELU = 5 };
+enum Epilogue : int { EPI_BF16 = 0, EPI_SWIGLU = 1, EPI_F32 = 2, EPI_ADD_NORM = 3, EPI_GATED_SILU = 4, EPI_GATED_GELU = 5,
+                      EPI_TOKEN_SILU = 6, EPI_TOKEN_GELU = 7 };
+__host__ __device__ constexpr bool token_gate(int epilogue) { return epilogue == EPI_TOKEN_SILU || epilogue == EPI_TOKEN_GELU; }
 constexpr int kSsStride = 16;      // floats per tile in the sums-of-squares array (rows beyond M hold zeros)
 
 struct LinearParams {
@@ -69,6 +73,11 @@ struct LinearParams {
     // stage of a two-stage argmax over the output columns (src/cuda/kernels.rs:803-873)
     float* best_value;
     int* best_index;
+    // EPI_TOKEN_*: the rows' tokens [M] and the table [vocab, table_stride], whose slice starts at column table_offset
+    const int* tokens;
+    const __nv_bfloat16* table;
+    int64_t table_stride;
+    int table_offset, vocab;
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -366,6 +375,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_linear_kernel(const Linear
             epi_r = *reinterpret_cast<const __nv_bfloat162*>(p.epi_res + (int64_t)((int)threadIdx.x % ROWS) * p.N + col);
             epi_w = *reinterpret_cast<const float2*>(p.epi_norm_w + col);
         }
+        if (token_gate(EPI) && (int)threadIdx.x < (TF / 2) * ROWS && (int)threadIdx.x % ROWS < p.M) {
+            int from = p.tokens[(int)threadIdx.x % ROWS];
+            if (from < 0 || from >= p.vocab) from = 0;      // the host validates; never read out of bounds
+            const __nv_bfloat16* e = p.table + (int64_t)from * p.table_stride + p.table_offset +
+                                     ((int)blockIdx.x + ti * (int)gridDim.x) * TF + 2 * ((int)threadIdx.x / ROWS);
+            epi_w = make_float2(__bfloat162float(e[0]), __bfloat162float(e[1]));
+        }
         for (int j = 0; j < bpw; ++j) {
             issue(true);
             cp_async_wait<STAGES - 1>();
@@ -470,6 +486,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_linear_kernel(const Linear
                     *reinterpret_cast<__nv_bfloat162*>(p.epi_res_out + at) = __floats2bfloat162_rn(c0, c1);
                     *reinterpret_cast<__nv_bfloat162*>(p.epi_xw + at) = __floats2bfloat162_rn(c0 * w2.x, c1 * w2.y);
                     ss = fmaf(c0, c0, c1 * c1);
+                } else if (token_gate(EPI)) {
+                    constexpr int ACT = EPI == EPI_TOKEN_SILU ? tbact::ACT_SILU : tbact::ACT_GELU_TANH;
+                    *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (int64_t)m * p.N + n0 + f) =
+                        __floats2bfloat162_rn(tbact::activate<ACT>(sum0) * epi_w.x, tbact::activate<ACT>(sum1) * epi_w.y);
                 } else if (EPI == EPI_F32) {
                     // columns rise from tile to tile, so "greater" alone keeps the lowest column of equal values
                     if (sum0 > best_v) { best_v = sum0; best_i = n0 + f; }
@@ -615,6 +635,8 @@ int dispatch(const LinearParams& p, int prologue, int epilogue, cudaStream_t str
     TB_CASE(PRO_NONE, EPI_SWIGLU)
     TB_CASE(PRO_NONE, EPI_GATED_SILU)
     TB_CASE(PRO_NONE, EPI_GATED_GELU)
+    TB_CASE(PRO_NONE, EPI_TOKEN_SILU)
+    TB_CASE(PRO_NONE, EPI_TOKEN_GELU)
     TB_CASE(PRO_NORM, EPI_BF16)
     TB_CASE(PRO_NORM, EPI_F32)
     TB_CASE(PRO_NORM, EPI_SWIGLU)
@@ -663,7 +685,7 @@ TB_EXPORT int tb_decode_linear_ex(const void* x, int64_t x_stride, const void* r
                                   const float* ss_in, int ss_tiles, const void* epi_res, const float* epi_norm_w,
                                   void* epi_res_out, void* epi_xw, float* epi_ss, float* best_value, int* best_index,
                                   cudaStream_t stream) {
-    if (!tb_decode_linear_supported(M, N, K, prologue)) return TB_ERR_BAD_SIZE;
+    if (!tb_decode_linear_supported(M, N, K, prologue) || token_gate(epilogue)) return TB_ERR_BAD_SIZE;
     const uintptr_t bits = (uintptr_t)x | (uintptr_t)res | (uintptr_t)upd | (uintptr_t)res_out | (uintptr_t)w |
                            (uintptr_t)epi_res | (uintptr_t)epi_res_out | (uintptr_t)epi_xw;
     const bool rows_ride = prologue == PRO_NONE || prologue == PRO_SCALED;
@@ -674,7 +696,7 @@ TB_EXPORT int tb_decode_linear_ex(const void* x, int64_t x_stride, const void* r
         (prologue != PRO_NONE || epi_res == nullptr || epi_norm_w == nullptr || epi_res_out == nullptr ||
          epi_xw == nullptr || epi_ss == nullptr || epi_res_out == epi_res || (uintptr_t)epi_norm_w % 8 != 0))
         return TB_ERR_BAD_ALIGN;
-    LinearParams p;
+    LinearParams p = {};
     p.x = (const __nv_bfloat16*)x;
     p.res = (const __nv_bfloat16*)res;
     p.upd = (const __nv_bfloat16*)upd;
@@ -715,4 +737,30 @@ TB_EXPORT int tb_decode_linear(const void* x, int64_t x_stride, const void* res,
     if (prologue == PRO_SCALED || epilogue == EPI_ADD_NORM) return TB_ERR_BAD_SIZE;
     return tb_decode_linear_ex(x, x_stride, res, upd, norm_w, eps, res_out, w, out, out_stride, M, N, K, prologue,
                                epilogue, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, stream);
+}
+
+// out[m, j] = round(act(x . w_j) * table[tokens[m], offset + j]) for a bfloat16 table [vocab, table_stride]; out [M, N] contiguous;
+// activation: 0 SiLU, 1 GELU in its tanh form.
+TB_EXPORT int tb_decode_linear_token_gate(const void* x, int64_t x_stride, const void* w, const int* tokens, const void* table,
+                                          int64_t table_stride, int offset, int vocab, void* out, int M, int N, int K,
+                                          int activation, cudaStream_t stream) {
+    if (!tb_decode_linear_supported(M, N, K, PRO_NONE)) return TB_ERR_BAD_SIZE;
+    if (activation < 0 || activation > 1 || offset < 0 || offset + N > table_stride || vocab < 1) return TB_ERR_BAD_SIZE;
+    if (((uintptr_t)x | (uintptr_t)w) % 16 != 0 || x_stride % 8 != 0 || (uintptr_t)out % 4 != 0) return TB_ERR_BAD_ALIGN;
+    LinearParams p = {};
+    p.x = (const __nv_bfloat16*)x;
+    p.w = (const __nv_bfloat16*)w;
+    p.out = out;
+    p.x_stride = x_stride;
+    p.out_stride = N;
+    p.M = M;
+    p.N = N;
+    p.K = K;
+    p.tokens = tokens;
+    p.table = (const __nv_bfloat16*)table;
+    p.table_stride = table_stride;
+    p.table_offset = offset;
+    p.vocab = vocab;
+    const int epilogue = activation == 0 ? EPI_TOKEN_SILU : EPI_TOKEN_GELU;
+    return M <= 8 ? dispatch<1>(p, PRO_NONE, epilogue, stream) : dispatch<2>(p, PRO_NONE, epilogue, stream);
 }

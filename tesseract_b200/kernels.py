@@ -554,6 +554,24 @@ def decode_linear(weight: torch.Tensor, out: Optional[torch.Tensor], *, x: Optio
     return out
 
 
+def decode_linear_token_gate(x: torch.Tensor, weight: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, offset: int,
+                             out: torch.Tensor, activation: int) -> torch.Tensor:
+    """:func:`token_gate` of the 32-bit product ``x @ weight^T`` for at most 16 rows, in the product's kernel."""
+    _cuda(x, weight, tokens, table, out)
+    rows, k = x.shape
+    n = weight.shape[0]
+    _need(x.dtype == weight.dtype == table.dtype == out.dtype == torch.bfloat16, "decode_linear_token_gate takes bfloat16")
+    _need(x.stride(1) == 1 and weight.is_contiguous() and weight.shape[1] == k, "decode_linear_token_gate layout")
+    _need(tokens.dtype == torch.int32 and tokens.is_contiguous() and tokens.numel() >= rows, "decode_linear_token_gate tokens")
+    _need(table.stride(1) == 1 and 0 <= offset and offset + n <= table.shape[1], "decode_linear_token_gate table")
+    _need(out.is_contiguous() and tuple(out.shape) == (rows, n), "decode_linear_token_gate out")
+    lib = load_library("decode_linear")
+    _check(lib.tb_decode_linear_token_gate(_ptr(x), _i64(x.stride(0)), _ptr(weight), _ptr(tokens), _ptr(table), _i64(table.stride(0)),
+                                           _i32(offset), _i32(table.shape[0]), _ptr(out), _i32(rows), _i32(n), _i32(k),
+                                           _i32(activation), _stream()), "decode_linear_token_gate")
+    return out
+
+
 _tcgen05_error = {}
 
 

@@ -81,9 +81,13 @@ class GatedTokenSlice(TokenInput):
         rows = residual.shape[0]
         if rounded is None:
             rounded = residual if self.runtime.is_float32 else residual.to(self.runtime.dtype)
-        z = self.gate_proj.forward(rounded, float32_out=True)
         g = torch.empty((rows, self.dim), dtype=self.runtime.dtype, device=residual.device)
-        kernels.token_gate(z, ctx.token_ids, self.table, self.slice * self.dim, g, self.activation)
+        if self.gate_proj.plan(rows, plan.F32).kernel == "decode_linear":
+            kernels.decode_linear_token_gate(rounded, self.gate_proj.weight, ctx.token_ids, self.table, self.slice * self.dim, g,
+                                             self.activation)
+        else:
+            z = self.gate_proj.forward(rounded, float32_out=True)
+            kernels.token_gate(z, ctx.token_ids, self.table, self.slice * self.dim, g, self.activation)
         y = self.out_proj.forward(g, float32_out=True)
         if following is None:
             kernels.norm_add_norm(residual, y, (kernels.NORM_RMS, self.norm_weight, None), None, None, None, self.eps)

@@ -129,6 +129,24 @@ def test_products_that_activate_their_sums_store_what_the_kernel_behind_them_wou
         assert torch.equal(product(torch.empty_like(want), epilogue), want)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+@pytest.mark.parametrize("n, k, offset", [(16, 32, 0), (128, 2048, 256), (4752, 96, 1)])
+def test_a_product_that_gates_by_token_stores_what_the_kernel_behind_it_would(rows, n, k, offset):
+    from tesseract_b200 import kernels
+
+    torch.manual_seed(14)
+    x, weight = dev(torch.randn(rows, k).bfloat16()), dev((torch.randn(n, k) * 0.2).bfloat16())
+    table = dev(torch.randn(9, offset + n + 3).bfloat16())
+    tokens = dev((torch.arange(rows, dtype=torch.int32) * 7) % 12 - 1)              # (one below and some behind the table: row 0)
+    z = kernels.decode_linear(weight, torch.empty(rows, n, device="cuda"), x=x, epilogue=kernels.EPI_F32)
+    for activation in (kernels.ACT_SILU, kernels.ACT_GELU_TANH):
+        want = kernels.token_gate(z, tokens, table, offset, torch.empty(rows, n, dtype=torch.bfloat16, device="cuda"), activation)
+        got = kernels.decode_linear_token_gate(x, weight, tokens, table, offset, torch.empty_like(want), activation)
+        assert torch.equal(got, want)
+    with pytest.raises(kernels.KernelError):
+        kernels.decode_linear_token_gate(x, weight, tokens, table, offset + 4, torch.empty_like(want), 0)
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 1, 1), (3, 5, 7), (64, 64, 16), (65, 130, 33), (200, 96, 96), (17, 331, 72),
                                      (2, 1000, 2048)])
 def test_gemm_f32(m, n, k):
