@@ -1,4 +1,4 @@
-// Plain paged attention: one warp per (query row, query head), keys walked in ascending
+// Plain paged attention: one warp (in steps of few rows a block) per (query row, query head), keys walked in ascending
 // blocks of 32 through the request's block table.  It serves the 32-bit path of every
 // model and any size the fast bfloat16 kernels refuse.
 //
@@ -163,11 +163,141 @@ attention_rows_kernel(const T* __restrict__ q, int64_t q_stride, T* __restrict__
     }
 }
 
+// The same work, to the bit, by a block a (row, head): eight warps take the scores of its key blocks side by side and leave them in
+// shared memory; since a running maximum is the same maximum however it is found, the weights of all blocks follow side by side as
+// well; what is left to go in order, block by block and key by key, is the sum over the weights and that over the values, a warp 32
+// columns of it, the next block's values on their way.  Runs of kRun blocks, so that any context fits.
+constexpr int kSharedWarps = 8, kRun = 64;
+
+template <typename T, int NC>
+__global__ void __launch_bounds__(kSharedWarps * 32, 2)
+attention_rows_shared_kernel(const T* q, int64_t q_stride, T* out, int64_t out_stride, const T* cache,
+                             const int* __restrict__ positions, const int* __restrict__ seq_of_row,
+                             const int* __restrict__ block_table, int bt_stride, int num_heads, int num_kv_heads, int head_dim,
+                             int page_size, int window, float scale) {
+    constexpr int UNDER = 32 / Vec16<T>::N;            // packets of a key under way
+    __shared__ float score[kRun * kKeyBlock];        // then the weights
+    __shared__ int64_t offset[kRun * kKeyBlock];     // of a key in its half of the cache
+    __shared__ float block_max[kRun], block_sum_of[kRun], max_so_far[kRun], qs[NC * 32];
+    pdl_trigger();
+    pdl_wait();                                      // rows, keys and the step's metadata come from kernels in front
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row = blockIdx.x, head = blockIdx.y, kv_head = head / (num_heads / num_kv_heads);
+    const int pos = positions[row];
+    const int first_key = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+    const int* table = block_table + (int64_t)seq_of_row[row] * bt_stride;
+    const T* qrow = q + (int64_t)row * q_stride + (int64_t)head * head_dim;
+    for (int i = threadIdx.x; i < head_dim; i += kSharedWarps * 32) qs[i] = Elem<T>::load(qrow + i);
+    __syncthreads();
+    const int64_t head_block = (int64_t)page_size * head_dim;
+    const int64_t page_block = 2 * (int64_t)num_kv_heads * head_block;
+    const T* kbase = cache + (int64_t)kv_head * head_block;
+    const T* vbase = kbase + (int64_t)num_kv_heads * head_block;
+    const int col = warp * 32 + lane;
+    const bool has_columns = warp < NC;
+
+    float m = -1.0e30f, l = 0.0f, acc = 0.0f;
+    const int last_block = pos / kKeyBlock;
+    for (int kb0 = first_key / kKeyBlock; kb0 <= last_block; kb0 += kRun) {
+        const int blocks = min(kRun, last_block - kb0 + 1);
+        for (int b = warp; b < blocks; b += kSharedWarps) {
+            const int key = (kb0 + b) * kKeyBlock + lane;
+            const bool valid = key >= first_key && key <= pos;
+            int64_t at = 0;
+            float s = -1.0e30f;
+            if (valid) {
+                at = (int64_t)table[key / page_size] * page_block + (int64_t)(key % page_size) * head_dim;
+                const T* kp = kbase + at;
+                float dot = 0.0f;
+                for (int i0 = 0; i0 < head_dim; i0 += UNDER * Vec16<T>::N) {
+                    float kv[UNDER][Vec16<T>::N];
+#pragma unroll
+                    for (int u = 0; u < UNDER; ++u)
+                        if (i0 + u * Vec16<T>::N < head_dim) Vec16<T>::load(kp + i0 + u * Vec16<T>::N, kv[u]);
+#pragma unroll
+                    for (int u = 0; u < UNDER; ++u)
+                        if (i0 + u * Vec16<T>::N < head_dim) {
+#pragma unroll
+                            for (int e = 0; e < Vec16<T>::N; ++e) dot = fmaf(qs[i0 + u * Vec16<T>::N + e], kv[u][e], dot);
+                        }
+                }
+                s = dot * scale;
+            }
+            score[b * kKeyBlock + lane] = s;
+            offset[b * kKeyBlock + lane] = at;
+            s = warp_max(s);
+            if (lane == 0) block_max[b] = s;
+        }
+        __syncthreads();
+        float v[2][kKeyBlock];
+        auto ask = [&](int b, float (&to)[kKeyBlock]) {
+            if (!has_columns || b >= blocks) return;
+            const int keys = min(kKeyBlock, pos - (kb0 + b) * kKeyBlock + 1);
+#pragma unroll
+            for (int j = 0; j < kKeyBlock; ++j)
+                to[j] = j < keys && col < head_dim ? Elem<T>::load(vbase + offset[b * kKeyBlock + j] + col) : 0.0f;
+        };
+        ask(0, v[0]);
+        for (int b = warp; b < blocks; b += kSharedWarps) {
+            float before = -1.0e30f;
+            for (int i = lane; i < b; i += 32) before = fmaxf(before, block_max[i]);
+            const float m_new = fmaxf(fmaxf(m, warp_max(before)), block_max[b]);
+            const int key = (kb0 + b) * kKeyBlock + lane;
+            const float p = key >= first_key && key <= pos ? expf(score[b * kKeyBlock + lane] - m_new) : 0.0f;
+            const float sum = warp_sum(p);
+            score[b * kKeyBlock + lane] = Elem<T>::round(p);
+            if (lane == 0) {
+                block_sum_of[b] = sum;
+                max_so_far[b] = m_new;
+            }
+        }
+        __syncthreads();
+        if (has_columns) {
+            auto take = [&](int b, const float (&values)[kKeyBlock]) {
+                const float m_new = max_so_far[b], corr = expf(m - m_new);
+                l = l * corr + block_sum_of[b];
+                acc *= corr;
+                const int keys = min(kKeyBlock, pos - (kb0 + b) * kKeyBlock + 1);
+#pragma unroll
+                for (int j = 0; j < kKeyBlock; ++j) {
+                    const float pj = score[b * kKeyBlock + j];
+                    if (j < keys && pj != 0.0f) acc = fmaf(pj, values[j], acc);
+                }
+                m = m_new;
+            };
+            for (int b = 0; b < blocks; b += 2) {
+                ask(b + 1, v[1]);
+                take(b, v[0]);
+                if (b + 1 >= blocks) break;
+                ask(b + 2, v[0]);
+                take(b + 1, v[1]);
+            }
+        }
+        m = max_so_far[blocks - 1];
+        __syncthreads();                             // (the next run writes over this one's scores)
+    }
+    if (has_columns && col < head_dim)
+        Elem<T>::store(out + (int64_t)row * out_stride + (int64_t)head * head_dim + col, acc / fmaxf(l, 1.0e-8f));
+}
+
 template <typename T>
 int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
            const int* positions, const int* seq_of_row, const int* block_table, int bt_stride, int rows,
            int num_heads, int num_kv_heads, int head_dim, int page_size, int window, float scale,
            cudaStream_t stream) {
+    // Few rows: 4 and 8 rows of 32 heads of 64 behind 130 keys, 32-bit, 9.4 and 9.7 us against 16.5 and 16.6 by a warp a (row, head), behind
+    // 6,000 keys 295 and 308 against 690 and 725; 16 rows 18.5 against 16.7, for then the blocks take turns on a multiprocessor (two fit).
+    // Of 128 or 256 numbers twice as many blocks still gain (16 rows of 32 heads of 128: 23.3 against 29.6), in bfloat16 they do not (40.8
+    // and 33.4), and heads of 32 in bfloat16 lose with any (17.6 and 14.2).
+    const int most = sizeof(T) == 4 ? (head_dim > 64 ? 592 : 296) : head_dim > 32 ? 296 : 0;
+    if ((int64_t)rows * num_heads <= most) {
+        auto kernel = head_dim <= 32 ? attention_rows_shared_kernel<T, 1> : head_dim <= 64 ? attention_rows_shared_kernel<T, 2>
+                    : head_dim <= 128 ? attention_rows_shared_kernel<T, 4> : attention_rows_shared_kernel<T, 8>;
+        const cudaError_t launched = tb_launch_pdl(kernel, dim3(rows, num_heads), dim3(kSharedWarps * 32), (size_t)0, stream, (const T*)q,
+                                                   q_stride, (T*)out, out_stride, (const T*)cache, positions, seq_of_row, block_table,
+                                                   bt_stride, num_heads, num_kv_heads, head_dim, page_size, window, scale);
+        return launched == cudaSuccess ? tb_launch_status() : (int)launched;
+    }
     dim3 grid(rows, (num_heads + kWarpsPerBlock - 1) / kWarpsPerBlock);
     const size_t smem = (size_t)kWarpsPerBlock * head_dim * sizeof(float);
 #define TB_LAUNCH(NC, UNDER)                                                                                          \
