@@ -154,8 +154,14 @@ constexpr int kTile = 16;            // the most rows of a tile
 template <int KIND>
 struct Coefficients { static constexpr int N = KIND == DELTA ? 44 : 32; };
 
-template <typename T, int KIND, int LPC, int NJ>
-__global__ void __launch_bounds__((kWorkers + kProducers) * 32)
+// (A block holds at most 32 columns: with eight lanes a column four warps of state.)  BLOCKS: on a multiprocessor.  With 128 registers a
+// thread two blocks of eight lanes a column fit, and steps that have them are bound by the chain of a group, which the other block
+// hides: 32 sequences of 75 rows, state space / delta rule, 276 / 203 us, one block 356 / 240.  A single prompt has a block a
+// multiprocessor and wants the registers (2,048 rows of the state space: 275 us, 326 with 128).
+constexpr int most_workers(int lpc) { return lpc / 2 < kWorkers ? lpc / 2 : kWorkers; }
+
+template <typename T, int KIND, int LPC, int NJ, int BLOCKS>
+__global__ void __launch_bounds__((most_workers(LPC) + kProducers) * 32, BLOCKS)
 matrix_recurrence_kernel(const T* __restrict__ rows, Recurrence p) {
     constexpr int DP = 4 * LPC * NJ;                 // numbers of q or k in shared memory (zeros behind dim)
     constexpr int CPL = 2, CW = 32 / LPC * CPL;
@@ -683,7 +689,11 @@ int launch_as(const void* rows, Recurrence p, int num_seqs, int single, cudaStre
     p.tile = DP > 512 ? kTile / 2 : kTile;
     const int VC = p.workers * CW;
     const size_t smem = sizeof(float) * 2 * (p.tile * (2 * DP + VC) + p.tile / kGroup * Coefficients<KIND>::N);
-    auto kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ>;
+    const int64_t blocks = (int64_t)num_seqs * p.heads * ((p.columns + VC - 1) / VC);
+    auto kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, 1>;
+    if constexpr (LPC == 8) {
+        if (blocks > 148) kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, 2>;
+    }
     if (smem > 40 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return (int)err;
@@ -786,23 +796,27 @@ recurrence_norm_kernel(const float* __restrict__ v, const float* __restrict__ au
 // The same in packets of four numbers, where sizes and rows allow them.
 template <typename T, bool WIDE, int KEEP>
 __global__ void __launch_bounds__(WIDE ? 256 : kNormThreads)
-recurrence_norm_packets_kernel(const float* __restrict__ v, const float* __restrict__ aux, const T* __restrict__ gate,
-                               int64_t gate_stride, const float* __restrict__ weight, int weight_len, T* __restrict__ out,
+recurrence_norm_packets_kernel(const float* v, const float* aux, const T* gate,
+                               int64_t gate_stride, const float* __restrict__ weight, int weight_len, T* out,
                                int64_t out_stride, int groups, int size, float eps, int gate_kind) {
     __shared__ float scratch[32];
     pdl_trigger();
-    pdl_wait();
     constexpr int STEP = WIDE ? 256 : 32;            // rows of up to 4 * STEP * KEEP numbers
     const int lane = WIDE ? threadIdx.x : threadIdx.x & 31;
     const int row = blockIdx.x;
     const int g = WIDE ? blockIdx.y : blockIdx.y * (kNormThreads / 32) + (threadIdx.x >> 5);
-    if (g >= groups) return;
+    if (g >= groups) return;                         // (a warp of its own)
     const float* src = v + ((int64_t)row * groups + g) * size;
     const T* grow = gate + (int64_t)row * gate_stride + (int64_t)g * size;
     T* dst = out + (int64_t)row * out_stride + (int64_t)g * size;
     const float* w = weight + (weight_len == size ? 0 : (int64_t)g * size);
     const int packets = size / 4;
-    float4 x[KEEP], z[KEEP];
+    constexpr int EARLY = KEEP < 4 ? KEEP : 4;       // packets of the weights that are asked for before the wait
+    float4 x[KEEP], z[KEEP], f[EARLY];
+#pragma unroll
+    for (int e = 0; e < EARLY; ++e)
+        if (e * STEP + lane < packets) f[e] = *reinterpret_cast<const float4*>(w + 4 * (e * STEP + lane));
+    pdl_wait();
     float before = 1.0f;
 #pragma unroll
     for (int e = 0; e < KEEP; ++e) {                 // everything the row needs is asked for at once
@@ -831,8 +845,8 @@ recurrence_norm_packets_kernel(const float* __restrict__ v, const float* __restr
     for (int e = 0; e < KEEP; ++e) {
         const int i = 4 * (e * STEP + lane);
         if (e * STEP + lane >= packets) continue;
-        const float4 f = *reinterpret_cast<const float4*>(w + i);
-        float4 y = make_float4(x[e].x * inv * f.x, x[e].y * inv * f.y, x[e].z * inv * f.z, x[e].w * inv * f.w);
+        const float4 by = e < EARLY ? f[e < EARLY ? e : 0] : *reinterpret_cast<const float4*>(w + i);
+        float4 y = make_float4(x[e].x * inv * by.x, x[e].y * inv * by.y, x[e].z * inv * by.z, x[e].w * inv * by.w);
         if (gate_kind != GATE_SILU_FIRST) { y.x *= z[e].x; y.y *= z[e].y; y.z *= z[e].z; y.w *= z[e].w; }
         store4<T>(dst + i, y);
     }
