@@ -69,8 +69,7 @@ struct Layout {
 
 template <int D, int DV>
 __global__ void __launch_bounds__(128)
-attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __restrict__ out, int64_t out_stride,
-                        const bf16* __restrict__ cache, const int* __restrict__ positions,
+attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
                         const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
                         int page_size, int mask_kind, int mask_size, float scale, float* __restrict__ parts) {
     typedef Layout<D, DV> L;
@@ -78,7 +77,6 @@ attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
     constexpr int COLS = DV / 4;                                  // value columns a warp owns
     extern __shared__ __align__(128) unsigned char smem[];
     pdl_trigger();
-    pdl_wait();                                                   // queries, pages and the step's metadata come from kernels in front
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int row = blockIdx.x, head0 = blockIdx.y * 16;
     const int pos = positions[row], seq = seq_of_row[row];
@@ -93,21 +91,30 @@ attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     float* stats = reinterpret_cast<float*>(smem + L::STAT_AT);
 
-    const int copy_row = tid >> 1, copy_half = tid & 1;
-    auto fill = [&](int tile) {
+    // a tile's copy: sixteen lanes a key, whose 16-byte chunks they take side by side, eight keys at a time
+    const int shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;      // (pages are a power of two of tokens in all but odd cases)
+    auto page_of = [&](int key) { return shift >= 0 ? key >> shift : key / page_size; };
+    auto look = [&](int tile, int (&pages)[KT / 8]) {             // where this thread's keys lie
+#pragma unroll
+        for (int i = 0; i < KT / 8; ++i) pages[i] = table[page_of(min(key_lo + tile * KT + i * 8 + (tid >> 4), pos))];
+    };
+    auto fill = [&](int tile, const int (&pages)[KT / 8]) {
         const uint32_t stage = base + (uint32_t)(tile & 1) * L::STAGE;
-        const int key = key_lo + tile * KT + copy_row;
-        const bool there = key <= pos;
-        const int k = there ? key : pos;
-        const bf16* kp = cache + (int64_t)table[k / page_size] * page_elems + (int64_t)(k % page_size) * D;
-        const int bytes = there ? 16 : 0;                         // (a key behind the last one is zero-filled)
-        constexpr int KC = D / 8;
-#pragma unroll 4
-        for (int c = 0; c < KC / 2; ++c) {
-            const int chunk = copy_half * (KC / 2) + c;
-            cp_async16(stage + copy_row * KS + chunk * 16, kp + chunk * 8, bytes);
+#pragma unroll
+        for (int i = 0; i < KT / 8; ++i) {
+            const int row = i * 8 + (tid >> 4), key = key_lo + tile * KT + row, k = min(key, pos);
+            const bf16* kp = cache + (int64_t)pages[i] * page_elems + (int64_t)(k - page_of(k) * page_size) * D;
+            const int bytes = key <= pos ? 16 : 0;                // (a key behind the last one is zero-filled)
+#pragma unroll
+            for (int c = 0; c < D / 8; c += 16) {
+                const int chunk = c + (tid & 15);
+                if (D % 128 == 0 || chunk < D / 8) cp_async16(stage + row * KS + chunk * 16, kp + chunk * 8, bytes);
+            }
         }
     };
+    int pages[KT / 8];
+    look(tile_first, pages);
+    pdl_wait();                                                   // queries and the step's keys come from kernels in front, its metadata does not
     // the sixteen heads' queries (heads the model does not have are rows of zeros)
     for (int index = tid; index < 16 * (D / 8); index += 128) {
         const int h = index / (D / 8), chunk = index % (D / 8);
@@ -115,8 +122,9 @@ attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
         const bf16* src = q + (int64_t)row * q_stride + (int64_t)(there ? head0 + h : head0) * D + chunk * 8;
         cp_async16(base + L::Q_AT + h * KS + chunk * 16, src, there ? 16 : 0);
     }
-    if (tile_first < tile_end) fill(tile_first);
+    if (tile_first < tile_end) fill(tile_first, pages);
     cp_async_commit();
+    look(tile_first + 1, pages);                                  // (a tile ahead from here on)
 
     float m[2] = {-1.0e30f, -1.0e30f}, l[2] = {0.0f, 0.0f};
     float o[COLS / 8][4];
@@ -127,7 +135,8 @@ attention_latent_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
 
     for (int tile = tile_first; tile < tile_end; ++tile) {
         if (tile + 1 < tile_end) {
-            fill(tile + 1);
+            fill(tile + 1, pages);
+            look(tile + 2, pages);
             cp_async_commit();
             cp_async_wait<1>();
         } else {

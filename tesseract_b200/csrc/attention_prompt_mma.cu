@@ -109,6 +109,31 @@ __device__ __forceinline__ float distance_bias(float weight, float rate, int dis
 }
 
 // BIASED: the scores lose their distance bias (a kernel of its own: the others keep their registers).
+// Pages are a power of two of tokens in all but odd cases, and a thread looks up many keys.
+struct Pages {
+    int size, shift;                                              // shift: -1 where it takes a division
+    __device__ __forceinline__ int of(int key) const { return shift >= 0 ? key >> shift : key / size; }
+    __device__ __forceinline__ int within(int key) const { return shift >= 0 ? key & (size - 1) : key % size; }
+};
+__device__ __forceinline__ Pages pages_of(int page_size) {
+    Pages p;
+    p.size = page_size;
+    p.shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;
+    return p;
+}
+
+// A key's and its value's 16-byte chunks, by eight lanes side by side (bytes 0: zeros).  By two threads a key, half a row each, a warp's
+// copies touched 32 half sectors of 16 rows, and the copies bound decoded rows: 128 rows of 8 kv heads of 128 behind 4,000 keys
+// 766 us, 426 so.
+template <int D, int DV>
+__device__ __forceinline__ void copy_key(uint32_t to_key, uint32_t to_value, const bf16* key, const bf16* value, int lane, int bytes) {
+#pragma unroll
+    for (int c = 0; c < D / 8; c += 8) cp_async16(to_key + (c + lane) * 16, key + (c + lane) * 8, bytes);
+#pragma unroll
+    for (int c = 0; c < DV / 8; c += 8)
+        if (DV % 64 == 0 || c + lane < DV / 8) cp_async16(to_value + (c + lane) * 16, value + (c + lane) * 8, bytes);
+}
+
 template <int D, int DV, bool BIASED>
 __global__ void __launch_bounds__(128)
 attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __restrict__ out, int64_t out_stride,
@@ -158,32 +183,29 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
     const int* pool_table = x.pool_table == nullptr ? nullptr : x.pool_table + (int64_t)seq * x.pool_bt_stride;
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(tile_smem);
 
-    // a tile's copy: two threads a key; one takes the first half of the key's and of the value's 16-byte chunks, the
-    // other the second half
-    const int copy_row = tid >> 1, copy_half = tid & 1;
+    // a tile's copy: eight lanes a key, whose 16-byte chunks they take side by side, sixteen keys at a time
+    const Pages paging = pages_of(page_size);
     auto fill = [&](int tile) {
         const uint32_t stage = smem_base + (uint32_t)(tile & 1) * STAGE;
-        const int at = tile * KT + copy_row;
-        const bool there = at < span;
-        const int a = there ? at : span - 1;
-        const bool averaged = averages && a < blocks_last;
-        const int k = a < blocks_last ? a : key_lo + a - blocks_last;
-        const bf16* from = averaged ? x.pool_cache : cache;
-        const int64_t base = (int64_t)(averaged ? pool_table : table)[k / page_size] * page_elems;
-        const int in_page = k % page_size;
-        const bf16* kp = from + k_off + base + (int64_t)in_page * D;
-        const bf16* vp = from + v_off + base + (int64_t)in_page * DV;
-        const int bytes = there ? 16 : 0;                         // (a key behind the last one is zero-filled)
-        constexpr int KC = D / 8, VC = DV / 8;
+        int pages[KT / 16];
+        auto key_at = [&](int i, bool& averaged) {
+            const int a = min(tile * KT + i * 16 + (tid >> 3), span - 1);
+            averaged = averages && a < blocks_last;
+            return a < blocks_last ? a : key_lo + a - blocks_last;
+        };
 #pragma unroll
-        for (int c = 0; c < (KC + 1) / 2; ++c) {
-            const int chunk = copy_half * ((KC + 1) / 2) + c;
-            if (chunk < KC) cp_async16(stage + copy_row * KS + chunk * 16, kp + chunk * 8, bytes);
+        for (int i = 0; i < KT / 16; ++i) {
+            bool averaged;
+            const int k = key_at(i, averaged);
+            pages[i] = (averaged ? pool_table : table)[paging.of(k)];
         }
 #pragma unroll
-        for (int c = 0; c < (VC + 1) / 2; ++c) {
-            const int chunk = copy_half * ((VC + 1) / 2) + c;
-            if (chunk < VC) cp_async16(stage + KT * KS + copy_row * VS + chunk * 16, vp + chunk * 8, bytes);
+        for (int i = 0; i < KT / 16; ++i) {
+            bool averaged;
+            const int k = key_at(i, averaged), row = i * 16 + (tid >> 3);
+            const bf16* from = (averaged ? x.pool_cache : cache) + (int64_t)pages[i] * page_elems;
+            copy_key<D, DV>(stage + row * KS, stage + KT * KS + row * VS, from + k_off + (int64_t)paging.within(k) * D,
+                            from + v_off + (int64_t)paging.within(k) * DV, tid & 7, tile * KT + row < span ? 16 : 0);
         }
     };
     fill(0);
@@ -364,19 +386,20 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
 // are the 16 rows of the first operand, so a key or value is fetched once for all of them; the block's four warps
 // share every tile of 64 keys, 16 keys a warp, each with a streaming softmax of its own, and their partial results
 // (maximum, sum, accumulator) meet in shared memory in warp order.
-template <int D, int DV, bool BIASED>
+// STAGES: tiles in shared memory.  Where every block has room for kDeep of them they are asked for that far ahead, with one barrier a
+// tile; the first tiles' pages are looked up before the wait (the step's metadata comes from no kernel), the others' a tile ahead.
+// (The queries are not __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
+template <int D, int DV, bool BIASED, int STAGES>
 __global__ void __launch_bounds__(128)
-attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __restrict__ out, int64_t out_stride,
-                      const bf16* __restrict__ cache, const int* __restrict__ positions,
+attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
                       const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
                       int kv_heads, int page_size, int mask_kind, int mask_size, float scale, int keys_per_value,
                       int out_f32, Extras x) {
     constexpr int KS = D * 2 + 16, VS = DV * 2 + 16;
     constexpr int STAGE = KT * (KS + VS);
     constexpr int PART = DV + 2;                                  // a row's accumulator, maximum and sum
-    extern __shared__ __align__(128) unsigned char tile_smem[];   // two stages, then [4 warps][16 rows][PART] floats
+    extern __shared__ __align__(128) unsigned char tile_smem[];   // the stages, then [4 warps][16 rows][PART] floats
     pdl_trigger();
-    pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int row = blockIdx.x, kv_head = blockIdx.y, per = heads / kv_heads;
     const int pos = positions[row], seq = seq_of_row[row];
@@ -393,34 +416,30 @@ attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __rest
     const int* table = block_table + (int64_t)seq * bt_stride;
     const int* pool_table = x.pool_table == nullptr ? nullptr : x.pool_table + (int64_t)seq * x.pool_bt_stride;
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(tile_smem);
-    const int copy_row = tid >> 1, copy_half = tid & 1;
-    auto fill = [&](int tile) {
-        const uint32_t stage = smem_base + (uint32_t)(tile & 1) * STAGE;
-        const int at = tile * KT + copy_row;
-        const bool there = at < span;
-        const int a = there ? at : span - 1;
-        const bool averaged = averages && a < blocks;
-        const int k = a < blocks ? a : key_lo + a - blocks;
-        const bf16* from = averaged ? x.pool_cache : cache;
-        const int64_t base = (int64_t)(averaged ? pool_table : table)[k / page_size] * page_elems;
-        const int in_page = k % page_size;
-        const bf16* kp = from + k_off + base + (int64_t)in_page * D;
-        const bf16* vp = from + v_off + base + (int64_t)in_page * DV;
-        const int bytes = there ? 16 : 0;
-        constexpr int KC = D / 8, VC = DV / 8;
+    const Pages paging = pages_of(page_size);
+    auto key_at = [&](int tile, int i) { return min(tile * KT + i * 16 + (tid >> 3), span - 1); };      // of the keys in walking order
+    auto look = [&](int tile, int (&pages)[KT / 16]) {            // where this thread's keys of a tile lie
 #pragma unroll
-        for (int c = 0; c < (KC + 1) / 2; ++c) {
-            const int chunk = copy_half * ((KC + 1) / 2) + c;
-            if (chunk < KC) cp_async16(stage + copy_row * KS + chunk * 16, kp + chunk * 8, bytes);
-        }
-#pragma unroll
-        for (int c = 0; c < (VC + 1) / 2; ++c) {
-            const int chunk = copy_half * ((VC + 1) / 2) + c;
-            if (chunk < VC) cp_async16(stage + KT * KS + copy_row * VS + chunk * 16, vp + chunk * 8, bytes);
+        for (int i = 0; i < KT / 16; ++i) {
+            const int a = key_at(tile, i);
+            pages[i] = (averages && a < blocks ? pool_table : table)[paging.of(a < blocks ? a : key_lo + a - blocks)];
         }
     };
-    fill(0);
-    cp_async_commit();
+    auto fill = [&](int tile, const int (&pages)[KT / 16]) {      // eight lanes a key, sixteen keys at a time
+        const uint32_t stage = smem_base + (uint32_t)(tile % STAGES) * STAGE;
+#pragma unroll
+        for (int i = 0; i < KT / 16; ++i) {
+            const int a = key_at(tile, i), k = a < blocks ? a : key_lo + a - blocks, copied = i * 16 + (tid >> 3);
+            const bf16* from = (averages && a < blocks ? x.pool_cache : cache) + (int64_t)pages[i] * page_elems;
+            copy_key<D, DV>(stage + copied * KS, stage + KT * KS + copied * VS, from + k_off + (int64_t)paging.within(k) * D,
+                            from + v_off + (int64_t)paging.within(k) * DV, tid & 7, tile * KT + copied < span ? 16 : 0);
+        }
+    };
+    int early[STAGES - 1][KT / 16], pages[KT / 16];
+#pragma unroll
+    for (int st = 0; st < STAGES - 1; ++st)
+        if (st < tiles) look(st, early[st]);
+    pdl_wait();                                                   // queries and the step's keys come from kernels in front
     uint32_t qa[D / 16][4];
     {
         const bool top_there = g < per, bottom_there = g + 8 < per;
@@ -434,6 +453,12 @@ attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __rest
             qa[ks][3] = bottom_there ? *reinterpret_cast<const uint32_t*>(bottom + ks * 16 + 2 * t + 8) : 0u;
         }
     }
+#pragma unroll
+    for (int st = 0; st < STAGES - 1; ++st) {
+        if (st < tiles) fill(st, early[st]);
+        cp_async_commit();
+    }
+    look(STAGES - 1, pages);                                      // (a tile ahead from here on)
     float m[2] = {-1.0e30f, -1.0e30f}, l[2] = {0.0f, 0.0f};
     if (x.sinks != nullptr && warp == 0) {                        // the sink is the start of ONE of the four running softmaxes
 #pragma unroll
@@ -458,15 +483,16 @@ attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __rest
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.0f;
     for (int tile = 0; tile < tiles; ++tile) {
-        if (tile + 1 < tiles) {
-            fill(tile + 1);
+        auto ask = [&]() {
+            if (tile + STAGES - 1 < tiles) fill(tile + STAGES - 1, pages);
             cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const uint32_t kstage = smem_base + (uint32_t)(tile & 1) * STAGE, vstage = kstage + KT * KS;
+            look(tile + STAGES, pages);
+        };
+        if (STAGES == 2) ask();
+        cp_async_wait<STAGES == 2 ? 1 : STAGES - 2>();
+        __syncthreads();                                          // (STAGES > 2: and the stage of the tile in front is free)
+        if (STAGES > 2) ask();
+        const uint32_t kstage = smem_base + (uint32_t)(tile % STAGES) * STAGE, vstage = kstage + KT * KS;
         const int at0 = tile * KT + warp * 16;                    // the warp's 16 keys of the tile
         if (at0 < span) {
             float s[2][4];
@@ -532,10 +558,10 @@ attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __rest
                 mma_bf16_16816(o[2 * jp + 1], lo, b + 2);
             }
         }
-        __syncthreads();
+        if (STAGES == 2) __syncthreads();
     }
     // the warps' partial results, then their sum in warp order
-    float* parts = reinterpret_cast<float*>(tile_smem + 2 * STAGE);
+    float* parts = reinterpret_cast<float*>(tile_smem + STAGES * STAGE);
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
@@ -572,13 +598,18 @@ attention_rows_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __rest
     }
 }
 
-template <int D, int DV>
+constexpr int kDeep = 5;
+constexpr int rows_smem(int d, int dv, int stages) { return stages * KT * (d * 2 + 16 + dv * 2 + 16) + 4 * 16 * (dv + 2) * 4; }
+// Whether as many blocks of kDeep stages run at once: 16 rows of 8 kv heads of 64, values of 128, behind 300 keys 9.5 us, 14.8 with two.
+bool deep_fits(int64_t blocks, int d, int dv) { return blocks <= 148 * (int64_t)(227 * 1024 / (rows_smem(d, dv, kDeep) + 1024)); }
+
+template <int D, int DV, int STAGES>
 int launch_rows(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache, const int* positions,
                 const int* seq_of_row, const int* block_table, int bt_stride, int rows, int heads, int kv_heads,
                 int page_size, int mask_kind, int mask_size, float scale, int keys_per_value, int out_f32, Extras x,
                 cudaStream_t stream) {
-    constexpr int smem = 2 * KT * (D * 2 + 16 + DV * 2 + 16) + 4 * 16 * (DV + 2) * 4;
-    auto kernel = x.bias_weight != nullptr ? attention_rows_kernel<D, DV, true> : attention_rows_kernel<D, DV, false>;
+    constexpr int smem = rows_smem(D, DV, STAGES);
+    auto kernel = x.bias_weight != nullptr ? attention_rows_kernel<D, DV, true, STAGES> : attention_rows_kernel<D, DV, false, STAGES>;
     if (smem > 40 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) return (int)err;
@@ -696,8 +727,9 @@ TB_EXPORT int tb_attention_rows_mma(const void* q, int64_t q_stride, void* out, 
     if (mask_kind != MASK_CAUSAL && mask_size < 1) return TB_ERR_BAD_SIZE;
     if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)cache) % 16 != 0 || q_stride % 2 != 0) return TB_ERR_BAD_ALIGN;
 #define TB_ROWS(D, DV)                                                                                              \
-    return launch_rows<D, DV>(q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride,   \
-                              rows, heads, kv_heads, page_size, mask_kind, mask_size, scale, keys_per_value, out_f32, x, stream)
+    return (deep_fits((int64_t)rows * kv_heads, D, DV) ? launch_rows<D, DV, kDeep> : launch_rows<D, DV, 2>)(         \
+        q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride, rows, heads, kv_heads,   \
+        page_size, mask_kind, mask_size, scale, keys_per_value, out_f32, x, stream)
     if (dim == 64 && vdim == 48) TB_ROWS(64, 48);
     if (dim == 64 && vdim == 64) TB_ROWS(64, 64);
     if (dim == 64 && vdim == 128) TB_ROWS(64, 128);

@@ -147,6 +147,33 @@ def test_a_product_that_gates_by_token_stores_what_the_kernel_behind_it_would(ro
         kernels.decode_linear_token_gate(x, weight, tokens, table, offset + 4, torch.empty_like(want), 0)
 
 
+@pytest.mark.parametrize("dim, vdim, per_value", [(64, 48, 1), (64, 64, 1), (64, 128, 2), (128, 64, 1), (128, 128, 1)])
+@pytest.mark.parametrize("mask, size", [(0, 1), (1, 100), (2, 64)])
+def test_attention_rows_mma_gives_few_rows_the_bits_of_many(dim, vdim, per_value, mask, size):
+    """Blocks that hold five tiles of keys and those that hold two, for rows that see one key up to ten tiles."""
+    from tesseract_b200 import kernels
+
+    kv, heads, page, rows = 8, 16, 16, 320
+    g = torch.Generator().manual_seed(dim + vdim + mask)
+    last = [0, 63, 64, 127, 128, 255, 256, 319, 320, 639]
+    positions = torch.tensor([last[i % 10] for i in range(rows)], dtype=torch.int32)
+    table = (torch.randperm(40 * 10, generator=g) + 1).to(torch.int32).view(10, 40)
+    cache = torch.randn(401, kv * page * dim + kv // per_value * page * vdim, generator=g).bfloat16()
+    q = torch.randn(rows, heads * dim, generator=g).bfloat16()
+    cache, table, seq = dev(cache), dev(table), torch.arange(rows, dtype=torch.int32) % 10
+
+    def run(lo, hi):
+        out = torch.empty(hi - lo, heads * vdim, device="cuda")
+        kernels.attention_rows_mma(dev(q[lo:hi]), out, cache, dev(positions[lo:hi]), dev(seq[lo:hi]), table, heads=heads, kv_heads=kv, dim=dim,
+                                   vdim=vdim, page_size=page, mask_kind=mask, mask_size=size, scale=dim ** -0.5, keys_per_value=per_value)
+        return out
+
+    many = run(0, rows)
+    assert torch.isfinite(many).all()
+    for lo, hi in ((0, 10), (9, 10), (100, 118)):
+        assert torch.equal(run(lo, hi), many[lo:hi])
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 1, 1), (3, 5, 7), (64, 64, 16), (65, 130, 33), (200, 96, 96), (17, 331, 72),
                                      (2, 1000, 2048)])
 def test_gemm_f32(m, n, k):
