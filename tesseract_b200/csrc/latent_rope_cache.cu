@@ -14,32 +14,51 @@
 
 namespace {
 
+// Bound by the chain of a launch in steps of few rows: there the first of gridDim.y blocks of a row takes the latent and the shared
+// part, the others the heads' parts, and where the row goes and a thread's first sines are found before the wait.  8 rows of 16 heads,
+// 512 + 64 numbers: 2.3 us, 3.7 before.  (The rows are not __restrict__: their loads stay behind the wait.)
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_rope_cache_kernel(const float* __restrict__ down, int64_t down_stride, const T* __restrict__ q,
-                         int64_t q_stride, T* __restrict__ q_full, int64_t full_stride, T* __restrict__ cache,
+latent_rope_cache_kernel(const float* down, int64_t down_stride, const T* q, int64_t q_stride, T* q_full, int64_t full_stride, T* cache,
                          const float* __restrict__ weight, const int* __restrict__ positions,
                          const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride,
                          const float* __restrict__ inv_freq, int heads, int dim, int rank, int rot_width, int rot_dims,
                          int page_size, float eps, float amplitude) {
     __shared__ float scratch[32];
     pdl_trigger();
-    pdl_wait();
     const int row = blockIdx.x;
     const int pos = positions[row];
     const int seq = seq_of_row[row];
     const int64_t page = block_table[(int64_t)seq * bt_stride + pos / page_size];
+    const int half = (rot_width + 1) / 2;
+    // slot 0 .. half-1 of "head" -1 is the shared key part, then the heads' query parts
+    const bool alone = gridDim.y == 1;
+    const int slots = alone || blockIdx.y > 0 ? (heads + 1) * half : half;
+    const int at = alone || blockIdx.y == 0 ? threadIdx.x : half + (blockIdx.y - 1) * blockDim.x + threadIdx.x;
+    const int step = alone || blockIdx.y == 0 ? blockDim.x : (gridDim.y - 1) * blockDim.x;
+    float sn = 0.0f, cs = 1.0f;
+    int turned = -1;
+    auto turn = [&](int i) {
+        if (i != turned) {
+            sincosf((float)pos * inv_freq[i], &sn, &cs);
+            sn *= amplitude;
+            cs *= amplitude;
+        }
+        turned = i;
+    };
+    if (at < slots && 2 * (at % half) + 1 < rot_dims) turn(at % half);
+    pdl_wait();
     const int width = rank + rot_width;
     T* entry = cache + (page * page_size + pos % page_size) * width;
     const float* drow = down + (int64_t)row * down_stride;
-    float ss = 0.0f;
-    for (int j = threadIdx.x; j < rank; j += blockDim.x) ss = fmaf(drow[j], drow[j], ss);
-    ss = block_sum(ss, scratch);
-    const float inv = 1.0f / sqrtf(ss / (float)rank + eps);
-    for (int j = threadIdx.x; j < rank; j += blockDim.x) Elem<T>::store(entry + j, drow[j] * inv * weight[j]);
-    // slot 0 .. half-1 of "head" -1 is the shared key part, then the heads' query parts
-    const int half = (rot_width + 1) / 2;
-    for (int e = threadIdx.x; e < (heads + 1) * half; e += blockDim.x) {
+    if (blockIdx.y == 0) {
+        float ss = 0.0f;
+        for (int j = threadIdx.x; j < rank; j += blockDim.x) ss = fmaf(drow[j], drow[j], ss);
+        ss = block_sum(ss, scratch);
+        const float inv = 1.0f / sqrtf(ss / (float)rank + eps);
+        for (int j = threadIdx.x; j < rank; j += blockDim.x) Elem<T>::store(entry + j, drow[j] * inv * weight[j]);
+    }
+    for (int e = at; e < slots; e += step) {
         const int head = e / half - 1, i = e % half;
         const int c = 2 * i;
         float u, v = 0.0f;
@@ -59,12 +78,9 @@ latent_rope_cache_kernel(const float* __restrict__ down, int64_t down_stride, co
             continue;
         }
         if (c + 1 < rot_dims) {
-            float sn, cs;
-            sincosf((float)pos * inv_freq[i], &sn, &cs);
-            sn *= amplitude;
-            cs *= amplitude;
-            Elem<T>::store(to, u * cs - v * sn);
-            Elem<T>::store(to + 1, v * cs + u * sn);
+            turn(i);
+            Elem<T>::store(to, fmaf(u, cs, -(v * sn)));      // (the products' roundings spelled out: they do not depend on the code around)
+            Elem<T>::store(to + 1, fmaf(v, cs, u * sn));
         } else {
             Elem<T>::store(to, u);
             Elem<T>::store(to + 1, v);
@@ -84,14 +100,16 @@ TB_EXPORT int tb_latent_rope_cache(const float* down, int64_t down_stride, const
     if (rows == 0) return 0;
     if (heads < 1 || dim < 0 || rank < 1 || rot_width < 0 || page_size < 1) return TB_ERR_BAD_SIZE;
     if (rot_dims < 0 || rot_dims % 2 || rot_dims > rot_width || (rot_dims > 0 && inv_freq == nullptr)) return TB_ERR_BAD_SIZE;
+    const int pairs = heads * ((rot_width + 1) / 2);
+    const dim3 grid(rows, rows <= 148 && pairs > 0 ? 1 + (pairs < 4 * 256 ? (pairs + 255) / 256 : 4) : 1);
     cudaError_t launched;
     if (dtype == TB_F32)
-        launched = tb_launch_pdl(latent_rope_cache_kernel<float>, dim3(rows), dim3(256), 0, stream, down, down_stride,
+        launched = tb_launch_pdl(latent_rope_cache_kernel<float>, grid, dim3(256), 0, stream, down, down_stride,
                                  (const float*)q, q_stride, (float*)q_full, full_stride, (float*)cache, weight, positions,
                                  seq_of_row, block_table, bt_stride, inv_freq, heads, dim, rank, rot_width, rot_dims,
                                  page_size, eps, amplitude);
     else if (dtype == TB_BF16)
-        launched = tb_launch_pdl(latent_rope_cache_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, down,
+        launched = tb_launch_pdl(latent_rope_cache_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, down,
                                  down_stride, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)q_full, full_stride,
                                  (__nv_bfloat16*)cache, weight, positions, seq_of_row, block_table, bt_stride, inv_freq,
                                  heads, dim, rank, rot_width, rot_dims, page_size, eps, amplitude);

@@ -147,6 +147,39 @@ def test_a_product_that_gates_by_token_stores_what_the_kernel_behind_it_would(ro
         kernels.decode_linear_token_gate(x, weight, tokens, table, offset + 4, torch.empty_like(want), 0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("q_heads, key_heads, value_heads, dim, vdim, rot, rank", [(32, 8, 4, 64, 128, 64, 512), (5, 3, 1, 33, 7, 16, 40), (64, 64, 64, 128, 64, 128, 16)])
+def test_rotations_give_few_rows_the_bits_of_many(dtype, q_heads, key_heads, value_heads, dim, vdim, rot, rank):
+    """Several blocks a row up to 148 rows, one beyond: pair rotation and the latent's, whole heads and cut ones."""
+    from tesseract_b200 import kernels
+
+    rows, page = 150, 8
+    g = torch.Generator().manual_seed(dim)
+    positions = torch.randint(0, 3 * page, (rows,), generator=g, dtype=torch.int32)
+    table = dev((torch.randperm(3 * rows, generator=g) + 1).to(torch.int32).view(rows, 3))
+    proj = torch.randn(rows, (q_heads + key_heads) * dim + value_heads * vdim, generator=g).to(dtype)
+    down, q = torch.randn(rows, rank + dim, generator=g), torch.randn(rows, q_heads * (4 + dim), generator=g).to(dtype)
+    inv_freq, weight = dev(torch.rand(rot // 2, generator=g)), dev(torch.randn(rank, generator=g))
+
+    def run(hi):
+        pages = 3 * rows + 1
+        q_out, cache = torch.zeros(hi, q_heads * dim, dtype=dtype, device="cuda"), torch.zeros(pages, page * (key_heads * dim + value_heads * vdim), dtype=dtype, device="cuda")
+        full, latent = torch.zeros(hi, q_heads * (rank + dim), dtype=dtype, device="cuda"), torch.zeros(pages, page * (rank + dim), dtype=dtype, device="cuda")
+        place = (dev(positions[:hi]), dev(torch.arange(hi, dtype=torch.int32)), table[:hi])
+        kernels.pair_rope_cache(dev(proj[:hi]), q_out, cache, *place, inv_freq, q_heads=q_heads, key_heads=key_heads, value_heads=value_heads,
+                                dim=dim, vdim=vdim, rot_dims=rot, page_size=page)
+        kernels.latent_rope_cache(dev(down[:hi]), dev(q[:hi]), full, latent, weight, *place, inv_freq, heads=q_heads, dim=4, rank=rank,
+                                  rot_width=dim, rot_dims=rot, page_size=page, eps=1e-5, amplitude=1.3)
+        own = table[:hi].flatten().long()
+        return q_out, cache[own], full, latent[own]
+
+    many = run(rows)
+    for hi in (1, 148):
+        few = run(hi)
+        assert all(torch.equal(one, two[:one.shape[0]]) for one, two in zip(few, many))
+        assert all(one.float().abs().sum() > 0 for one in few)
+
+
 @pytest.mark.parametrize("dim, vdim, per_value", [(64, 48, 1), (64, 64, 1), (64, 128, 2), (128, 64, 1), (128, 128, 1)])
 @pytest.mark.parametrize("mask, size", [(0, 1), (1, 100), (2, 64)])
 def test_attention_rows_mma_gives_few_rows_the_bits_of_many(dim, vdim, per_value, mask, size):
