@@ -304,8 +304,8 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
     attention_rows_kernel<T, NC, UNDER><<<grid, kWarpsPerBlock * 32, smem, stream>>>(                                 \
         (const T*)q, q_stride, (T*)out, out_stride, (const T*)cache, positions, seq_of_row, block_table,       \
         bt_stride, num_heads, num_kv_heads, head_dim, page_size, window, scale)
-    // Few warps a multiprocessor (decoded rows) are bound by the latency of their loads, and more under way shorten it: 4 rows of 32
-    // heads of 64 behind some 100 keys take 13.4 us in 32-bit with 32 under way, 30.7 as they are needed.  The registers that this
+    // Few warps a multiprocessor are bound by the latency of their loads, and more under way shorten it: 4 rows of 32 heads of 64 behind
+    // some 100 keys (which the blocks above take by now) 13.4 us in 32-bit with 32 under way, 30.7 as they are needed.  The registers that this
     // takes hold back other warps as soon as there are more: 64 rows of 32 heads of 128 behind 300 keys, 32-bit, 8 / 16 under way or
     // as needed 140 / 288 / 251.  So 592 blocks, four a multiprocessor, take the form that was the fastest or close to it over all
     // of them (32-bit: 0.4 to 0.8 of the time as needed, bfloat16 0.65 to 0.9), and steps that fill the chip take few or none:
