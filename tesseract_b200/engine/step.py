@@ -102,7 +102,9 @@ class Stepper:
             if count == 0:
                 raise StepError(f"request {entry.request!r} brings no tokens")
             ids = entry.tokens
-            if count == 1 and type(ids[0]) is int:          # (a decoded row: an array would cost more than the check)
+            # (a decoded row: an array would cost more than the check.  Lists and tuples alone: bytes and a dict can be indexed too,
+            # a set cannot, and all three are refused below)
+            if count == 1 and type(ids) in (list, tuple) and type(ids[0]) is int:
                 low = high = ids[0]
             else:
                 ids = np.asarray(ids)
