@@ -1231,7 +1231,7 @@ def kazodra_kernels(size, pk):
             cache = torch.zeros(seqs * pages_per_seq + 1, page_elems, dtype=torch.bfloat16, device=dev)
             return lambda: kernels.pair_rope_cache(proj, q, cache, positions, seq_of_row, table, pair_freq, q_heads=2 * H,
                                                    key_heads=2 * G, value_heads=G, dim=d, vdim=dv, rot_dims=d,
-                                                   page_size=page)
+                                                   page_size=page, indices_copied=True)
 
         timed(f"pair_rope_cache/{label}", rotate, rows * channels * 2 * 2)
 
@@ -1259,7 +1259,7 @@ def kazodra_kernels(size, pk):
             if new > 1:
                 return lambda: kernels.attention_prompt_mma(q, maps, cache, positions, row_start, table, num_seqs=seqs,
                                                             **common)
-            return lambda: kernels.attention_rows_mma(q, maps, cache, positions, seq_of_row, table, **common)
+            return lambda: kernels.attention_rows_mma(q, maps, cache, positions, seq_of_row, table, **common, indices_copied=True)
 
         if kernels.attention_prompt_mma_supported(torch.bfloat16, d, dv):
             timed(f"{'attention_prompt_mma' if new > 1 else 'attention_rows_mma'} (two maps, causal)/{label}", two_maps_mma,
@@ -1282,7 +1282,7 @@ def kazodra_kernels(size, pk):
             cache = torch.zeros(seqs * pages_per_seq + 1, page * entry, dtype=torch.bfloat16, device=dev)
             return lambda: kernels.latent_rope_cache(down, q, q_full, cache, w, positions, seq_of_row, table, rot_freq,
                                                      heads=LH, dim=ld, rank=rank, rot_width=rot, rot_dims=rot,
-                                                     page_size=page, eps=1e-5)
+                                                     page_size=page, eps=1e-5, indices_copied=True)
 
         timed(f"latent_rope_cache/{label}", latent_write, rows * (entry * (4 + 2) + LH * rot * 2 * 2))
 
@@ -1308,7 +1308,7 @@ def kazodra_kernels(size, pk):
             return lambda: kernels.attention_latent_mma(q_full, mixed, cache, positions, seq_of_row, table, heads=LH,
                                                         dim=entry, vdim=rank, page_size=page,
                                                         mask_kind=kernels.MASK_WINDOW, mask_size=window,
-                                                        scale=(ld + rot) ** -0.5)
+                                                        scale=(ld + rot) ** -0.5, indices_copied=True)
 
         if kernels.attention_latent_mma_supported(torch.bfloat16, entry, rank):
             timed(f"attention_latent_mma (window {window})/{label}", latent_attend_mma,
@@ -1435,7 +1435,7 @@ def ladedra_kernels(size, pk):
                 if kernel == "attention_prompt_mma":
                     return lambda: kernels.attention_prompt_mma(q, o, cache, positions, row_start, table, num_seqs=seqs, **common)
                 if kernel == "attention_rows_mma":
-                    return lambda: kernels.attention_rows_mma(q, o, cache, positions, seq_of_row, table, **common)
+                    return lambda: kernels.attention_rows_mma(q, o, cache, positions, seq_of_row, table, **common, indices_copied=True)
                 return lambda: kernels.attention_masked(q, None, o, cache, positions, seq_of_row, table, sink=False, **common)
             return make
 
@@ -1486,7 +1486,7 @@ def ladedra_kernels(size, pk):
             cache = torch.zeros(seqs * pages_per_seq + 1, page * entry, dtype=torch.bfloat16, device=dev)
             return lambda: kernels.latent_rope_cache(down, q, q_full, cache, w, positions, seq_of_row, table, pair_freq,
                                                      heads=LH, dim=ld, rank=rank, rot_width=rot, rot_dims=rot,
-                                                     page_size=page, eps=1e-5, amplitude=amplitude)
+                                                     page_size=page, eps=1e-5, amplitude=amplitude, indices_copied=True)
 
         timed(f"latent_rope_cache/{label}", latent_write, rows * (entry * (4 + 2) + LH * rot * 2 * 2))
 
@@ -1499,7 +1499,7 @@ def ladedra_kernels(size, pk):
             cache = torch.randn(seqs * pages_per_seq + 1, page * entry, device=dev).bfloat16()
             return lambda: kernels.attention_latent_mma(q_full, mixed, cache, positions, seq_of_row, table, heads=LH,
                                                         dim=entry, vdim=rank, page_size=page, mask_kind=kernels.MASK_CAUSAL,
-                                                        mask_size=0, scale=(ld + rot) ** -0.5)
+                                                        mask_size=0, scale=(ld + rot) ** -0.5, indices_copied=True)
 
         if kernels.attention_latent_mma_supported(torch.bfloat16, entry, rank):
             timed(f"attention_latent_mma (causal)/{label}", latent_attend, rows * LH * (entry + rank) * 2 + latent_read,
@@ -1630,7 +1630,7 @@ def rirulix_kernels(size, pk):
                 if kernel == "prompt":
                     return lambda: kernels.attention_prompt_mma(q, y, cache, positions, row_start, table, num_seqs=seqs, **common)
                 if kernel == "rows":
-                    return lambda: kernels.attention_rows_mma(q, y, cache, positions, seq_of_row, table, **common)
+                    return lambda: kernels.attention_rows_mma(q, y, cache, positions, seq_of_row, table, **common, indices_copied=True)
                 return lambda: kernels.attention_masked(q, None, y, cache, positions, seq_of_row, table, sink=False, **common)
             return make
 
@@ -1829,7 +1829,7 @@ def tibivik_kernels(size, pk):
                               **extras(k))
                 if kernel == "prompt":
                     return lambda: kernels.attention_prompt_mma(q, y, cache, positions, row_start, table, num_seqs=seqs, **common)
-                return lambda: kernels.attention_rows_mma(q, y, cache, positions, seq_of_row, table, **common)
+                return lambda: kernels.attention_rows_mma(q, y, cache, positions, seq_of_row, table, **common, indices_copied=True)
             return make
 
         kind = "prompt" if rows > 256 else "rows"
@@ -2037,7 +2037,7 @@ def pekodra_kernels(size, pk):
                 cache = torch.randn(seqs * pages_per_seq + 1, page_elems, device=dev).bfloat16()
                 return lambda: kernels.attention_rows_mma(q, o, cache, positions, seq_of_row, table, heads=H, kv_heads=G,
                                                           dim=d, vdim=d, page_size=page, mask_kind=kernels.MASK_WINDOW,
-                                                          mask_size=window, scale=d ** -0.5)
+                                                          mask_size=window, scale=d ** -0.5, indices_copied=True)
 
             timed(f"attention_rows_mma (window {window})/{label}", attend_rows, rows * H * d * 2 * 2 + kv_read,
                   flops=keys_seen * H * 2 * d * 2)

@@ -114,7 +114,7 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
     };
     int pages[KT / 8];
     look(tile_first, pages);
-    pdl_wait();                                                   // queries and the step's keys come from kernels in front, its metadata does not
+    pdl_wait();                                                   // queries and the step's keys come from kernels in front (its metadata does not: see `early` below)
     // the sixteen heads' queries (heads the model does not have are rows of zeros)
     for (int index = tid; index < 16 * (D / 8); index += 128) {
         const int h = index / (D / 8), chunk = index % (D / 8);
@@ -536,7 +536,7 @@ int splits_for(int rows, int heads) {
 template <int D, int DV>
 int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache, const int* positions,
            const int* seq_of_row, const int* block_table, int bt_stride, int rows, int num_seqs, int heads, int page_size, int mask_kind,
-           int mask_size, float scale, float* parts, cudaStream_t stream) {
+           int mask_size, float scale, float* parts, int early, cudaStream_t stream) {
     constexpr int smem = Layout<D, DV>::BYTES;
     auto kernel = attention_latent_kernel<D, DV>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -560,7 +560,7 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
     }
     if (splits > 1 && parts == nullptr) return TB_ERR_BAD_SIZE;
     if (splits > 1 && (uintptr_t)parts % 8 != 0) return TB_ERR_BAD_ALIGN;
-    cudaError_t launched = tb_launch_pdl(kernel, dim3(rows, (heads + 15) / 16, splits), dim3(128), (size_t)smem, stream,
+    cudaError_t launched = tb_launch(early, kernel, dim3(rows, (heads + 15) / 16, splits), dim3(128), (size_t)smem, stream,
                                          (const bf16*)q, q_stride, (bf16*)out, out_stride, (const bf16*)cache, positions,
                                          seq_of_row, block_table, bt_stride, heads, page_size, mask_kind, mask_size, scale,
                                          splits > 1 ? parts : (float*)nullptr);
@@ -588,11 +588,13 @@ TB_EXPORT int tb_attention_latent_mma_splits(int rows, int heads) {
 // q: bfloat16 [rows, heads * dim] (row stride q_stride, elements); out: bfloat16 [rows, heads * vdim]; cache: this
 // layer's pages ([page_size][dim] a page); positions, seq_of_row: int32 [rows]; num_seqs: the sequences that the
 // rows belong to (it picks the kernel only); mask_kind: 0 causal, 1 window; parts:
-// float32 [rows, splits, heads, vdim + 2] of scratch where tb_attention_latent_mma_splits says more than 1.
+// float32 [rows, splits, heads, vdim + 2] of scratch where tb_attention_latent_mma_splits says more than 1; early: no
+// kernel that may still run when this one's turn comes writes positions, seq_of_row or block_table (copies do not count);
+// the kernel then begins beside the one in front, else behind it.
 TB_EXPORT int tb_attention_latent_mma(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
                                       const int* positions, const int* seq_of_row, const int* block_table, int bt_stride,
                                       int rows, int num_seqs, int heads, int dim, int vdim, int page_size, int mask_kind,
-                                      int mask_size, float scale, float* parts, cudaStream_t stream) {
+                                      int mask_size, float scale, float* parts, int early, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (!tb_attention_latent_mma_supported(dim, vdim)) return TB_ERR_BAD_SIZE;
     if (heads < 1 || (heads + 15) / 16 > 65535 || page_size < 1) return TB_ERR_BAD_SIZE;
@@ -602,7 +604,7 @@ TB_EXPORT int tb_attention_latent_mma(const void* q, int64_t q_stride, void* out
         return TB_ERR_BAD_ALIGN;
 #define TB_ATTEND(D, DV)                                                                                             \
     return launch<D, DV>(q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride, rows,   \
-                         num_seqs, heads, page_size, mask_kind, mask_size, scale, parts, stream)
+                         num_seqs, heads, page_size, mask_kind, mask_size, scale, parts, early, stream)
     if (dim == 576) TB_ATTEND(576, 512);
     if (dim == 288) TB_ATTEND(288, 256);
     TB_ATTEND(160, 128);

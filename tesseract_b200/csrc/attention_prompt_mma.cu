@@ -387,7 +387,8 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
 // share every tile of 64 keys, 16 keys a warp, each with a streaming softmax of its own, and their partial results
 // (maximum, sum, accumulator) meet in shared memory in warp order.
 // STAGES: tiles in shared memory.  Where every block has room for kDeep of them they are asked for that far ahead, with one barrier a
-// tile; the first tiles' pages are looked up before the wait (the step's metadata comes from no kernel), the others' a tile ahead.
+// tile; the first tiles' pages are looked up before the wait (launched early only where no kernel may still write them), the others' a tile
+// ahead.
 // (The queries are not __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
 template <int D, int DV, bool BIASED, int STAGES>
 __global__ void __launch_bounds__(128)
@@ -607,14 +608,14 @@ template <int D, int DV, int STAGES>
 int launch_rows(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache, const int* positions,
                 const int* seq_of_row, const int* block_table, int bt_stride, int rows, int heads, int kv_heads,
                 int page_size, int mask_kind, int mask_size, float scale, int keys_per_value, int out_f32, Extras x,
-                cudaStream_t stream) {
+                int early, cudaStream_t stream) {
     constexpr int smem = rows_smem(D, DV, STAGES);
     auto kernel = x.bias_weight != nullptr ? attention_rows_kernel<D, DV, true, STAGES> : attention_rows_kernel<D, DV, false, STAGES>;
     if (smem > 40 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) return (int)err;
     }
-    cudaError_t launched = tb_launch_pdl(kernel, dim3(rows, kv_heads), dim3(128), (size_t)smem, stream, (const bf16*)q,
+    cudaError_t launched = tb_launch(early, kernel, dim3(rows, kv_heads), dim3(128), (size_t)smem, stream, (const bf16*)q,
                                          q_stride, (bf16*)out, out_stride, (const bf16*)cache, positions, seq_of_row,
                                          block_table, bt_stride, heads, kv_heads, page_size, mask_kind, mask_size, scale,
                                          keys_per_value, out_f32, x);
@@ -700,14 +701,15 @@ TB_EXPORT int tb_attention_prompt_mma(const void* q, int64_t q_stride, void* out
 }
 
 // The same attention for steps of few rows: one block a (row, kv head), any positions.  At most 16 query heads a kv
-// head; seq_of_row: int32 [rows].
+// head; seq_of_row: int32 [rows].  early: no kernel that may still run when this one's turn comes writes positions, seq_of_row,
+// block_table or pool_table (copies do not count); the kernel then begins beside the one in front, else behind it.
 TB_EXPORT int tb_attention_rows_mma(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
                                     const int* positions, const int* seq_of_row, const int* block_table, int bt_stride,
                                     int rows, int heads, int kv_heads, int dim, int vdim, int page_size, int mask_kind,
                                     int mask_size, float scale, int keys_per_value, int out_f32, const float* sinks,
                                     float softcap, const void* pool_cache, const int* pool_table, int pool_bt_stride,
                                     int pool, int keep_first, const float* bias_weight, const float* bias_rate,
-                                    const void* head_gate, int64_t head_gate_stride, cudaStream_t stream) {
+                                    const void* head_gate, int64_t head_gate_stride, int early, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (!extras_fit(mask_kind, keep_first, bias_weight, bias_rate)) return TB_ERR_BAD_SIZE;
     if (mask_kind == MASK_WINDOW_POOLED && (pool < 1 || pool_cache == nullptr || pool_table == nullptr || keys_per_value != 1 ||
@@ -729,7 +731,7 @@ TB_EXPORT int tb_attention_rows_mma(const void* q, int64_t q_stride, void* out, 
 #define TB_ROWS(D, DV)                                                                                              \
     return (deep_fits((int64_t)rows * kv_heads, D, DV) ? launch_rows<D, DV, kDeep> : launch_rows<D, DV, 2>)(         \
         q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride, rows, heads, kv_heads,   \
-        page_size, mask_kind, mask_size, scale, keys_per_value, out_f32, x, stream)
+        page_size, mask_kind, mask_size, scale, keys_per_value, out_f32, x, early, stream)
     if (dim == 64 && vdim == 48) TB_ROWS(64, 48);
     if (dim == 64 && vdim == 64) TB_ROWS(64, 64);
     if (dim == 64 && vdim == 128) TB_ROWS(64, 128);

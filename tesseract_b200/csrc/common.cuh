@@ -22,13 +22,14 @@ enum TbDtype : int { TB_F32 = 0, TB_BF16 = 1 };
 // Programmatic dependent launch.  A kernel started with tb_launch_pdl may begin while the kernel before it in
 // the stream is still draining; everything it does before pdl_wait() must not depend on that kernel's results
 // (reading weights is fine).  pdl_trigger() in a kernel lets the next such kernel start early.  Both are no-ops
-// for kernels launched the ordinary way.
+// for kernels launched the ordinary way.  A kernel that reads more than weights before pdl_wait() (where a row lies: positions,
+// block tables) is started with tb_launch, early only if its caller vouches that no kernel in front may still be writing that.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KernelArgs, typename... Args>
-static inline cudaError_t tb_launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem,
-                                        cudaStream_t stream, Args... args) {
+static inline cudaError_t tb_launch(bool early, void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -38,8 +39,14 @@ static inline cudaError_t tb_launch_pdl(void (*kernel)(KernelArgs...), dim3 grid
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
-    config.numAttrs = 1;
+    config.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&config, kernel, KernelArgs(args)...);
+}
+
+template <typename... KernelArgs, typename... Args>
+static inline cudaError_t tb_launch_pdl(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t stream, Args... args) {
+    return tb_launch(true, kernel, grid, block, smem, stream, args...);
 }
 
 static inline int tb_launch_status() {

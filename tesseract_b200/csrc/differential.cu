@@ -104,11 +104,13 @@ differential_combine_kernel(const float* __restrict__ maps, const T* __restrict_
 
 }  // namespace
 
-// proj: [rows, q_heads * dim | key_heads * dim | value_heads * vdim | ...] (row stride proj_stride, elements).
+// proj: [rows, q_heads * dim | key_heads * dim | value_heads * vdim | ...] (row stride proj_stride, elements).  early: no kernel that
+// may still run when this one's turn comes writes positions, seq_of_row or block_table (copies do not count); the kernel then begins
+// beside the one in front, else behind it.
 TB_EXPORT int tb_pair_rope_cache(const void* proj, int64_t proj_stride, void* q_out, int64_t q_stride, void* cache,
                                  const int* positions, const int* seq_of_row, const int* block_table, int bt_stride,
                                  const float* inv_freq, int rows, int q_heads, int key_heads, int value_heads, int dim,
-                                 int vdim, int rot_dims, int page_size, int dtype, cudaStream_t stream) {
+                                 int vdim, int rot_dims, int page_size, int dtype, int early, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (q_heads < 1 || key_heads < 1 || value_heads < 1 || dim < 1 || vdim < 1 || page_size < 1) return TB_ERR_BAD_SIZE;
     if (rot_dims < 0 || rot_dims % 2 || rot_dims > dim || (rot_dims > 0 && inv_freq == nullptr)) return TB_ERR_BAD_SIZE;
@@ -116,11 +118,11 @@ TB_EXPORT int tb_pair_rope_cache(const void* proj, int64_t proj_stride, void* q_
     const dim3 grid(rows, rows <= 148 && pairs > 256 ? (pairs < 8 * 256 ? (pairs + 255) / 256 : 8) : 1);
     cudaError_t launched;
     if (dtype == TB_F32)
-        launched = tb_launch_pdl(pair_rope_cache_kernel<float>, grid, dim3(256), 0, stream, (const float*)proj,
+        launched = tb_launch(early, pair_rope_cache_kernel<float>, grid, dim3(256), 0, stream, (const float*)proj,
                                  proj_stride, (float*)q_out, q_stride, (float*)cache, positions, seq_of_row, block_table,
                                  bt_stride, inv_freq, q_heads, key_heads, value_heads, dim, vdim, rot_dims, page_size);
     else if (dtype == TB_BF16)
-        launched = tb_launch_pdl(pair_rope_cache_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream,
+        launched = tb_launch(early, pair_rope_cache_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream,
                                  (const __nv_bfloat16*)proj, proj_stride, (__nv_bfloat16*)q_out, q_stride,
                                  (__nv_bfloat16*)cache, positions, seq_of_row, block_table, bt_stride, inv_freq, q_heads,
                                  key_heads, value_heads, dim, vdim, rot_dims, page_size);

@@ -91,12 +91,14 @@ latent_rope_cache_kernel(const float* down, int64_t down_stride, const T* q, int
 }  // namespace
 
 // down: float32 [rows, rank + rot_width]; q: [rows, heads * (dim + rot_width)]; q_full: [rows, heads * (rank + rot_width)]
-// (only the rotated parts are written); cache: pages of [page_size][rank + rot_width]; weight: float32 [rank].
+// (only the rotated parts are written); cache: pages of [page_size][rank + rot_width]; weight: float32 [rank].  early: no kernel
+// that may still run when this one's turn comes writes positions, seq_of_row or block_table (copies do not count); the kernel then
+// begins beside the one in front, else behind it.
 TB_EXPORT int tb_latent_rope_cache(const float* down, int64_t down_stride, const void* q, int64_t q_stride, void* q_full,
                                    int64_t full_stride, void* cache, const float* weight, const int* positions,
                                    const int* seq_of_row, const int* block_table, int bt_stride, const float* inv_freq,
                                    int rows, int heads, int dim, int rank, int rot_width, int rot_dims, int page_size,
-                                   float eps, float amplitude, int dtype, cudaStream_t stream) {
+                                   float eps, float amplitude, int dtype, int early, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (heads < 1 || dim < 0 || rank < 1 || rot_width < 0 || page_size < 1) return TB_ERR_BAD_SIZE;
     if (rot_dims < 0 || rot_dims % 2 || rot_dims > rot_width || (rot_dims > 0 && inv_freq == nullptr)) return TB_ERR_BAD_SIZE;
@@ -104,12 +106,12 @@ TB_EXPORT int tb_latent_rope_cache(const float* down, int64_t down_stride, const
     const dim3 grid(rows, rows <= 148 && pairs > 0 ? 1 + (pairs < 4 * 256 ? (pairs + 255) / 256 : 4) : 1);
     cudaError_t launched;
     if (dtype == TB_F32)
-        launched = tb_launch_pdl(latent_rope_cache_kernel<float>, grid, dim3(256), 0, stream, down, down_stride,
+        launched = tb_launch(early, latent_rope_cache_kernel<float>, grid, dim3(256), 0, stream, down, down_stride,
                                  (const float*)q, q_stride, (float*)q_full, full_stride, (float*)cache, weight, positions,
                                  seq_of_row, block_table, bt_stride, inv_freq, heads, dim, rank, rot_width, rot_dims,
                                  page_size, eps, amplitude);
     else if (dtype == TB_BF16)
-        launched = tb_launch_pdl(latent_rope_cache_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, down,
+        launched = tb_launch(early, latent_rope_cache_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, down,
                                  down_stride, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)q_full, full_stride,
                                  (__nv_bfloat16*)cache, weight, positions, seq_of_row, block_table, bt_stride, inv_freq,
                                  heads, dim, rank, rot_width, rot_dims, page_size, eps, amplitude);

@@ -104,7 +104,7 @@ class _Graph:
             num_rows=batch, num_seqs=batch, token_ids=self.tokens, positions=self.d["positions"],
             seq_of_row=arange[:batch], row_start=arange, seq_begin=self.d["positions"], state_slots=self.d["slots"],
             groups=groups, host_new=[1] * batch, host_begin=(), host_slots=(), max_new=1,
-            max_context=columns * cache.page_size)
+            max_context=columns * cache.page_size, indices_copied=True)
         self.want_rows = arange[:batch]
         self.logits: Optional[torch.Tensor] = None
         self.graph: Optional[torch.cuda.CUDAGraph] = None
@@ -334,7 +334,7 @@ class _ChunkGraph:
             row_start=row_start, seq_begin=d[2 * total:2 * total + seqs],
             state_slots=d[2 * total + seqs:2 * total + 2 * seqs], groups=groups,
             host_new=host_new, host_begin=(), host_slots=(), max_new=max(rows if portions else 0, tail),
-            max_context=columns * cache.page_size)
+            max_context=columns * cache.page_size, indices_copied=True)
         # capture on harmless metadata: positions 0.., the scratch slot, the scratch page; a tail of all rows but one
         host = self.hosts[0].numpy()
         host[total:total + portions * rows] = np.tile(np.arange(rows, dtype=np.int32), portions)

@@ -158,7 +158,8 @@ class Stepper:
         ctx = StepContext(
             num_rows=num_rows, num_seqs=num_seqs, token_ids=device[0], positions=device[1], seq_of_row=device[2],
             row_start=device[3], seq_begin=device[4], state_slots=device[5], groups=groups,
-            host_new=new, host_begin=begin, host_slots=slots, max_new=max(new), max_context=max_context)
+            host_new=new, host_begin=begin, host_slots=slots, max_new=max(new), max_context=max_context,
+            indices_copied=True)
         return ctx, (device[6] if want_rows.size else None), int(want_rows.size)
 
     def step(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:

@@ -957,9 +957,11 @@ def attention_rows_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, 
                        vdim: int, page_size: int, mask_kind: int, mask_size: int, scale: float,
                        keys_per_value: int = 1, sinks: Optional[torch.Tensor] = None, softcap: float = 0.0,
                        pooled=None, keep_first: int = 0, distance_bias=None,
-                       head_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       head_gate: Optional[torch.Tensor] = None, indices_copied: bool = False) -> torch.Tensor:
     """:func:`attention_prompt_mma` for steps of few rows at any positions: a block a (row, kv head), the kv head's
-    query heads (at most 16) side by side in the tensor-core tile."""
+    query heads (at most 16) side by side in the tensor-core tile.  ``indices_copied``: the caller vouches that
+    ``positions``, ``seq_of_row`` and the block tables came by copies, or from kernels that were done before the kernel in
+    front of this one began; they are then read beside that kernel, which may still run, instead of behind it."""
     _cuda(q, out, cache, positions, seq_of_row, block_table)
     rows = q.shape[0]
     _need(q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.shape[1] == heads * dim, "attention_rows_mma q")
@@ -974,7 +976,7 @@ def attention_rows_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, 
                                      _i32(rows), _i32(heads), _i32(kv_heads), _i32(dim), _i32(vdim), _i32(page_size),
                                      _i32(mask_kind), _i32(mask_size), _f32(scale), _i32(keys_per_value),
                                      _i32(1 if out.dtype == torch.float32 else 0), _ptr(sinks), _f32(softcap), *extras,
-                                     _stream()), "attention_rows_mma")
+                                     _i32(1 if indices_copied else 0), _stream()), "attention_rows_mma")
     return out
 
 
@@ -1663,10 +1665,11 @@ def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, *, he
 def pair_rope_cache(proj: torch.Tensor, q_out: torch.Tensor, cache: torch.Tensor, positions: torch.Tensor,
                     seq_of_row: torch.Tensor, block_table: torch.Tensor, inv_freq: Optional[torch.Tensor], *,
                     q_heads: int, key_heads: int, value_heads: int, dim: int, vdim: int, rot_dims: int,
-                    page_size: int) -> None:
+                    page_size: int, indices_copied: bool = False) -> None:
     """Rotation of neighbouring pairs of the first ``rot_dims`` numbers of every query and key head of ``proj``
     (``[q_heads * dim | key_heads * dim | value_heads * vdim | ...]``); queries into ``q_out``, keys and values into the
-    pages of ``cache`` (``[key_heads, page, dim]`` keys then ``[value_heads, page, vdim]`` values)."""
+    pages of ``cache`` (``[key_heads, page, dim]`` keys then ``[value_heads, page, vdim]`` values).
+    ``indices_copied``: as for :func:`attention_rows_mma`."""
     _cuda(proj, q_out, cache, positions, seq_of_row, block_table, inv_freq)
     rows = q_out.shape[0]
     channels = (q_heads + key_heads) * dim + value_heads * vdim
@@ -1682,8 +1685,8 @@ def pair_rope_cache(proj: torch.Tensor, q_out: torch.Tensor, cache: torch.Tensor
     _check(lib.tb_pair_rope_cache(_ptr(proj), _i64(proj.stride(0)), _ptr(q_out), _i64(q_out.stride(0)), _ptr(cache),
                                   _ptr(positions), _ptr(seq_of_row), _ptr(block_table), _i32(block_table.stride(0)),
                                   _ptr(inv_freq), _i32(rows), _i32(q_heads), _i32(key_heads), _i32(value_heads), _i32(dim),
-                                  _i32(vdim), _i32(rot_dims), _i32(page_size), _i32(_code(proj.dtype)), _stream()),
-           "pair_rope_cache")
+                                  _i32(vdim), _i32(rot_dims), _i32(page_size), _i32(_code(proj.dtype)),
+                                  _i32(1 if indices_copied else 0), _stream()), "pair_rope_cache")
 
 
 def differential_combine(maps: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, *, heads: int,
@@ -1710,11 +1713,12 @@ def differential_combine(maps: torch.Tensor, gate: Optional[torch.Tensor], out: 
 def latent_rope_cache(down: torch.Tensor, q: torch.Tensor, q_full: torch.Tensor, cache: torch.Tensor,
                       weight: torch.Tensor, positions: torch.Tensor, seq_of_row: torch.Tensor, block_table: torch.Tensor,
                       inv_freq: Optional[torch.Tensor], *, heads: int, dim: int, rank: int, rot_width: int,
-                      rot_dims: int, page_size: int, eps: float, amplitude: float = 1.0) -> None:
+                      rot_dims: int, page_size: int, eps: float, amplitude: float = 1.0,
+                      indices_copied: bool = False) -> None:
     """``down`` float32 ``[T, rank + rot_width]``: the first ``rank`` numbers over their root mean square times
     ``weight`` and the rotated rest go into the row's page (``[page, rank + rot_width]`` a page); the rotated parts of the
     query heads (``q`` ``[T, heads * (dim + rot_width)]``) go into ``q_full`` ``[T, heads * (rank + rot_width)]`` behind
-    each head's first ``rank`` numbers, which this kernel leaves alone."""
+    each head's first ``rank`` numbers, which this kernel leaves alone.  ``indices_copied``: as for :func:`attention_rows_mma`."""
     _cuda(down, q, q_full, cache, weight, positions, seq_of_row, block_table, inv_freq)
     rows = q.shape[0]
     _need(down.dtype == torch.float32 and down.stride(1) == 1 and tuple(down.shape) == (rows, rank + rot_width),
@@ -1734,7 +1738,8 @@ def latent_rope_cache(down: torch.Tensor, q: torch.Tensor, q_full: torch.Tensor,
                                     _i64(q_full.stride(0)), _ptr(cache), _ptr(weight), _ptr(positions), _ptr(seq_of_row),
                                     _ptr(block_table), _i32(block_table.stride(0)), _ptr(inv_freq), _i32(rows), _i32(heads),
                                     _i32(dim), _i32(rank), _i32(rot_width), _i32(rot_dims), _i32(page_size), _f32(eps),
-                                    _f32(amplitude), _i32(_code(q.dtype)), _stream()), "latent_rope_cache")
+                                    _f32(amplitude), _i32(_code(q.dtype)), _i32(1 if indices_copied else 0), _stream()),
+           "latent_rope_cache")
 
 
 def attention_latent_mma_supported(dtype: torch.dtype, dim: int, vdim: int) -> bool:
@@ -1745,11 +1750,12 @@ def attention_latent_mma_supported(dtype: torch.dtype, dim: int, vdim: int) -> b
 
 def attention_latent_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, positions: torch.Tensor,
                          seq_of_row: torch.Tensor, block_table: torch.Tensor, *, heads: int, dim: int, vdim: int,
-                         page_size: int, mask_kind: int, mask_size: int, scale: float) -> torch.Tensor:
+                         page_size: int, mask_kind: int, mask_size: int, scale: float, indices_copied: bool = False) -> torch.Tensor:
     """:func:`attention_masked` with ``kv_heads = 1`` and ``keys_per_value = 0`` (pages of ``[page_size, dim]`` vectors
     whose first ``vdim`` numbers are the value) on the tensor cores, for bfloat16: a block a row (in portions of many
     rows three neighbouring rows) and sixteen query heads; exact bfloat16 products with 32-bit accumulation for the scores, 32-bit softmax, the weights as two bfloat16 halves.
-    In a step of few rows every row's keys are shared out among several blocks, and a second kernel adds their results."""
+    In a step of few rows every row's keys are shared out among several blocks, and a second kernel adds their results.
+    ``indices_copied``: as for :func:`attention_rows_mma`."""
     _cuda(q, out, cache, positions, seq_of_row, block_table)
     rows = q.shape[0]
     _need(q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.shape[1] == heads * dim, "attention_latent_mma q")
@@ -1763,7 +1769,8 @@ def attention_latent_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
     _check(lib.tb_attention_latent_mma(_ptr(q), _i64(q.stride(0)), _ptr(out), _i64(out.stride(0)), _ptr(cache),
                                        _ptr(positions), _ptr(seq_of_row), _ptr(block_table), _i32(block_table.stride(0)),
                                        _i32(rows), _i32(block_table.shape[0]), _i32(heads), _i32(dim), _i32(vdim), _i32(page_size),
-                                       _i32(mask_kind), _i32(mask_size), _f32(scale), _ptr(parts), _stream()), "attention_latent_mma")
+                                       _i32(mask_kind), _i32(mask_size), _f32(scale), _ptr(parts), _i32(1 if indices_copied else 0),
+                                       _stream()), "attention_latent_mma")
     if splits > 1:
         global launch_count
         launch_count += 1          # (the kernel that adds the runs up)

@@ -314,6 +314,9 @@ class StepContext:
     host_slots: Sequence[int] = ()
     max_new: int = 1
     max_context: int = 1
+    # the index tensors (positions, rows, slots, block tables) came by copies, or were there before the step's first kernel was
+    # launched: kernels may read them while the kernel in front still runs.  Not so where a kernel of the step makes them.
+    indices_copied: bool = False
     # what a part leaves for parts of later layers of the same step (rows of the step, by name)
     carried: Dict[str, torch.Tensor] = field(default_factory=dict)
 

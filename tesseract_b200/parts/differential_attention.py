@@ -131,13 +131,14 @@ class DifferentialAttention(Mixer):
         q = torch.empty((rows, self.q_width), dtype=proj.dtype, device=proj.device)
         kernels.pair_rope_cache(proj, q, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table, self.inv_freq,
                                 q_heads=2 * H, key_heads=2 * G, value_heads=G, dim=self.key_dim, vdim=self.value_dim,
-                                rot_dims=self.rot_dims, page_size=cache.page_size)
+                                rot_dims=self.rot_dims, page_size=cache.page_size, indices_copied=ctx.indices_copied)
         maps = torch.empty((rows, 2 * H * self.value_dim), dtype=torch.float32, device=proj.device)
         choice = self.attention_choice(rows)
         common = dict(heads=2 * H, kv_heads=2 * G, dim=self.key_dim, vdim=self.value_dim, page_size=cache.page_size,
                       mask_kind=_MASKS[self.mask_kind], mask_size=self.mask_size, scale=self.scale, keys_per_value=2)
         if choice == "attention_rows_mma":
-            kernels.attention_rows_mma(q, maps, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table, **common)
+            kernels.attention_rows_mma(q, maps, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table,
+                                       indices_copied=ctx.indices_copied, **common)
         elif choice == "attention_prompt_mma":
             kernels.attention_prompt_mma(q, maps, cache.storage, ctx.positions, ctx.row_start, group.block_table,
                                          num_seqs=ctx.num_seqs, **common)

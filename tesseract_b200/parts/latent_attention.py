@@ -142,12 +142,14 @@ class LatentAttention(Mixer):
         self._per_head(q.view(rows, H, d + dr)[:, :, :d], self.up_k_t, q_full.view(rows, H, self.entry)[:, :, :rank])
         kernels.latent_rope_cache(down, q, q_full, cache.storage, self.down_norm, ctx.positions, ctx.seq_of_row,
                                   group.block_table, self.inv_freq, heads=H, dim=d, rank=rank, rot_width=dr,
-                                  rot_dims=self.rot_dims, page_size=cache.page_size, eps=self.eps, amplitude=self.amplitude)
+                                  rot_dims=self.rot_dims, page_size=cache.page_size, eps=self.eps, amplitude=self.amplitude,
+                                  indices_copied=ctx.indices_copied)
         mixed = torch.empty((rows, H * rank), dtype=q.dtype, device=q.device)
         if self.attention_choice(rows) == "attention_latent_mma":
             kernels.attention_latent_mma(q_full, mixed, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table,
                                          heads=H, dim=self.entry, vdim=rank, page_size=cache.page_size,
-                                         mask_kind=_MASKS[self.mask_kind], mask_size=self.mask_size, scale=self.scale)
+                                         mask_kind=_MASKS[self.mask_kind], mask_size=self.mask_size, scale=self.scale,
+                                         indices_copied=ctx.indices_copied)
         else:
             kernels.attention_masked(q_full, None, mixed, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table,
                                      heads=H, kv_heads=1, dim=self.entry, vdim=rank, page_size=cache.page_size,

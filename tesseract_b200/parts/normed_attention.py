@@ -264,7 +264,8 @@ class NormedAttention(Mixer):
             kernels.attention_rows_mma(q, attended, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table,
                                        heads=self.num_heads, kv_heads=self.num_kv_heads, dim=self.key_dim,
                                        vdim=self.value_dim, page_size=cache.page_size, mask_kind=_MASKS[self.mask_kind],
-                                       mask_size=self.mask_size, scale=self.scale, **extras)
+                                       mask_size=self.mask_size, scale=self.scale,
+                                       indices_copied=ctx.indices_copied, **extras)
         elif choice == "attention_prompt_mma":
             kernels.attention_prompt_mma(q, attended, cache.storage, ctx.positions, ctx.row_start, group.block_table,
                                          num_seqs=ctx.num_seqs, heads=self.num_heads, kv_heads=self.num_kv_heads,

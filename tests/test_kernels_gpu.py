@@ -180,6 +180,58 @@ def test_rotations_give_few_rows_the_bits_of_many(dtype, q_heads, key_heads, val
         assert all(one.float().abs().sum() > 0 for one in few)
 
 
+@pytest.mark.parametrize("name", ["pair_rope_cache", "latent_rope_cache", "attention_rows_mma", "attention_latent_mma"])
+def test_positions_may_come_from_the_kernel_just_in_front(name):
+    """``select_tokens`` lets its successor begin before it has stored: without the caller's word for the index arrays, the four
+    kernels that read them first must see what it stores."""
+    from tesseract_b200 import kernels
+
+    rows, heads, kv, dim, rank, rot, page = 5, 4, 2, 64, 128, 32, 16
+    g = torch.Generator().manual_seed(7)
+    entry = rank + rot
+    true = dev(torch.tensor([3, 40, 17, 0, 63], dtype=torch.int32))
+    seq, table = dev(torch.arange(rows, dtype=torch.int32)), dev((torch.randperm(4 * rows, generator=g) + 1).to(torch.int32).view(rows, 4))
+    x = dev(torch.randn(rows, 4096, generator=g).bfloat16())
+    pages = dev(torch.randn(4 * rows + 1, page * 2 * kv * dim, generator=g).bfloat16())
+    vectors = dev(torch.randn(4 * rows + 1, page * entry, generator=g).bfloat16())
+    down, weight, freq = dev(torch.randn(rows, entry, generator=g)), dev(torch.ones(rank)), dev(torch.rand(16, generator=g))
+
+    def run(positions, made=lambda: None):
+        place = (positions, seq, table)
+        if name == "pair_rope_cache":
+            out, cache = torch.zeros(rows, heads * dim, dtype=torch.bfloat16, device="cuda"), torch.zeros_like(pages)
+            made()
+            kernels.pair_rope_cache(x[:, :(heads + 2 * kv) * dim], out, cache, *place, freq, q_heads=heads, key_heads=kv, value_heads=kv,
+                                    dim=dim, vdim=dim, rot_dims=32, page_size=page)
+            return out, cache
+        if name == "latent_rope_cache":
+            out, cache = torch.zeros(rows, heads * entry, dtype=torch.bfloat16, device="cuda"), torch.zeros_like(vectors)
+            made()
+            kernels.latent_rope_cache(down, x[:, :heads * (dim + rot)], out, cache, weight, *place, freq, heads=heads, dim=dim, rank=rank,
+                                      rot_width=rot, rot_dims=rot, page_size=page, eps=1e-5)
+            return out, cache
+        latent = name == "attention_latent_mma"
+        width, value = (entry, rank) if latent else (dim, dim)
+        out = torch.zeros(rows, heads * value, dtype=torch.bfloat16, device="cuda")
+        sizes = dict(heads=heads, dim=width, vdim=value, page_size=page, mask_kind=kernels.MASK_CAUSAL, mask_size=0, scale=0.1)
+        q = x[:, :heads * width]
+        made()
+        if latent:
+            kernels.attention_latent_mma(q, out, vectors, *place, **sizes)
+        else:
+            kernels.attention_rows_mma(q, out, pages, *place, kv_heads=kv, **sizes)
+        return (out,)
+
+    want = run(true)
+    torch.cuda.synchronize()
+    source, none, late = true.clone(), torch.full_like(true, -1), torch.zeros_like(true)
+
+    for _ in range(20):
+        late.zero_()
+        got = run(late, lambda: kernels.select_tokens(source, none, none, late, 64))
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("dim, vdim, per_value", [(64, 48, 1), (64, 64, 1), (64, 128, 2), (128, 64, 1), (128, 128, 1)])
 @pytest.mark.parametrize("mask, size", [(0, 1), (1, 100), (2, 64)])
 def test_attention_rows_mma_gives_few_rows_the_bits_of_many(dim, vdim, per_value, mask, size):
