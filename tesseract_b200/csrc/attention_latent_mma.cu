@@ -71,7 +71,7 @@ template <int D, int DV>
 __global__ void __launch_bounds__(128)
 attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
                         const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
-                        int page_size, int mask_kind, int mask_size, float scale, float* __restrict__ parts) {
+                        const Paging paging, int mask_kind, int mask_size, float scale, float* __restrict__ parts) {
     typedef Layout<D, DV> L;
     constexpr int KS = L::KS, PS = L::PS;
     constexpr int COLS = DV / 4;                                  // value columns a warp owns
@@ -86,24 +86,22 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
     const int per_split = (tiles + (int)gridDim.z - 1) / (int)gridDim.z;
     const int tile_first = parts == nullptr ? 0 : min(tiles, (int)blockIdx.z * per_split);
     const int tile_end = parts == nullptr ? tiles : min(tiles, tile_first + per_split);
-    const int64_t page_elems = (int64_t)page_size * D;
+    const int64_t page_elems = (int64_t)paging.size * D;
     const int* table = block_table + (int64_t)seq * bt_stride;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     float* stats = reinterpret_cast<float*>(smem + L::STAT_AT);
 
     // a tile's copy: sixteen lanes a key, whose 16-byte chunks they take side by side, eight keys at a time
-    const int shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;      // (pages are a power of two of tokens in all but odd cases)
-    auto page_of = [&](int key) { return shift >= 0 ? key >> shift : key / page_size; };
     auto look = [&](int tile, int (&pages)[KT / 8]) {             // where this thread's keys lie
 #pragma unroll
-        for (int i = 0; i < KT / 8; ++i) pages[i] = table[page_of(min(key_lo + tile * KT + i * 8 + (tid >> 4), pos))];
+        for (int i = 0; i < KT / 8; ++i) pages[i] = table[paging.page_of(min(key_lo + tile * KT + i * 8 + (tid >> 4), pos))];
     };
     auto fill = [&](int tile, const int (&pages)[KT / 8]) {
         const uint32_t stage = base + (uint32_t)(tile & 1) * L::STAGE;
 #pragma unroll
         for (int i = 0; i < KT / 8; ++i) {
             const int row = i * 8 + (tid >> 4), key = key_lo + tile * KT + row, k = min(key, pos);
-            const bf16* kp = cache + (int64_t)pages[i] * page_elems + (int64_t)(k - page_of(k) * page_size) * D;
+            const bf16* kp = cache + (int64_t)pages[i] * page_elems + (int64_t)paging.within(k) * D;
             const int bytes = key <= pos ? 16 : 0;                // (a key behind the last one is zero-filled)
 #pragma unroll
             for (int c = 0; c < D / 8; c += 16) {
@@ -113,7 +111,7 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
         }
     };
     int pages[KT / 8];
-    look(tile_first, pages);
+    if (tile_first < tile_end) look(tile_first, pages);
     pdl_wait();                                                   // queries and the step's keys come from kernels in front (its metadata does not: see `early` below)
     // the sixteen heads' queries (heads the model does not have are rows of zeros)
     for (int index = tid; index < 16 * (D / 8); index += 128) {
@@ -124,7 +122,7 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
     }
     if (tile_first < tile_end) fill(tile_first, pages);
     cp_async_commit();
-    look(tile_first + 1, pages);                                  // (a tile ahead from here on)
+    if (tile_first + 1 < tile_end) look(tile_first + 1, pages);   // (a tile ahead from here on)
 
     float m[2] = {-1.0e30f, -1.0e30f}, l[2] = {0.0f, 0.0f};
     float o[COLS / 8][4];
@@ -562,7 +560,7 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
     if (splits > 1 && (uintptr_t)parts % 8 != 0) return TB_ERR_BAD_ALIGN;
     cudaError_t launched = tb_launch(early, kernel, dim3(rows, (heads + 15) / 16, splits), dim3(128), (size_t)smem, stream,
                                          (const bf16*)q, q_stride, (bf16*)out, out_stride, (const bf16*)cache, positions,
-                                         seq_of_row, block_table, bt_stride, heads, page_size, mask_kind, mask_size, scale,
+                                         seq_of_row, block_table, bt_stride, heads, tb_paging(page_size), mask_kind, mask_size, scale,
                                          splits > 1 ? parts : (float*)nullptr);
     if (launched != cudaSuccess) return (int)launched;
     if (splits > 1) {

@@ -108,23 +108,9 @@ __device__ __forceinline__ float distance_bias(float weight, float rate, int dis
     return weight * v;
 }
 
-// BIASED: the scores lose their distance bias (a kernel of its own: the others keep their registers).
-// Pages are a power of two of tokens in all but odd cases, and a thread looks up many keys.
-struct Pages {
-    int size, shift;                                              // shift: -1 where it takes a division
-    __device__ __forceinline__ int of(int key) const { return shift >= 0 ? key >> shift : key / size; }
-    __device__ __forceinline__ int within(int key) const { return shift >= 0 ? key & (size - 1) : key % size; }
-};
-__device__ __forceinline__ Pages pages_of(int page_size) {
-    Pages p;
-    p.size = page_size;
-    p.shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;
-    return p;
-}
-
 // A key's and its value's 16-byte chunks, by eight lanes side by side (bytes 0: zeros).  By two threads a key, half a row each, a warp's
 // copies touched 32 half sectors of 16 rows, and the copies bound decoded rows: 128 rows of 8 kv heads of 128 behind 4,000 keys
-// 766 us, 426 so.
+// 770 us, 401 so.
 template <int D, int DV>
 __device__ __forceinline__ void copy_key(uint32_t to_key, uint32_t to_value, const bf16* key, const bf16* value, int lane, int bytes) {
 #pragma unroll
@@ -134,12 +120,13 @@ __device__ __forceinline__ void copy_key(uint32_t to_key, uint32_t to_value, con
         if (DV % 64 == 0 || c + lane < DV / 8) cp_async16(to_value + (c + lane) * 16, value + (c + lane) * 8, bytes);
 }
 
+// BIASED: the scores lose their distance bias (a kernel of its own: the others keep their registers).
 template <int D, int DV, bool BIASED>
 __global__ void __launch_bounds__(128)
 attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __restrict__ out, int64_t out_stride,
                         const bf16* __restrict__ cache, const int* __restrict__ positions,
                         const int* __restrict__ row_start, const int* __restrict__ block_table, int bt_stride,
-                        int num_seqs, int heads, int kv_heads, int page_size, int mask_kind, int mask_size, float scale,
+                        int num_seqs, int heads, int kv_heads, const Paging paging, int mask_kind, int mask_size, float scale,
                         int keys_per_value, int out_f32, Extras x) {
     constexpr int KS = D * 2 + 16, VS = DV * 2 + 16;              // bytes of a key row and a value row in shared memory
     constexpr int STAGE = KT * (KS + VS);
@@ -176,15 +163,14 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
     const int span = blocks_last + pos_last - key_lo + 1;
     const int tiles = (span - 1) / KT + 1;
     // keys_per_value key heads in a row read one value head: the page holds kv_heads / keys_per_value of those
-    const int64_t page_elems = (int64_t)kv_heads * page_size * D + (int64_t)(kv_heads / keys_per_value) * page_size * DV;
-    const int64_t k_off = (int64_t)kv_head * page_size * D;
-    const int64_t v_off = (int64_t)kv_heads * page_size * D + (int64_t)(kv_head / keys_per_value) * page_size * DV;
+    const int64_t page_elems = (int64_t)kv_heads * paging.size * D + (int64_t)(kv_heads / keys_per_value) * paging.size * DV;
+    const int64_t k_off = (int64_t)kv_head * paging.size * D;
+    const int64_t v_off = (int64_t)kv_heads * paging.size * D + (int64_t)(kv_head / keys_per_value) * paging.size * DV;
     const int* table = block_table + (int64_t)seq * bt_stride;
     const int* pool_table = x.pool_table == nullptr ? nullptr : x.pool_table + (int64_t)seq * x.pool_bt_stride;
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(tile_smem);
 
     // a tile's copy: eight lanes a key, whose 16-byte chunks they take side by side, sixteen keys at a time
-    const Pages paging = pages_of(page_size);
     auto fill = [&](int tile) {
         const uint32_t stage = smem_base + (uint32_t)(tile & 1) * STAGE;
         int pages[KT / 16];
@@ -197,7 +183,7 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
         for (int i = 0; i < KT / 16; ++i) {
             bool averaged;
             const int k = key_at(i, averaged);
-            pages[i] = (averaged ? pool_table : table)[paging.of(k)];
+            pages[i] = (averaged ? pool_table : table)[paging.page_of(k)];
         }
 #pragma unroll
         for (int i = 0; i < KT / 16; ++i) {
@@ -394,7 +380,7 @@ template <int D, int DV, bool BIASED, int STAGES>
 __global__ void __launch_bounds__(128)
 attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
                       const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
-                      int kv_heads, int page_size, int mask_kind, int mask_size, float scale, int keys_per_value,
+                      int kv_heads, const Paging paging, int mask_kind, int mask_size, float scale, int keys_per_value,
                       int out_f32, Extras x) {
     constexpr int KS = D * 2 + 16, VS = DV * 2 + 16;
     constexpr int STAGE = KT * (KS + VS);
@@ -411,19 +397,18 @@ attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_st
     const int span = blocks + pos - key_lo + 1;
     const int tiles = (span - 1) / KT + 1;
     // keys_per_value key heads in a row read one value head: the page holds kv_heads / keys_per_value of those
-    const int64_t page_elems = (int64_t)kv_heads * page_size * D + (int64_t)(kv_heads / keys_per_value) * page_size * DV;
-    const int64_t k_off = (int64_t)kv_head * page_size * D;
-    const int64_t v_off = (int64_t)kv_heads * page_size * D + (int64_t)(kv_head / keys_per_value) * page_size * DV;
+    const int64_t page_elems = (int64_t)kv_heads * paging.size * D + (int64_t)(kv_heads / keys_per_value) * paging.size * DV;
+    const int64_t k_off = (int64_t)kv_head * paging.size * D;
+    const int64_t v_off = (int64_t)kv_heads * paging.size * D + (int64_t)(kv_head / keys_per_value) * paging.size * DV;
     const int* table = block_table + (int64_t)seq * bt_stride;
     const int* pool_table = x.pool_table == nullptr ? nullptr : x.pool_table + (int64_t)seq * x.pool_bt_stride;
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(tile_smem);
-    const Pages paging = pages_of(page_size);
     auto key_at = [&](int tile, int i) { return min(tile * KT + i * 16 + (tid >> 3), span - 1); };      // of the keys in walking order
     auto look = [&](int tile, int (&pages)[KT / 16]) {            // where this thread's keys of a tile lie
 #pragma unroll
         for (int i = 0; i < KT / 16; ++i) {
             const int a = key_at(tile, i);
-            pages[i] = (averages && a < blocks ? pool_table : table)[paging.of(a < blocks ? a : key_lo + a - blocks)];
+            pages[i] = (averages && a < blocks ? pool_table : table)[paging.page_of(a < blocks ? a : key_lo + a - blocks)];
         }
     };
     auto fill = [&](int tile, const int (&pages)[KT / 16]) {      // eight lanes a key, sixteen keys at a time
@@ -459,7 +444,6 @@ attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_st
         if (st < tiles) fill(st, early[st]);
         cp_async_commit();
     }
-    look(STAGES - 1, pages);                                      // (a tile ahead from here on)
     float m[2] = {-1.0e30f, -1.0e30f}, l[2] = {0.0f, 0.0f};
     if (x.sinks != nullptr && warp == 0) {                        // the sink is the start of ONE of the four running softmaxes
 #pragma unroll
@@ -483,16 +467,7 @@ attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_st
     for (int j = 0; j < DV / 8; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.0f;
-    for (int tile = 0; tile < tiles; ++tile) {
-        auto ask = [&]() {
-            if (tile + STAGES - 1 < tiles) fill(tile + STAGES - 1, pages);
-            cp_async_commit();
-            look(tile + STAGES, pages);
-        };
-        if (STAGES == 2) ask();
-        cp_async_wait<STAGES == 2 ? 1 : STAGES - 2>();
-        __syncthreads();                                          // (STAGES > 2: and the stage of the tile in front is free)
-        if (STAGES > 2) ask();
+    auto consume = [&](int tile) {
         const uint32_t kstage = smem_base + (uint32_t)(tile % STAGES) * STAGE, vstage = kstage + KT * KS;
         const int at0 = tile * KT + warp * 16;                    // the warp's 16 keys of the tile
         if (at0 < span) {
@@ -559,8 +534,30 @@ attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_st
                 mma_bf16_16816(o[2 * jp + 1], lo, b + 2);
             }
         }
+    };
+    // ask: for the tile STAGES - 1 further on, and where the one behind it lies.  Two loops: rows of few tiles look up nothing that
+    // they do not copy, and those of many have no branch around the look-ups (what is loaded in one is waited for at its end).  With that
+    // and no branch at a key's page, 4 rows of 8 kv heads of 64 behind 30 / 130 / 4,000 keys take 2.4 / 3.9 / 56.9 us instead of
+    // 3.0 / 5.6 / 68.3; 8 rows behind 4,000 with the look-ups in a branch 80, without 67.
+    auto step = [&](int tile, bool ask) {
+        auto next = [&]() {
+            if (ask) fill(tile + STAGES - 1, pages);
+            cp_async_commit();
+            if (ask) look(tile + STAGES, pages);
+        };
+        if (STAGES == 2) next();
+        cp_async_wait<STAGES == 2 ? 1 : STAGES - 2>();
+        __syncthreads();                                          // (STAGES > 2: and the stage of the tile in front is free)
+        if (STAGES > 2) next();
+        consume(tile);
         if (STAGES == 2) __syncthreads();
+    };
+    int tile = 0;
+    if (tiles >= STAGES) {
+        look(STAGES - 1, pages);                                  // (a tile ahead from here on)
+        for (; tile + STAGES - 1 < tiles; ++tile) step(tile, true);
     }
+    for (; tile < tiles; ++tile) step(tile, false);
     // the warps' partial results, then their sum in warp order
     float* parts = reinterpret_cast<float*>(tile_smem + STAGES * STAGE);
 #pragma unroll
@@ -601,7 +598,8 @@ attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_st
 
 constexpr int kDeep = 5;
 constexpr int rows_smem(int d, int dv, int stages) { return stages * KT * (d * 2 + 16 + dv * 2 + 16) + 4 * 16 * (dv + 2) * 4; }
-// Whether as many blocks of kDeep stages run at once: 16 rows of 8 kv heads of 64, values of 128, behind 300 keys 9.5 us, 14.8 with two.
+// Whether as many blocks of kDeep stages run at once: 16 rows of 8 kv heads of 64, values of 128, behind 300 / 4,000 keys 7.8 / 58.4 us,
+// with two 9.4 / 78.5.  (A few blocks are within 10 % either way: 4 rows of 64 and 64 behind 300 keys 6.0 and 5.7, behind 130 3.9 and 4.2.)
 bool deep_fits(int64_t blocks, int d, int dv) { return blocks <= 148 * (int64_t)(227 * 1024 / (rows_smem(d, dv, kDeep) + 1024)); }
 
 template <int D, int DV, int STAGES>
@@ -617,7 +615,7 @@ int launch_rows(const void* q, int64_t q_stride, void* out, int64_t out_stride, 
     }
     cudaError_t launched = tb_launch(early, kernel, dim3(rows, kv_heads), dim3(128), (size_t)smem, stream, (const bf16*)q,
                                          q_stride, (bf16*)out, out_stride, (const bf16*)cache, positions, seq_of_row,
-                                         block_table, bt_stride, heads, kv_heads, page_size, mask_kind, mask_size, scale,
+                                         block_table, bt_stride, heads, kv_heads, tb_paging(page_size), mask_kind, mask_size, scale,
                                          keys_per_value, out_f32, x);
     return launched == cudaSuccess ? tb_launch_status() : (int)launched;
 }
@@ -636,7 +634,7 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
     const dim3 grid((rows + QT - 1) / QT + num_seqs, heads);
     cudaError_t launched = tb_launch_pdl(kernel, grid, dim3(128), (size_t)smem, stream, (const bf16*)q, q_stride,
                                          (bf16*)out, out_stride, (const bf16*)cache, positions, row_start, block_table,
-                                         bt_stride, num_seqs, heads, kv_heads, page_size, mask_kind, mask_size, scale,
+                                         bt_stride, num_seqs, heads, kv_heads, tb_paging(page_size), mask_kind, mask_size, scale,
                                          keys_per_value, out_f32, x);
     return launched == cudaSuccess ? tb_launch_status() : (int)launched;
 }

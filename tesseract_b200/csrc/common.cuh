@@ -49,6 +49,24 @@ static inline cudaError_t tb_launch_pdl(void (*kernel)(KernelArgs...), dim3 grid
     return tb_launch(true, kernel, grid, block, smem, stream, args...);
 }
 
+// Where a key lies in pages of `size` tokens, without a division or a branch (a thread of the attention kernels looks up four to eight keys
+// a tile, and a branch to a division or a shift at each made portions of 20 tokens a tenth slower).  With 2^l the smallest power of two that is not below size,
+// N = 32 + max(l - 1, 0) and m = (2^N - 1) / size rounded down (m < 2^32), (key + 1) * m / 2^N rounded down is key / size for every
+// key and size below 2^31: m * size = 2^N - 1 - r with r < size, so the quotient falls short of (key + 1) / size by
+// (key + 1) * (r + 1) / (size * 2^N), which is more than nothing and, as (key + 1) * (r + 1) <= 2^31 * 2^l, no more than 1 / size.
+struct Paging {
+    uint32_t inverse;
+    int shift, size;
+    __device__ __forceinline__ int page_of(int key) const { return (int)(__umulhi((uint32_t)key + 1u, inverse) >> shift); }
+    __device__ __forceinline__ int within(int key) const { return key - page_of(key) * size; }
+};
+static inline Paging tb_paging(int page_size) {
+    Paging p = {0, 0, page_size};
+    while (((int64_t)2 << p.shift) < page_size) ++p.shift;
+    p.inverse = (uint32_t)((((uint64_t)1 << (32 + p.shift)) - 1) / (uint64_t)page_size);
+    return p;
+}
+
 static inline int tb_launch_status() {
     cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;

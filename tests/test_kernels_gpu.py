@@ -259,6 +259,73 @@ def test_attention_rows_mma_gives_few_rows_the_bits_of_many(dim, vdim, per_value
         assert torch.equal(run(lo, hi), many[lo:hi])
 
 
+@pytest.mark.parametrize("page", [1, 2, 12, 24, 37, 64])
+@pytest.mark.parametrize("dim, vdim, per_value, mask, size", [(64, 48, 1, 0, 1), (64, 64, 1, 1, 100), (64, 128, 2, 2, 70), (128, 128, 1, 0, 1)])
+def test_pages_of_any_size_give_the_bits_of_pages_of_sixteen(page, dim, vdim, per_value, mask, size):
+    """A key's page without a division: the same keys in pages of any size, for portions, for few rows (five tiles ahead) and for many."""
+    from tesseract_b200 import kernels
+
+    kv, heads, seqs = 4, 8, 3
+    spans = [(0, 200), (500, 90), (40, 1)]                       # (first position, rows)
+    length = max(first + n for first, n in spans)
+    g = torch.Generator().manual_seed(page + dim)
+    k, v = (torch.randn(seqs, length, h, d, generator=g).bfloat16() for h, d in ((kv, dim), (kv // per_value, vdim)))
+    rows = sum(n for _, n in spans)
+    q = dev(torch.randn(rows, heads * dim, generator=g).bfloat16())
+    positions = dev(torch.cat([torch.arange(b, b + n) for b, n in spans]).to(torch.int32))
+    of_row = dev(torch.tensor([i for i, (_, n) in enumerate(spans) for _ in range(n)], dtype=torch.int32))
+    starts = dev(torch.tensor([0, 200, 290, 291], dtype=torch.int32))
+    common = dict(heads=heads, kv_heads=kv, dim=dim, vdim=vdim, mask_kind=mask, mask_size=size, scale=dim ** -0.5, keys_per_value=per_value)
+
+    def run(page):
+        each = -(-length // page)
+        table = (torch.randperm(seqs * each, generator=torch.Generator().manual_seed(1)) + 1).to(torch.int32).view(seqs, each)
+        cache = torch.zeros(seqs * each + 1, page * (kv * dim + kv // per_value * vdim), dtype=torch.bfloat16)
+        for values, at in ((k, 0), (v, kv * page * dim)):
+            h, d = values.shape[2:]
+            padded = torch.zeros(seqs, each * page, h, d, dtype=torch.bfloat16)
+            padded[:, :length] = values
+            cache[table.long(), at:at + h * page * d] = padded.view(seqs, each, page, h, d).transpose(2, 3).reshape(seqs, each, -1)
+        cache, table = dev(cache), dev(table)
+        outs = [torch.empty(n, heads * vdim, device="cuda") for n in (rows, rows, 5)]
+        kernels.attention_prompt_mma(q, outs[0], cache, positions, starts, table, num_seqs=seqs, page_size=page, **common)
+        kernels.attention_rows_mma(q, outs[1], cache, positions, of_row, table, page_size=page, **common)
+        kernels.attention_rows_mma(q[rows - 5:], outs[2], cache, positions[rows - 5:], of_row[rows - 5:], table, page_size=page, **common)
+        return outs
+
+    want = run(16)
+    assert torch.isfinite(want[0]).all() and torch.equal(want[1][rows - 5:], want[2])
+    assert all(torch.equal(a, b) for a, b in zip(run(page), want))
+
+
+@pytest.mark.parametrize("page", [1, 12, 37])
+@pytest.mark.parametrize("dim, vdim, heads", [(576, 512, 16), (160, 128, 20)])
+@pytest.mark.parametrize("rows", [3, 200])
+def test_latent_pages_of_any_size_give_the_bits_of_pages_of_sixteen(page, dim, vdim, heads, rows):
+    from tesseract_b200 import kernels
+
+    length, seqs = 300, 3
+    g = torch.Generator().manual_seed(page)
+    vectors = torch.randn(seqs, length, dim, generator=g).bfloat16()
+    q = dev(torch.randn(rows, heads * dim, generator=g).bfloat16())
+    positions, of_row = torch.randint(0, length, (rows,), generator=g, dtype=torch.int32), torch.arange(rows, dtype=torch.int32) % seqs
+    positions[0], positions[1] = 0, length - 1
+
+    def run(page):
+        each = -(-length // page)
+        table = (torch.randperm(seqs * each, generator=torch.Generator().manual_seed(1)) + 1).to(torch.int32).view(seqs, each)
+        padded = torch.zeros(seqs, each * page, dim, dtype=torch.bfloat16)
+        padded[:, :length] = vectors
+        cache = torch.zeros(seqs * each + 1, page * dim, dtype=torch.bfloat16)
+        cache[table.long()] = padded.view(seqs, each, page * dim)
+        out = torch.empty(rows, heads * vdim, dtype=torch.bfloat16, device="cuda")
+        return kernels.attention_latent_mma(q, out, dev(cache), dev(positions), dev(of_row), dev(table), heads=heads, dim=dim, vdim=vdim,
+                                            page_size=page, mask_kind=kernels.MASK_WINDOW, mask_size=130, scale=dim ** -0.5)
+
+    want = run(16)
+    assert torch.isfinite(want).all() and torch.equal(run(page), want)
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 1, 1), (3, 5, 7), (64, 64, 16), (65, 130, 33), (200, 96, 96), (17, 331, 72),
                                      (2, 1000, 2048)])
 def test_gemm_f32(m, n, k):
