@@ -154,14 +154,9 @@ constexpr int kTile = 16;            // the most rows of a tile
 template <int KIND>
 struct Coefficients { static constexpr int N = KIND == DELTA ? 44 : 32; };
 
-// (A block holds at most 32 columns: with eight lanes a column four warps of state.)  BLOCKS: on a multiprocessor.  With 128 registers a
-// thread two blocks of eight lanes a column fit, and steps that have them are bound by the chain of a group, which the other block
-// hides: 32 sequences of 75 rows, state space / delta rule, 276 / 203 us, one block 356 / 240.  A single prompt has a block a
-// multiprocessor and wants the registers (2,048 rows of the state space: 275 us, 326 with 128).
-constexpr int most_workers(int lpc) { return lpc / 2 < kWorkers ? lpc / 2 : kWorkers; }
-
-template <typename T, int KIND, int LPC, int NJ, int BLOCKS>
-__global__ void __launch_bounds__((most_workers(LPC) + kProducers) * 32, BLOCKS)
+// WORKERS: the most warps of state in a block (a block holds at most 32 columns); BLOCKS: those that are to fit on a multiprocessor.
+template <typename T, int KIND, int LPC, int NJ, int WORKERS, int BLOCKS>
+__global__ void __launch_bounds__((WORKERS + kProducers) * 32, BLOCKS)
 matrix_recurrence_kernel(const T* __restrict__ rows, Recurrence p) {
     constexpr int DP = 4 * LPC * NJ;                 // numbers of q or k in shared memory (zeros behind dim)
     constexpr int CPL = 2, CW = 32 / LPC * CPL;
@@ -670,6 +665,36 @@ matrix_recurrence_step_kernel(const T* __restrict__ rows, Recurrence p, int runs
     }
 }
 
+// Which compilation of the kernel a step takes.  Many blocks are bound by the chain of a group of rows, which other blocks on the
+// multiprocessor hide, and few want the registers: with a block a multiprocessor as many as the compiler likes (first form), else
+// few enough for `fit` blocks.  Where the lines lie was measured over 1 to 64 sequences of 2 to 64 heads; us, first form / with `fit`:
+//   state space, 64 heads of 64: dim 32 at 384 blocks 43 / 49, at 1,024 38.5 / 34.6, at 8,192 261 / 214; dim 64 at 512 57 / 66, at
+//     4,096 167 / 166, at 8,192 290 / 281; dim 96 at 192 blocks of two warps 39.2 / 37.8, at 8,192 332 / 337; dim 128 at 8,192 552 / 446
+//   matrix memory, 16 heads of 128: dim 32 at 400 blocks 29.6 / 30.3, at 640 34.5 / 29.9, at 5,120 191 / 150; dim 64 at 160 86 / 112, at
+//     320 59 / 51, at 5,120 217 / 187; dim 128 at 160 149 / 115, at 5,120 414 / 276; one sequence (144 blocks of two warps) dim 32
+//     138 / 128, dim 64 151 / 143
+//   delta rule, 16 heads of 128: dim 32 at 192 blocks of two warps 33.5 / 31.2, at 256 of four 35 / 50, at 320 32 / 28, at 4,096 172 / 150;
+//     dim 64 / 96 / 128 at 256 55 / 44, 63 / 56, 71 / 70, at 4,096 303 / 204, 342 / 256, 373 / 319; sixteen lanes a column, dim 128, at
+//     192 blocks of four warps 59 / 46, of two 35.5 / 37.1
+// (Blocks of two warps of state with the delta rule at dims 65 to 96 have a third form, for they leave two of them 168 registers: 192
+// blocks 38 us, 43 with the 128 that two whole blocks leave.)
+constexpr int most_workers(int lpc, int nj) { return lpc == 8 || (lpc == 16 && nj == 2) ? 4 : kWorkers; }     // (16 lanes of 2: few blocks alone)
+constexpr int crowd_fit(int kind, int lpc, int nj) {          // 1: the first form serves all steps
+    if (lpc == 16) return kind == DELTA && nj == 2 ? 2 : 1;
+    if (lpc != 8 || (nj == 3 && kind == MEMORY)) return 1;
+    return nj == 1 ? (kind == DELTA ? 3 : 4) : nj == 2 ? (kind == DELTA ? 2 : 3) : 2;
+}
+bool crowded(int kind, int lpc, int nj, int workers, int64_t blocks) {
+    if (lpc == 16) return workers == 4 && blocks > 148;
+    if (kind == MEMORY && nj < 3 && workers < 4) {
+        if (workers == 2) return blocks <= 148;
+        if (nj == 1 && blocks > 148) return true;
+    }
+    if (kind == STATE_SPACE && nj == 3) return workers < 4 && blocks > 148;
+    if (kind == DELTA && nj == 1) return blocks > (workers < 4 ? 148 : 296);
+    return blocks > (nj == 1 ? 444 : nj == 4 || kind == DELTA ? 148 : kind == MEMORY ? 296 : 4000);
+}
+
 template <typename T, int KIND, int LPC, int NJ>
 int launch_as(const void* rows, Recurrence p, int num_seqs, int single, cudaStream_t stream) {
     constexpr int CW = 32 / LPC * 2, DP = 4 * LPC * NJ;
@@ -684,15 +709,21 @@ int launch_as(const void* rows, Recurrence p, int num_seqs, int single, cudaStre
         return launched == cudaSuccess ? tb_launch_status() : (int)launched;
     }
     // few blocks: fewer columns a block, so that more multiprocessors take part
-    p.workers = min(kWorkers, 32 / CW);
+    p.workers = min(most_workers(LPC, NJ), 32 / CW);
     while (p.workers > 1 && (int64_t)num_seqs * p.heads * ((p.columns + p.workers * CW - 1) / (p.workers * CW)) < kFewBlocks) p.workers /= 2;
     p.tile = DP > 512 ? kTile / 2 : kTile;
     const int VC = p.workers * CW;
     const size_t smem = sizeof(float) * 2 * (p.tile * (2 * DP + VC) + p.tile / kGroup * Coefficients<KIND>::N);
     const int64_t blocks = (int64_t)num_seqs * p.heads * ((p.columns + VC - 1) / VC);
-    auto kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, 1>;
-    if constexpr (LPC == 8) {
-        if (blocks > 148) kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, 2>;
+    constexpr int MOST = most_workers(LPC, NJ), FIT = crowd_fit(KIND, LPC, NJ);
+    auto kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, MOST, 1>;
+    if constexpr (FIT > 1) {
+        if (crowded(KIND, LPC, NJ, p.workers, blocks)) {
+            kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, MOST, FIT>;
+            if constexpr (KIND == DELTA && NJ == 3) {
+                if (p.workers <= 2) kernel = matrix_recurrence_kernel<T, KIND, LPC, NJ, 2, FIT>;
+            }
+        }
     }
     if (smem > 40 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

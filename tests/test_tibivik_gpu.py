@@ -320,6 +320,51 @@ def test_cuts_of_the_recurrence_differ_by_rounding(kind, m):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads", [4, 8])
+@pytest.mark.parametrize("dim", [24, 62, 64, 90, 128])
+@pytest.mark.parametrize("kind", ["STATE_SPACE", "MATRIX_MEMORY", "DELTA_RULE"])
+def test_a_sequence_has_the_same_bits_among_any_number_of_others(kind, dim, heads, dtype):
+    """Steps of few blocks and of many take kernels compiled for different numbers of blocks a multiprocessor: 1 to 130 sequences reach
+    every one of them, with whole blocks and with blocks of one and two warps."""
+    from tesseract_b200 import kernels
+
+    code, vdim, most = getattr(kernels, kind), 128, 130
+    qk = 1 if kind == "STATE_SPACE" else heads
+    g = torch.Generator().manual_seed(dim + heads)
+    lengths = [37] + [3 + (7 * i) % 23 for i in range(1, most)]
+    starts = [sum(lengths[:i]) for i in range(most + 1)]
+    rows = torch.randn(starts[-1], 2 * qk * dim + heads * vdim, generator=g).to(dtype).to(dev())
+    gates = torch.randn(starts[-1], 2 * heads, generator=g).to(dev())
+    vectors = [(-torch.rand(heads, generator=g)).to(dev()) for _ in range(3 if kind == "STATE_SPACE" else 2)]
+    shape = kernels.matrix_state_shape(code, heads, dim, vdim)
+    before = torch.randn(most, *shape, generator=g).to(dev())
+
+    def run(count):
+        T, state, running = starts[count], before[:count].clone(), torch.zeros(count, *shape[:2], device=dev())
+        out, aux = torch.empty(T, heads * vdim, device=dev()), torch.zeros(T, heads, 2, device=dev())
+        memory = kind == "MATRIX_MEMORY"
+        kernels.matrix_recurrence(code, rows[:T], (0, qk * dim, 2 * qk * dim), gates[:T], vectors, state, out, i32(starts[:count + 1]),
+                                  i32(list(range(count))), num_seqs=count, heads=heads, qk_heads=qk, dim=dim, vdim=vdim, max_new=37,
+                                  q_scale=0.3, cap=5.0, running=running if memory else None, aux=aux if memory else None)
+        return out, aux, state, running
+
+    def share(of):                            # the lanes of a column: from 120 blocks on half as many for the largest sizes
+        return dim > 96 and of * heads * -(-(vdim + (kind == "MATRIX_MEMORY")) // 32) < 120
+
+    runs = {}
+    for count in (1, 2, 3, 4, 6, 8, 20, most):
+        got = run(count)
+        assert all(torch.isfinite(x).all() for x in got) and got[0].abs().sum() > 0
+        fewer = runs.get(share(count))
+        if fewer is not None:
+            assert all(torch.equal(one, two[:one.shape[0]]) for one, two in zip(fewer, got)), count
+        elif runs:                            # the sums over a column in another order
+            for one, two in zip(next(iter(runs.values())), got):
+                assert float((one - two[:one.shape[0]]).abs().max()) <= 2e-5 * max(1.0, float(one.abs().max())), count
+        runs[share(count)] = got
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["state_space", "matrix_memory", "gated_delta"])
 def test_recurrences_remember_one_token_over_hundreds(dtype, kind):
     """One token writes; 520 silent ones follow; the last one asks.  With decays near one its value must still be there."""
