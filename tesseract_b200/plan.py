@@ -105,14 +105,18 @@ def product(dtype: torch.dtype, rows: int, out_features: int, in_features: int, 
     """The kernel for ``[rows, in] @ [out, in]^T``.  ``norm``: ``"norm"`` or ``"add_norm"`` if an RMSNorm (with the
     residual addition) stands in front and may be folded in, ``"prepared"`` if the product in front has done that
     norm's work; ``epilogue``: ``bf16``, ``f32`` (logits), or ``swiglu``, ``gated_silu`` or ``gated_gelu`` (the weight's rows interleave
-    eight gates and eight up projections; the last two without a norm folded in front); ``follow``: an addition and an RMSNorm of the product's own width follow it."""
+    eight gates and eight up projections; in front of the last two a norm always runs on its own); ``follow``: an addition and an
+    RMSNorm of the product's own width follow it."""
     if dtype == torch.float32:
         return ProductPlan("gemm_f32", False, F32, activation_apart=epilogue in OVER_GATE_AND_UP)
+    if epilogue in (GATED_SILU, GATED_GELU):
+        norm = None                   # (the kernels have these epilogues without a norm in front)
     if rows <= DECODE_LINEAR_MAX_ROWS and contiguous_rows:
         if norm == "prepared":
             if _decode_linear_takes(rows, out_features, in_features, kernels.PRO_NONE):
                 return ProductPlan("decode_linear", True, epilogue, takes_prepared=True)
-            return ProductPlan("library", False, BF16 if epilogue == SWIGLU else epilogue, activation_apart=epilogue == SWIGLU)
+            apart = epilogue in OVER_GATE_AND_UP
+            return ProductPlan("library", False, BF16 if apart else epilogue, activation_apart=apart)
         if follow and norm is None and epilogue == BF16 and _decode_linear_takes(rows, out_features, in_features,
                                                                                 kernels.PRO_NONE):
             return ProductPlan("decode_linear", False, BF16, prepares_norm=True)

@@ -3,6 +3,7 @@ the decode attention uses.  The parts do what these functions answer, so pinning
 
 import itertools
 
+import pytest
 import torch
 
 from tesseract_b200 import plan
@@ -79,6 +80,18 @@ def test_products_of_the_1b_sizes():
         assert plan.product(BF, rows, vocab, hidden, epilogue="f32") == plan.ProductPlan("library", False, "f32")
     assert plan.DECODE_LINEAR_MAX_ROWS == 16 and plan.SKINNY_MAX_ROWS == 128
     assert plan.FUSED_GATE_UP_MIN_ROWS == plan.DECODE_LINEAR_MAX_ROWS + 1
+
+
+@pytest.mark.parametrize("epilogue", [plan.GATED_SILU, plan.GATED_GELU])
+@pytest.mark.parametrize("norm", [None, "norm", "add_norm", "prepared"])
+def test_a_norm_in_front_of_a_gated_epilogue_runs_on_its_own(epilogue, norm):
+    # no kernel has these epilogues with a norm folded in front: the plan must not promise one, whatever stands in front
+    for rows, kernel in ((1, "decode_linear"), (16, "decode_linear"), (17, "skinny_tcgen05"), (128, "skinny_tcgen05")):
+        assert plan.product(BF, rows, 2 * 8192, 2048, epilogue=epilogue, norm=norm) == plan.ProductPlan(kernel, False, epilogue)
+    for rows, out, width in ((129, 2 * 8192, 2048), (2048, 2 * 8192, 2048), (4, 2 * 200, 72), (40, 2 * 200, 76)):
+        apart = plan.product(BF, rows, out, width, epilogue=epilogue, norm=norm)
+        assert apart.activation_apart and apart.epilogue == "bf16" and not apart.norm_folded and not apart.takes_prepared
+    assert plan.product(F32, 5, 2 * 200, 72, epilogue=epilogue, norm=norm) == plan.ProductPlan("gemm_f32", False, "f32", activation_apart=True)
 
 
 def test_products_of_sizes_a_kernel_does_not_take_fall_to_the_next():
