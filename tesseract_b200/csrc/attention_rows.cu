@@ -175,7 +175,7 @@ attention_rows_shared_kernel(const T* q, int64_t q_stride, T* out, int64_t out_s
                              const int* __restrict__ positions, const int* __restrict__ seq_of_row,
                              const int* __restrict__ block_table, int bt_stride, int num_heads, int num_kv_heads, int head_dim,
                              int page_size, int window, float scale) {
-    constexpr int UNDER = 32 / Vec16<T>::N;            // packets of a key under way
+    constexpr int UNDER = sizeof(T) == 4 ? 8 : 1;    // packets of a key under way (bfloat16: four at a time spilled, and took 4 to 14 % longer)
     __shared__ float score[kRun * kKeyBlock];        // then the weights
     __shared__ int64_t offset[kRun * kKeyBlock];     // of a key in its half of the cache
     __shared__ float block_max[kRun], block_sum_of[kRun], max_so_far[kRun], qs[NC * 32];
@@ -283,13 +283,14 @@ attention_rows_shared_kernel(const T* q, int64_t q_stride, T* out, int64_t out_s
 template <typename T>
 int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
            const int* positions, const int* seq_of_row, const int* block_table, int bt_stride, int rows,
-           int num_heads, int num_kv_heads, int head_dim, int page_size, int window, float scale,
+           int num_heads, int num_kv_heads, int head_dim, int page_size, int reach, int window, float scale,
            cudaStream_t stream) {
-    // Few rows: 4 and 8 rows of 32 heads of 64 behind 130 keys, 32-bit, 9.4 and 9.7 us against 16.5 and 16.6 by a warp a (row, head), behind
-    // 6,000 keys 295 and 308 against 690 and 725; 16 rows 18.5 against 16.7, for then the blocks take turns on a multiprocessor (two fit).
-    // Of 128 or 256 numbers twice as many blocks still gain (16 rows of 32 heads of 128: 23.3 against 29.6), in bfloat16 they do not (40.8
-    // and 33.4), and heads of 32 in bfloat16 lose with any (17.6 and 14.2).
-    const int most = sizeof(T) == 4 ? (head_dim > 64 ? 592 : 296) : head_dim > 32 ? 296 : 0;
+    // Few rows by a block, us against a warp a (row, head).  32-bit, up to 296 blocks (two fit a multiprocessor): 32 heads of 64 behind
+    // 130 keys, 4 / 8 / 16 rows 9.4 / 9.6 / 18.5 against 16.4 / 16.4 / 16.5, 4 rows behind 5,000 251 against 614; above 64 numbers also
+    // where the blocks take two turns, unless few keys leave the turns' own cost: 32 rows of 16 heads of 128 behind 130 keys 24.0 and
+    // 28.4, behind 48 shorter, behind 30 / 16 9.2 / 8.6 and 8.4 / 6.4.  bfloat16, up to 296 blocks: 4 rows of 32 heads of 64 behind 130
+    // keys 18.5 and 23.2, behind 12 6.2 and 4.7; of 256 behind 16 keys 8.5 and 11.1; heads of 32 and less longer behind any (17.6, 14.2).
+    const int most = sizeof(T) == 4 ? (head_dim > 64 && reach > 32 ? 592 : 296) : head_dim > (reach > 16 ? 32 : 64) ? 296 : 0;
     if ((int64_t)rows * num_heads <= most) {
         auto kernel = head_dim <= 32 ? attention_rows_shared_kernel<T, 1> : head_dim <= 64 ? attention_rows_shared_kernel<T, 2>
                     : head_dim <= 128 ? attention_rows_shared_kernel<T, 4> : attention_rows_shared_kernel<T, 8>;
@@ -338,21 +339,22 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
 
 // q: rows x (num_heads*head_dim) with row stride q_stride (elements); out likewise.
 // cache: base of the cache entry, [page][K|V][kv_head][page_size][head_dim].
-// head_dim must be a multiple of 8 (16-byte key rows) and at most 256.
+// head_dim must be a multiple of 8 (16-byte key rows) and at most 256.  reach: the keys that a request's table can hold, at
+// most (it picks the form only; both give the same bits).
 TB_EXPORT int tb_attention_rows(const void* q, int64_t q_stride, void* out, int64_t out_stride, const void* cache,
                                 const int* positions, const int* seq_of_row, const int* block_table,
                                 int bt_stride, int rows, int num_heads, int num_kv_heads, int head_dim,
-                                int page_size, int window, float scale, int dtype, cudaStream_t stream) {
+                                int page_size, int reach, int window, float scale, int dtype, cudaStream_t stream) {
     if (rows == 0) return 0;
     if (head_dim <= 0 || head_dim > 256 || head_dim % 8 != 0) return TB_ERR_BAD_SIZE;
     if (num_kv_heads <= 0 || num_heads % num_kv_heads != 0) return TB_ERR_BAD_SIZE;
     if ((uintptr_t)cache % 16 != 0) return TB_ERR_BAD_ALIGN;
     if (dtype == TB_F32)
         return launch<float>(q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table, bt_stride,
-                             rows, num_heads, num_kv_heads, head_dim, page_size, window, scale, stream);
+                             rows, num_heads, num_kv_heads, head_dim, page_size, reach, window, scale, stream);
     if (dtype == TB_BF16)
         return launch<__nv_bfloat16>(q, q_stride, out, out_stride, cache, positions, seq_of_row, block_table,
-                                     bt_stride, rows, num_heads, num_kv_heads, head_dim, page_size, window, scale,
-                                     stream);
+                                     bt_stride, rows, num_heads, num_kv_heads, head_dim, page_size, reach, window,
+                                     scale, stream);
     return TB_ERR_BAD_DTYPE;
 }

@@ -219,7 +219,8 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, seq_of_row: torch.
 def attention_rows(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, positions: torch.Tensor,
                    seq_of_row: torch.Tensor, block_table: torch.Tensor, num_heads: int, num_kv_heads: int,
                    head_dim: int, page_size: int, window: int, scale: float) -> torch.Tensor:
-    """Plain paged attention, one warp per (row, head).  ``q``/``out``: ``[T, num_heads*head_dim]`` views."""
+    """Plain paged attention, a warp (in steps of few rows a block) per (row, head) and the same order of every sum either way.
+    ``q``/``out``: ``[T, num_heads*head_dim]`` views."""
     _cuda(q, out, cache, positions, seq_of_row, block_table)
     rows = q.shape[0]
     _need(q.stride(1) == 1 and out.stride(1) == 1 and q.shape[1] == num_heads * head_dim and out.shape == q.shape,
@@ -233,7 +234,8 @@ def attention_rows(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, posi
     _check(lib.tb_attention_rows(_ptr(q), _i64(q.stride(0)), _ptr(out), _i64(out.stride(0)), _ptr(cache),
                                  _ptr(positions), _ptr(seq_of_row), _ptr(block_table), _i32(block_table.stride(0)),
                                  _i32(rows), _i32(num_heads), _i32(num_kv_heads), _i32(head_dim), _i32(page_size),
-                                 _i32(window), _f32(scale), _i32(_code(q.dtype)), _stream()), "attention_rows")
+                                 _i32(min(block_table.shape[1] * page_size, 2 ** 31 - 1)), _i32(window), _f32(scale),
+                                 _i32(_code(q.dtype)), _stream()), "attention_rows")
     return out
 
 

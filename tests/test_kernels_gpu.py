@@ -526,6 +526,42 @@ def test_attention_rows_gives_few_rows_the_bits_of_many(dtype, d, nh):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [16, 48, 64, 104, 256])
+@pytest.mark.parametrize("window", [0, 100, 2100, 3000])
+def test_attention_rows_carries_few_rows_over_runs_of_keys(dtype, d, window):
+    """A block takes 64 key blocks at a time: rows behind the ends of one, two and three such runs, and windows that begin inside a key
+    block and reach over an end, against a step of so many rows that each takes a warp.  Behind few keys the widths of the tables on
+    either side of the lines between the two forms."""
+    from tesseract_b200 import kernels
+
+    nh, kv, page, longest = 4, 2, 16, 5040
+    last = [2046, 2047, 2048, 2079, 2080, 4095, 4096, 5000, 5039]
+    seqs, g = 3, torch.Generator().manual_seed(d)
+    cache = dev(torch.randn(seqs * longest // page + 1, 2, kv, page, d, generator=g).to(dtype))
+    table = dev((torch.randperm(seqs * longest // page, generator=g) + 1).to(torch.int32).view(seqs, longest // page))
+    rows = 300
+    positions = torch.tensor([last[i % 9] for i in range(rows)], dtype=torch.int32)
+    of_row = dev(torch.arange(rows, dtype=torch.int32) % seqs)
+    q = dev(torch.randn(rows, nh * d, generator=g).to(dtype))
+
+    def run(lo, hi, positions, columns):
+        out = torch.empty(hi - lo, nh * d, dtype=dtype, device="cuda")
+        kernels.attention_rows(q[lo:hi], out, cache, dev(positions[lo:hi]), of_row[lo:hi], table[:, :columns], nh, kv, d, page, window, d ** -0.5)
+        return out
+
+    many = run(0, rows, positions, table.shape[1])
+    assert torch.isfinite(many).all()
+    for lo, hi in ((0, 9), (9, 83), (100, 101)):                     # up to 74 rows, 296 blocks
+        assert torch.equal(run(lo, hi, positions, table.shape[1]), many[lo:hi])
+    for columns in (1, 2, 3, 128, 129):
+        short = torch.tensor([(7 * i) % (16 * columns) for i in range(rows)], dtype=torch.int32)
+        short[0] = 16 * columns - 1
+        want = run(0, rows, short, columns)
+        for lo, hi in ((0, 5), (0, 74), (140, 288)):                 # 20, 296 and 592 blocks
+            assert torch.equal(run(lo, hi, short, columns), want[lo:hi])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d, nh", [(24, 4), (56, 4), (104, 4), (232, 4)])
 def test_attention_rows_gives_steps_of_any_size_the_same_bits(dtype, d, nh):
     """Steps that fill the chip ask for a key's numbers as they need them, smaller ones for several at a time."""
