@@ -259,6 +259,41 @@ def test_attention_rows_mma_gives_few_rows_the_bits_of_many(dim, vdim, per_value
         assert torch.equal(run(lo, hi), many[lo:hi])
 
 
+@pytest.mark.parametrize("extra", ["sinks", "pooled", "kept", "bias", "kept and biased", "gate"])
+@pytest.mark.parametrize("dim, vdim", [(64, 48), (64, 64), (64, 128), (128, 64), (128, 128)])
+def test_attention_rows_mma_gives_few_rows_the_bits_of_many_with_all_it_can_add(dim, vdim, extra):
+    """The same for what a row may add to its keys and scores: five tiles ahead and two must walk the same keys in the same order."""
+    from tesseract_b200 import kernels
+
+    kv, heads, page, pool, window, rows = 8, 16, 16, 4, 90, 320
+    g = torch.Generator().manual_seed(dim + vdim)
+    last = [0, 40, 90, 130, 255, 330, 500, 639, 638, 637]
+    positions = torch.tensor([last[i % 10] for i in range(rows)], dtype=torch.int32)
+    table = (torch.randperm(40 * 10, generator=g) + 1).to(torch.int32).view(10, 40)
+    cache = dev(torch.randn(401, kv * page * (dim + vdim), generator=g).bfloat16())
+    q = torch.randn(rows, heads * dim, generator=g).bfloat16()
+    table, seq = dev(table), torch.arange(rows, dtype=torch.int32) % 10
+    sinks, weight, rate = (dev(torch.rand(heads, generator=g)) for _ in range(3))
+    averages = dev(torch.randn(101, kv * page * (dim + vdim), generator=g).bfloat16())
+    pools = dev((torch.randperm(100, generator=g) + 1).to(torch.int32).view(10, 10))          # 160 averaged blocks of 4 tokens
+    gates = torch.randn(rows, heads, generator=g).bfloat16()
+    mask = kernels.MASK_WINDOW_POOLED if extra == "pooled" else kernels.MASK_WINDOW
+
+    def run(lo, hi):
+        added = {"sinks": dict(sinks=sinks, softcap=20.0), "pooled": dict(pooled=(averages, pools, pool), sinks=sinks),
+                 "kept": dict(keep_first=70), "bias": dict(distance_bias=(weight, rate)),
+                 "kept and biased": dict(keep_first=5, distance_bias=(weight, rate)), "gate": dict(head_gate=dev(gates[lo:hi]))}[extra]
+        out = torch.empty(hi - lo, heads * vdim, device="cuda")
+        kernels.attention_rows_mma(dev(q[lo:hi]), out, cache, dev(positions[lo:hi]), dev(seq[lo:hi]), table, heads=heads, kv_heads=kv, dim=dim,
+                                   vdim=vdim, page_size=page, mask_kind=mask, mask_size=window, scale=dim ** -0.5, **added)
+        return out
+
+    many = run(0, rows)
+    assert torch.isfinite(many).all()
+    for lo, hi in ((0, 10), (7, 8), (100, 118)):
+        assert torch.equal(run(lo, hi), many[lo:hi])
+
+
 @pytest.mark.parametrize("page", [1, 2, 12, 24, 37, 64])
 @pytest.mark.parametrize("dim, vdim, per_value, mask, size", [(64, 48, 1, 0, 1), (64, 64, 1, 1, 100), (64, 128, 2, 2, 70), (128, 128, 1, 0, 1)])
 def test_pages_of_any_size_give_the_bits_of_pages_of_sixteen(page, dim, vdim, per_value, mask, size):
