@@ -69,8 +69,9 @@ struct Layout {
 
 template <int D, int DV>
 __global__ void __launch_bounds__(128)
-attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
-                        const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
+attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache,
+                        const int* __restrict__ positions, const int* __restrict__ seq_of_row,
+                        const int* __restrict__ block_table, int bt_stride, int heads,
                         const Paging paging, int mask_kind, int mask_size, float scale, float* __restrict__ parts) {
     typedef Layout<D, DV> L;
     constexpr int KS = L::KS, PS = L::PS;
@@ -91,7 +92,8 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     float* stats = reinterpret_cast<float*>(smem + L::STAT_AT);
 
-    // a tile's copy: sixteen lanes a key, whose 16-byte chunks they take side by side, eight keys at a time
+    // a tile's copy: sixteen lanes a key, whose 16-byte chunks they take side by side, eight keys at a time.  (Where the first tile's
+    // keys lie is looked up before the wait: the launch is an early one only where no kernel may still write that.)
     auto look = [&](int tile, int (&pages)[KT / 8]) {             // where this thread's keys lie
 #pragma unroll
         for (int i = 0; i < KT / 8; ++i) pages[i] = table[paging.page_of(min(key_lo + tile * KT + i * 8 + (tid >> 4), pos))];
@@ -112,7 +114,7 @@ attention_latent_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_
     };
     int pages[KT / 8];
     if (tile_first < tile_end) look(tile_first, pages);
-    pdl_wait();                                                   // queries and the step's keys come from kernels in front (its metadata does not: see `early` below)
+    pdl_wait();                                                   // queries and the step's keys come from kernels in front
     // the sixteen heads' queries (heads the model does not have are rows of zeros)
     for (int index = tid; index < 16 * (D / 8); index += 128) {
         const int h = index / (D / 8), chunk = index % (D / 8);

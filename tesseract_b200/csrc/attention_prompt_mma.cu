@@ -373,15 +373,15 @@ attention_prompt_kernel(const bf16* __restrict__ q, int64_t q_stride, bf16* __re
 // share every tile of 64 keys, 16 keys a warp, each with a streaming softmax of its own, and their partial results
 // (maximum, sum, accumulator) meet in shared memory in warp order.
 // STAGES: tiles in shared memory.  Where every block has room for kDeep of them they are asked for that far ahead, with one barrier a
-// tile; the first tiles' pages are looked up before the wait (launched early only where no kernel may still write them), the others' a tile
-// ahead.
-// (The queries are not __restrict__: loads that the compiler takes for constant may be moved in front of the wait.)
+// tile; the first tiles' pages are looked up before the wait (the launch is an early one only where no kernel may still write them),
+// the others' a tile ahead.  (The queries are not __restrict__: loads that the compiler takes for constant may be moved in front of
+// the wait.)
 template <int D, int DV, bool BIASED, int STAGES>
 __global__ void __launch_bounds__(128)
-attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache, const int* __restrict__ positions,
-                      const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride, int heads,
-                      int kv_heads, const Paging paging, int mask_kind, int mask_size, float scale, int keys_per_value,
-                      int out_f32, Extras x) {
+attention_rows_kernel(const bf16* q, int64_t q_stride, bf16* out, int64_t out_stride, const bf16* cache,
+                      const int* __restrict__ positions, const int* __restrict__ seq_of_row,
+                      const int* __restrict__ block_table, int bt_stride, int heads, int kv_heads,
+                      const Paging paging, int mask_kind, int mask_size, float scale, int keys_per_value, int out_f32, Extras x) {
     constexpr int KS = D * 2 + 16, VS = DV * 2 + 16;
     constexpr int STAGE = KT * (KS + VS);
     constexpr int PART = DV + 2;                                  // a row's accumulator, maximum and sum

@@ -285,11 +285,12 @@ int launch(const void* q, int64_t q_stride, void* out, int64_t out_stride, const
            const int* positions, const int* seq_of_row, const int* block_table, int bt_stride, int rows,
            int num_heads, int num_kv_heads, int head_dim, int page_size, int reach, int window, float scale,
            cudaStream_t stream) {
-    // Few rows by a block, us against a warp a (row, head).  32-bit, up to 296 blocks (two fit a multiprocessor): 32 heads of 64 behind
-    // 130 keys, 4 / 8 / 16 rows 9.4 / 9.6 / 18.5 against 16.4 / 16.4 / 16.5, 4 rows behind 5,000 251 against 614; above 64 numbers also
-    // where the blocks take two turns, unless few keys leave the turns' own cost: 32 rows of 16 heads of 128 behind 130 keys 24.0 and
-    // 28.4, behind 48 shorter, behind 30 / 16 9.2 / 8.6 and 8.4 / 6.4.  bfloat16, up to 296 blocks: 4 rows of 32 heads of 64 behind 130
-    // keys 18.5 and 23.2, behind 12 6.2 and 4.7; of 256 behind 16 keys 8.5 and 11.1; heads of 32 and less longer behind any (17.6, 14.2).
+    // Few rows by a block, us against a warp a (row, head).  32-bit, up to 296 blocks (two fit a multiprocessor): 32 heads of 64
+    // behind 130 keys, 4 / 8 / 16 rows 9.4 / 9.6 / 18.5 against 16.4 / 16.4 / 16.5, 4 rows behind 5,000 251 against 614.  Above 64
+    // numbers also where the blocks take two turns, unless the keys are few: 32 rows of 16 heads of 128 behind 130 / 48 / 30 / 16 keys
+    // 24.0 / 11.9 / 9.2 / 8.6 against 28.4 / 12.4 / 8.4 / 6.4.  bfloat16, up to 296 blocks: 4 rows of 32 heads of 64 behind 130 keys
+    // 18.5 against 23.2, behind 12 6.2 against 4.7; 4 of 16 heads of 256 behind 16 8.5 against 11.1; heads of 32 and less behind any
+    // keys longer (17.6 against 14.2).
     const int most = sizeof(T) == 4 ? (head_dim > 64 && reach > 32 ? 592 : 296) : head_dim > (reach > 16 ? 32 : 64) ? 296 : 0;
     if ((int64_t)rows * num_heads <= most) {
         auto kernel = head_dim <= 32 ? attention_rows_shared_kernel<T, 1> : head_dim <= 64 ? attention_rows_shared_kernel<T, 2>

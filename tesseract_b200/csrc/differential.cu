@@ -14,11 +14,13 @@
 namespace {
 
 // Bound by the chain of a launch in steps of few rows: gridDim.y blocks share a row there, and where the row goes and the sines of a
-// thread's first pair (mostly of all its pairs) are found before the wait, for neither depends on a kernel in front.  8 rows of 32 + 8
-// heads of 64: 1.7 us, 4.2 before.  (The rows are not __restrict__: their loads stay behind the wait.)
+// thread's first pair (mostly of all its pairs) are found before the wait, for neither depends on a kernel in front (the launch is
+// an early one only where the caller vouches for that).  8 rows of 32 + 8 heads of 64: 1.7 us, 4.2 before.  (The rows are not __restrict__:
+// their loads stay behind the wait.)
 template <typename T>
 __global__ void __launch_bounds__(256)
-pair_rope_cache_kernel(const T* proj, int64_t proj_stride, T* q_out, int64_t q_stride, T* cache, const int* __restrict__ positions, const int* __restrict__ seq_of_row,
+pair_rope_cache_kernel(const T* proj, int64_t proj_stride, T* q_out, int64_t q_stride, T* cache,
+                       const int* __restrict__ positions, const int* __restrict__ seq_of_row,
                        const int* __restrict__ block_table, int bt_stride, const float* __restrict__ inv_freq,
                        int q_heads, int key_heads, int value_heads, int dim, int vdim, int rot_dims, int page_size) {
     pdl_trigger();

@@ -15,12 +15,13 @@
 namespace {
 
 // Bound by the chain of a launch in steps of few rows: there the first of gridDim.y blocks of a row takes the latent and the shared
-// part, the others the heads' parts, and where the row goes and a thread's first sines are found before the wait.  8 rows of 16 heads,
-// 512 + 64 numbers: 2.3 us, 3.7 before.  (The rows are not __restrict__: their loads stay behind the wait.)
+// part, the others the heads' parts, and where the row goes and a thread's first sines are found before the wait (the launch is an
+// early one only where the caller vouches for the index arrays).  8 rows of 16 heads, 512 + 64 numbers: 2.3 us, 3.7 before.  (The
+// rows are not __restrict__: their loads stay behind the wait.)
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_rope_cache_kernel(const float* down, int64_t down_stride, const T* q, int64_t q_stride, T* q_full, int64_t full_stride, T* cache,
-                         const float* __restrict__ weight, const int* __restrict__ positions,
+latent_rope_cache_kernel(const float* down, int64_t down_stride, const T* q, int64_t q_stride, T* q_full,
+                         int64_t full_stride, T* cache, const float* __restrict__ weight, const int* __restrict__ positions,
                          const int* __restrict__ seq_of_row, const int* __restrict__ block_table, int bt_stride,
                          const float* __restrict__ inv_freq, int heads, int dim, int rank, int rot_width, int rot_dims,
                          int page_size, float eps, float amplitude) {

@@ -430,7 +430,8 @@ class ChunkGraphs:
         """Rows that a tail of ``n`` tokens takes in its graph: more than ``n`` (a padding row at least)."""
         if n == 0:
             return 0
-        bucket = 32          # (a prompt of 23 tokens: 1,008 us on 32 rows, 1,067 on 64)
+        bucket = 32          # (1B sizes, prompts of 2 / 8 / 15 / 23 / 31 tokens: 1,083 / 1,023 / 1,024 / 1,023 / 1,081 us on 32 rows,
+                             #  1,138 / 1,082 / 1,081 / 1,079 / 1,089 on 64)
         while bucket <= n and bucket < self.rows:
             bucket <<= 1
         return min(bucket, self.rows)

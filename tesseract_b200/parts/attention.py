@@ -114,7 +114,7 @@ class Attention(Mixer):
                               write_kv=cache.writes)
         q = qkv[:, :self.q_width]
         if choice.rows:
-            # the 32-bit path: one warp per (row, head), a fixed order of every reduction
+            # the 32-bit path: a warp or, in steps of few rows, a block per (row, head), the same order of every reduction
             kernels.attention_rows(q, attended, cache.storage, ctx.positions, ctx.seq_of_row, group.block_table,
                                    self.num_heads, self.num_kv_heads, self.head_dim, cache.page_size, self.window,
                                    self.scale)

@@ -236,7 +236,7 @@ class AttentionPlan:
 
     def __str__(self) -> str:
         if self.rows:
-            return "attention_rows (one warp per row and head, fixed order)"
+            return "attention_rows (a warp, in steps of few rows a block, per row and head; fixed order)"
         if self.fused_decode:
             return f"attention_decode (rotation and cache write folded in; {self.splits} split(s), merge: {self.merge})"
         parts = ["rope_kv_write"]
@@ -343,9 +343,12 @@ def describe(model, row_counts: Sequence[int] = (1, 8, 16, 17, 64, 512, 2048), c
                 lines.append(f"    gate/up  {product(dtype, rows, gu.out_features, gu.in_features, epilogue=epilogue, norm='prepared' if prepared else 'add_norm')}")
                 lines.append(f"    down     {product(dtype, rows, down.out_features, down.in_features, follow=True)}")
             elif ffn is not None and hasattr(ffn, "products"):
-                lines.append(f"    feed-forward '{ffn.kind}' (its own kernel between the products)")
-                for name, linear, epilogue in ffn.products():
-                    lines.append(f"      {name:10s} {product(dtype, rows, linear.out_features, linear.in_features, epilogue=epilogue)}")
+                choices = [(name, product(dtype, rows, linear.out_features, linear.in_features, epilogue=epilogue))
+                           for name, linear, epilogue in ffn.products()]
+                inside = any(choice.epilogue in OVER_GATE_AND_UP for _, choice in choices)
+                lines.append(f"    feed-forward '{ffn.kind}' "
+                             f"({'activated by the product in front' if inside else 'its own kernel between the products'})")
+                lines.extend(f"      {name:10s} {choice}" for name, choice in choices)
             elif ffn is not None:
                 lines.append(f"    feed-forward '{ffn.kind}' (its own code)")
             gates = getattr(block, "gates", None)
