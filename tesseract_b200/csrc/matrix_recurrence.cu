@@ -824,9 +824,10 @@ recurrence_norm_kernel(const float* __restrict__ v, const float* __restrict__ au
     for (int i = kKeepNumbers * STEP + lane; i < size; i += STEP) finish(i, value(i));
 }
 
-// The same in packets of four numbers, where sizes and rows allow them.
-template <typename T, bool WIDE, int KEEP>
-__global__ void __launch_bounds__(WIDE ? 256 : kNormThreads)
+// The same in packets of four numbers, where sizes and rows allow them.  EARLY: packets of the weights that are asked for before the
+// wait; BLOCKS: those that are to fit on a multiprocessor, 0 where the compiler may choose (see launch_norm).
+template <typename T, bool WIDE, int KEEP, int EARLY, int BLOCKS>
+__global__ void __launch_bounds__(WIDE ? 256 : kNormThreads, BLOCKS)
 recurrence_norm_packets_kernel(const float* v, const float* aux, const T* gate,
                                int64_t gate_stride, const float* __restrict__ weight, int weight_len, T* out,
                                int64_t out_stride, int groups, int size, float eps, int gate_kind) {
@@ -842,8 +843,7 @@ recurrence_norm_packets_kernel(const float* v, const float* aux, const T* gate,
     T* dst = out + (int64_t)row * out_stride + (int64_t)g * size;
     const float* w = weight + (weight_len == size ? 0 : (int64_t)g * size);
     const int packets = size / 4;
-    constexpr int EARLY = KEEP < 4 ? KEEP : 4;       // packets of the weights that are asked for before the wait
-    float4 x[KEEP], z[KEEP], f[EARLY];
+    float4 x[KEEP], z[KEEP], f[EARLY > 0 ? EARLY : 1];
 #pragma unroll
     for (int e = 0; e < EARLY; ++e)
         if (e * STEP + lane < packets) f[e] = *reinterpret_cast<const float4*>(w + 4 * (e * STEP + lane));
@@ -894,11 +894,22 @@ int launch_norm(const float* v, const float* aux, const void* gate, int64_t gate
     launched = tb_launch_pdl(KERNEL, GRID, dim3(THREADS), (size_t)0, stream, v, aux, (const T*)gate, gate_stride, weight,   \
                              weight_len, (T*)out, out_stride, groups, size, eps, gate_kind)
     const dim3 narrow(rows, (groups + 3) / 4), wide(rows, groups);
-    if (packets && size <= 128) TB_NORM((recurrence_norm_packets_kernel<T, false, 1>), narrow, kNormThreads);
-    else if (packets && size <= 256) TB_NORM((recurrence_norm_packets_kernel<T, false, 2>), narrow, kNormThreads);
-    else if (packets && size <= 1024) TB_NORM((recurrence_norm_packets_kernel<T, false, 8>), narrow, kNormThreads);
-    else if (packets && size <= 4096) TB_NORM((recurrence_norm_packets_kernel<T, true, 4>), wide, 256);
-    else if (packets && size <= 8192) TB_NORM((recurrence_norm_packets_kernel<T, true, 8>), wide, 256);
+    const int64_t warps4 = (int64_t)narrow.x * narrow.y, blocks = (int64_t)rows * groups;
+    // Few blocks are bound by the chain of a launch: weights in registers before the wait take 0.4 to 0.6 us off it (a bfloat16 row of
+    // 2,048 / 4,096 / 6,144 / 8 x 512 numbers 1.7 / 1.9 / 2.8 / 1.8 us, 2.1 / 2.6 / 3.2 / 2.3 without).  Where there are more blocks than
+    // those registers leave room for (3, 1 and 3 a multiprocessor) they cost more: 2,048 rows of 2,048 / 4,096 / 6,144 / 8,192 numbers
+    // 9.1 / 13.4 / 45.0 / 49.5 us, held to 4, 4, 2 and 2 blocks 8.2 / 12.0 / 28.1 / 32.3; of 8 x 512 / 16 x 260 25.0 / 44.6, without early
+    // weights 21.2 / 36.4 (1,000 rows of 4 x 1,024 7.6 and 7.4, 300 of 16 x 260 5.7 and 6.0).  In 32-bit four blocks of 2,048 to 4,096
+    // numbers have no room for early weights: 2,048 rows 14.7 / 20.1, with them 16.0 / 19.7.
+    constexpr int CROWDED = sizeof(T) == 4 ? 0 : 4;
+    if (packets && size <= 128) TB_NORM((recurrence_norm_packets_kernel<T, false, 1, 1, 0>), narrow, kNormThreads);
+    else if (packets && size <= 256) TB_NORM((recurrence_norm_packets_kernel<T, false, 2, 2, 0>), narrow, kNormThreads);
+    else if (packets && size <= 1024 && warps4 <= (size > 512 ? 888 : 1332)) TB_NORM((recurrence_norm_packets_kernel<T, false, 8, 4, 0>), narrow, kNormThreads);
+    else if (packets && size <= 1024) TB_NORM((recurrence_norm_packets_kernel<T, false, 8, 0, 0>), narrow, kNormThreads);
+    else if (packets && size <= 4096 && blocks <= 444) TB_NORM((recurrence_norm_packets_kernel<T, true, 4, 4, 0>), wide, 256);
+    else if (packets && size <= 4096) TB_NORM((recurrence_norm_packets_kernel<T, true, 4, CROWDED, 4>), wide, 256);
+    else if (packets && size <= 8192 && blocks <= 148) TB_NORM((recurrence_norm_packets_kernel<T, true, 8, 4, 0>), wide, 256);
+    else if (packets && size <= 8192) TB_NORM((recurrence_norm_packets_kernel<T, true, 8, 4, 2>), wide, 256);
     else if (size <= 256) TB_NORM((recurrence_norm_kernel<T, false>), narrow, kNormThreads);
     else TB_NORM((recurrence_norm_kernel<T, true>), wide, kNormThreads);
 #undef TB_NORM

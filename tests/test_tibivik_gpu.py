@@ -320,6 +320,38 @@ def test_cuts_of_the_recurrence_differ_by_rounding(kind, m):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gate_kind", [0, 1, 2])
+@pytest.mark.parametrize("groups, size", [(8, 512), (3, 1024), (2, 1028), (1, 4096), (1, 4100), (1, 6144), (2, 8192)])
+def test_the_norm_of_a_row_has_the_same_bits_among_any_number_of_others(groups, size, gate_kind, dtype):
+    """Steps of few blocks hold weights in registers that those of many have no room for: rows on both sides of the lines, against
+    the formula in 64 bits."""
+    from tesseract_b200 import kernels
+
+    most = {8: 700, 3: 1400, 2: 250, 1: 460}[groups]
+    g = torch.Generator().manual_seed(size)
+    v, aux = torch.randn(most, groups * size, generator=g).to(dev()), torch.randn(most, groups, 2, generator=g).to(dev())
+    gate = torch.randn(most, groups * size, generator=g).to(dtype).to(dev())
+    weight = torch.randn(size, generator=g).to(dev())
+
+    def run(rows):
+        out = torch.empty(rows, groups * size, dtype=dtype, device=dev())
+        kernels.recurrence_norm(v[:rows], gate[:rows], weight, out, groups=groups, size=size, eps=1e-5, gate_kind=gate_kind, aux=aux[:rows])
+        return out
+
+    many = run(most)
+    for rows in (1, 70, 74, 75, 148, 149, 222, 223, 444, 445):
+        assert torch.equal(run(min(rows, most)), many[:rows]), rows
+    x = v[:5].double().view(5, groups, size) / (torch.maximum(aux[:5, :, 0].double().abs(), torch.exp(-aux[:5, :, 1].double())) + 1e-6)[..., None]
+    z = gate[:5].double().view(5, groups, size)
+    act = torch.sigmoid(z) if gate_kind == 0 else z * torch.sigmoid(z)
+    x = x * act if gate_kind == 2 else x
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * weight.double() * (1.0 if gate_kind == 2 else act)
+    # (32-bit sums of up to 8,192 squares and a dozen roundings, then the rounding to the run dtype)
+    limit = 2e-5 if dtype == torch.float32 else 2.0 ** -8
+    assert ((many[:5].double().view(5, groups, size) - want).abs() <= limit * (want.abs() + 0.01)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads", [4, 8])
 @pytest.mark.parametrize("dim", [24, 62, 64, 90, 128])
 @pytest.mark.parametrize("kind", ["STATE_SPACE", "MATRIX_MEMORY", "DELTA_RULE"])
